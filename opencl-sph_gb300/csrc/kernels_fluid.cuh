@@ -58,9 +58,8 @@ __device__ __forceinline__ void density_one(const SceneDesc &S, unsigned n, unsi
     const bool active = item < n;
     const unsigned k = item;
     const unsigned i = active ? min(S.cellparticles[k], S.pnum - 1) : 0u;
-    const float h = *S.h;
-    const DistBounds B = dist_bounds(h);
-    const float h2 = __fmul_rn(h, h);
+    const ScenePair B = scene_pair(S);
+    const float h = B.h, h2 = B.h2;
     const float3 ipos = active ? xyz(S.spos[k]) : make_float3(0.f, 0.f, 0.f);
     const NegPoint nip = neg_point(ipos);
     Planes P;
@@ -71,7 +70,7 @@ __device__ __forceinline__ void density_one(const SceneDesc &S, unsigned n, unsi
     Kahan rho;
     unsigned count = 0, total = 0;
     bool overflow = false;
-    const StencilRows rows(S, active ? S.gridcell[i] : 0u);
+    const StencilRows rows(S, active ? S.srow[k] : make_uint2(0u, 0u));
     const float4 *__restrict__ spos = S.spos;
 #pragma unroll 1
     for (int r = 0; r < 9; ++r) {
@@ -143,7 +142,7 @@ __device__ __forceinline__ void density_one(const SceneDesc &S, unsigned n, unsi
         }
     }
     if (active) {
-        const float value = poly6_density(rho.s, h2, h, *S.mass);
+        const float value = rho.s * B.coef * *S.mass;
         if (original) {
             S.density0[i] = value;
         } else {
@@ -222,9 +221,9 @@ __device__ __forceinline__ void integrate(const SceneDesc &S, unsigned i, float3
 struct FluidI {
     float3 ipos, ivel;
     float2 nxy, nvxy;  // -ipos and -ivel's x, y lanes (the packed differences)
-    float inv_rhoi, pi, h, rho0, stiff, visc, kv;
+    float inv_rhoi, pi, h, rho0, stiff;
     float vk, pk;  // visc kv and -kv / 2, the pair term's constant factors
-    DistBounds B;
+    float lt, le;
 };
 
 __device__ __forceinline__ FluidI fluid_i(const SceneDesc &S, float3 ipos, float3 ivel, float rhoi) {
@@ -234,16 +233,15 @@ __device__ __forceinline__ FluidI fluid_i(const SceneDesc &S, float3 ipos, float
     I.nxy = make_float2(-ipos.x, -ipos.y);
     I.nvxy = make_float2(-ivel.x, -ivel.y);
     I.inv_rhoi = rcp_approx(rhoi);
-    I.h = *S.h;
-    I.B = dist_bounds(I.h);
+    const ScenePair B = scene_pair(S);
+    I.h = B.h;
+    I.lt = B.lt;
+    I.le = B.le;
     I.rho0 = *S.restdens;
     I.stiff = *S.stiffness;
-    I.visc = *S.viscosity;
-    const float h3 = I.h * I.h * I.h;
-    I.kv = 45.0f / (SPH_PI_F * h3 * h3);  // 45 / (pi h^6)
     I.pi = fluid_pressure(rhoi, I.rho0, I.stiff);
-    I.vk = __fmul_rn(I.visc, I.kv);
-    I.pk = __fmul_rn(-0.5f, I.kv);
+    I.vk = __fmul_rn(*S.viscosity, B.kv);
+    I.pk = __fmul_rn(-0.5f, B.kv);
     return I;
 }
 
@@ -263,7 +261,7 @@ __device__ __forceinline__ float fluid_pair_p(const FluidI &I, float pi, float3 
     const float dz = __fsub_rn(jpos.z, I.ipos.z);
     const float2 sq = __fmul2_rn(dxy, dxy);
     const float r2 = __fadd_rn(__fadd_rn(sq.x, sq.y), __fmul_rn(dz, dz));
-    if ((!IN_RANGE && !(r2 <= I.B.le)) || r2 == 0.f) return r2;
+    if ((!IN_RANGE && !(r2 <= I.le)) || r2 == 0.f) return r2;
     const float rinv = rsqrtf(r2);
     const float dist = __fmul_rn(r2, rinv);
     const float din = __fsub_rn(I.h, dist);
@@ -323,16 +321,16 @@ __device__ __forceinline__ void walk_pair(const FluidI &I, bool solid_i, float4 
     if (MIXED) {
         const bool solid_j = v.w < 0.f;
         if (solid_i && solid_j) {
-            count += norm2(sub3(xyz(p), I.ipos)) <= I.B.lt;
+            count += norm2(sub3(xyz(p), I.ipos)) <= I.lt;
             return;
         }
         if (solid_i || solid_j) {
             count += fluid_pair_p<true>(I, fmaxf(I.pi, 0.f), xyz(p), xyz(v), fmaxf(p.w, 0.f), fabsf(v.w), f) <=
-                     I.B.lt;
+                     I.lt;
             return;
         }
     }
-    count += fluid_pair<true>(I, xyz(p), xyz(v), p.w, v.w, f) <= I.B.lt;
+    count += fluid_pair<true>(I, xyz(p), xyz(v), p.w, v.w, f) <= I.lt;
 }
 
 // The stencil scan: every candidate of the 27 cells, in the reference's
@@ -347,7 +345,7 @@ __device__ __forceinline__ unsigned fluid_scan(const SceneDesc &S, unsigned cell
     for_each_neighbour(S, cell, [&](unsigned kk) {
         const bool solid_j = MIXED && S.phase[min(S.cellparticles[kk], S.pnum - 1)] != 0u;
         if (solid_i && solid_j) {
-            count += norm2(sub3(xyz(spos[kk]), I.ipos)) <= I.B.lt;
+            count += norm2(sub3(xyz(spos[kk]), I.ipos)) <= I.lt;
             return;
         }
         const float rho = sdens[kk];
@@ -356,7 +354,7 @@ __device__ __forceinline__ unsigned fluid_scan(const SceneDesc &S, unsigned cell
             pi = fmaxf(pi, 0.f);
             pj = fmaxf(pj, 0.f);
         }
-        count += fluid_pair_p(I, pi, xyz(spos[kk]), xyz(svel[kk]), pj, rcp_approx(rho), f) <= I.B.lt;
+        count += fluid_pair_p(I, pi, xyz(spos[kk]), xyz(svel[kk]), pj, rcp_approx(rho), f) <= I.lt;
     }, [&] { f.end_row(); });
     return count;
 }
@@ -372,7 +370,7 @@ __global__ void k_forces_fluids(const SceneDesc *__restrict__ scenes, BlockMap m
         const FluidI I = fluid_i(S, xyz(S.spos[k]), xyz(S.svel[k]), S.sdens[k]);
         const bool solid_i = mixed_solid<MIXED>(S, i);
         BlockSum3 f;
-        fluid_scan<MIXED>(S, S.gridcell[i], I, f, solid_i);
+        fluid_scan<MIXED>(S, S.srow[k].x, I, f, solid_i);
         fluid_finish(S, i, I, f, fuse_step, mixed_extra<MIXED>(S, i, solid_i));
     }
     SPH_END_WORK
@@ -396,7 +394,7 @@ __global__ void __maxnreg__(64) k_forces_fluids_masked(const SceneDesc *__restri
         const unsigned k = item;
         const unsigned i = min(S.cellparticles[k], S.pnum - 1);
         const FluidI I = fluid_i(S, xyz(S.spos[k]), xyz(S.svel[k]), S.sdens[k]);
-        const unsigned cell = S.gridcell[i];
+        const StencilRows rows(S, S.srow[k]);
         const bool solid_i = mixed_solid<MIXED>(S, i);
         BlockSum3 f;
         unsigned count = 0;  // num_neighbours, which the density pass left to this one
@@ -406,7 +404,6 @@ __global__ void __maxnreg__(64) k_forces_fluids_masked(const SceneDesc *__restri
             const float4 *__restrict__ svel = S.svel;
             // two neighbours per iteration: both loads are in flight
             // before the first pair's arithmetic (same order)
-            const StencilRows rows(S, cell);
             // the next row's bounds and low mask word are loaded while this
             // row is walked
             unsigned nb, ne;
@@ -451,7 +448,7 @@ __global__ void __maxnreg__(64) k_forces_fluids_masked(const SceneDesc *__restri
                 f.end_row();
             }
         } else {
-            count = fluid_scan<MIXED>(S, cell, I, f, solid_i);
+            count = fluid_scan<MIXED>(S, rows.cell, I, f, solid_i);
         }
         if (!S.num_symmetry_planes) S.num_neighbours[i] = count;
         fluid_finish(S, i, I, f, fuse_step, mixed_extra<MIXED>(S, i, solid_i));

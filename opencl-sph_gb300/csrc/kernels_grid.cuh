@@ -362,7 +362,10 @@ __global__ void __launch_bounds__(1024) k_sort_big_cells(const SceneDesc *__rest
 // density when asked; for solids also the rest position with the body
 // number -- and in a mixed scene SPH_SOLID_PHASE_BIT for a solid-phase
 // particle -- and 1/density0 in the velocity copy's w).  Gathers once so
-// the pair loops stream float4s.
+// the pair loops stream float4s.  It also writes what every pair pass would
+// otherwise work out again in each thread, while this memory-bound kernel
+// has issue slots to spare: the particle's stencil rows (srow) and the
+// scene's constants (write_scene_pair).
 __global__ void k_gather(const SceneDesc *__restrict__ scenes, BlockMap map, int with_vel, int with_dens,
                          int with_solid) {
     SPH_FOR_WORK(map)
@@ -371,6 +374,9 @@ __global__ void k_gather(const SceneDesc *__restrict__ scenes, BlockMap map, int
         if (i >= S.pnum) i = 0;  // host-written garbage
         float3 p = ld3(S.position, i);
         S.spos[item] = make_float4(p.x, p.y, p.z, 0.f);
+        const unsigned cell = S.gridcell[i];
+        S.srow[item] = make_uint2(cell, StencilRows(S, cell).bits);
+        if (item == 0) write_scene_pair(S);
         const bool solid = with_solid && S.spos0;
         if (with_vel || solid) {
             float3 v = ld3(S.velocity, i);

@@ -37,7 +37,7 @@ __global__ void k_original_density_mixed(const SceneDesc *__restrict__ scenes, B
         const float3 ipos = xyz(S.spos[k]);
         const unsigned ph = S.phase[i];
         Kahan rho;
-        for_each_neighbour(S, S.gridcell[i], [&](unsigned kk) {
+        for_each_neighbour(S, S.srow[k].x, [&](unsigned kk) {
             const unsigned j = min(S.cellparticles[kk], S.pnum - 1);
             if (S.phase[j] != ph) return;
             const float r2 = norm2(sub3(xyz(S.spos[kk]), ipos));
@@ -46,7 +46,7 @@ __global__ void k_original_density_mixed(const SceneDesc *__restrict__ scenes, B
                 rho.add(d * d * d);
             }
         });
-        S.density0[i] = poly6_density(rho.s, C.h2, C.h, C.mass);
+        S.density0[i] = rho.s * C.coef * C.mass;
     }
     SPH_END_WORK
 }
@@ -65,8 +65,8 @@ __device__ __forceinline__ bool solid_partner(float4 q4, unsigned kk, unsigned k
 // loads are in flight before the first one's tests (the solid particles of
 // a mixed scene are too few warps to hide the latency otherwise).
 template <class F>
-__device__ __forceinline__ void for_each_candidate_sorted(const SceneDesc &S, unsigned cell, F &&f) {
-    const StencilRows rows(S, cell);
+__device__ __forceinline__ void for_each_candidate_sorted(const SceneDesc &S, uint2 srow, F &&f) {
+    const StencilRows rows(S, srow);
     const float4 *__restrict__ spos = S.spos;
     const float4 *__restrict__ spos0 = S.spos0;
 #pragma unroll 1
@@ -117,10 +117,10 @@ __global__ void k_deformations_mixed(const SceneDesc *__restrict__ scenes, Block
                 aqq[5] = __fmaf_rn(wq.y, q.z, aqq[5]);
             };
             if (masked && S.ncand[k] != SPH_NCAND_SCAN)
-                for_each_masked(S, k, StencilRows(S, S.gridcell[i]),
+                for_each_masked(S, k, StencilRows(S, S.srow[k]),
                                 [&](unsigned kk) { visit(kk, S.spos[kk], S.spos0[kk]); });
             else
-                for_each_candidate_sorted(S, S.gridcell[i], visit);
+                for_each_candidate_sorted(S, S.srow[k], visit);
             float inv[6];
             sym_inverse(aqq, inv);
             float F[9];
@@ -156,7 +156,7 @@ __global__ void k_forces_solids_mixed(const SceneDesc *__restrict__ scenes, Bloc
             for (int c = 0; c < 6; ++c) si[c] = S.stress[6 * (size_t)i + c];
             const float rho0i = S.density0[i];
             Kahan3 fe_s, fv_s;
-            for_each_candidate_sorted(S, S.gridcell[i], [&](unsigned kk, float4 p4, float4 q4) {
+            for_each_candidate_sorted(S, S.srow[k], [&](unsigned kk, float4 p4, float4 q4) {
                 if (!solid_partner(q4, kk, k)) return;
                 const float3 jpos = xyz(p4);
                 const float3 x = sub3(ipos0, xyz(q4));

@@ -221,16 +221,13 @@ struct SolidConsts {
 };
 __device__ __forceinline__ SolidConsts solid_consts(const SceneDesc &S) {
     SolidConsts c;
-    c.h = *S.h;
-    // rounded on its own, as the density pass rounds it: inlined, h * h
-    // could otherwise fuse with a later h2 - r2 into one FMA in some kernels
-    c.h2 = __fmul_rn(c.h, c.h);
-    DistBounds b = dist_bounds(c.h);
-    c.le = b.le;
-    c.lt = b.lt;
-    float h3 = c.h2 * c.h;
-    c.kv = 45.0f / (SPH_PI_F * h3 * h3);
-    c.coef = 315.0f / (64.0f * SPH_PI_F * h3 * h3 * h3);
+    const ScenePair p = scene_pair(S);
+    c.h = p.h;
+    c.h2 = p.h2;
+    c.le = p.le;
+    c.lt = p.lt;
+    c.kv = p.kv;
+    c.coef = p.coef;
     c.mass = *S.mass;
     return c;
 }
@@ -260,7 +257,7 @@ __global__ void k_rotations_and_strains_planes(const SceneDesc *__restrict__ sce
             const float3 ipos0 = ld3(S.originalpos, i);
             Planes P;
             load_planes(S, ipos, C.h, P);
-            const unsigned cell = S.gridcell[i];
+            const unsigned cell = S.srow[k].x;
             float apq[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
             for_each_neighbour(S, cell, [&](unsigned kk) {
                 const unsigned j = min(S.cellparticles[kk], S.pnum - 1);
@@ -450,7 +447,7 @@ __global__ void k_deformations_planes(const SceneDesc *__restrict__ scenes, Bloc
             aqq[1] += wq.y * q.y; aqq[5] += wq.y * q.z;
             aqq[2] += wq.z * q.z;
         };
-        for_each_neighbour(S, S.gridcell[i], [&](unsigned kk) {
+        for_each_neighbour(S, S.srow[k].x, [&](unsigned kk) {
             const unsigned j = min(S.cellparticles[kk], S.pnum - 1);
             const float3 jpos = xyz(S.spos[kk]);
             const float3 jpos0 = ld3(S.originalpos, j);
@@ -522,7 +519,7 @@ __global__ void k_forces_solids_planes(const SceneDesc *__restrict__ scenes, Blo
         Planes P;
         load_planes(S, ipos, C.h, P);
         Kahan3 fe_s, fv_s, fec_s, fvc_s;
-        for_each_neighbour(S, S.gridcell[i], [&](unsigned kk) {
+        for_each_neighbour(S, S.srow[k].x, [&](unsigned kk) {
             const unsigned j = min(S.cellparticles[kk], S.pnum - 1);
             const float3 jpos = xyz(S.spos[kk]);
             const float3 jpos0 = ld3(S.originalpos, j);
@@ -688,7 +685,7 @@ __global__ void __maxnreg__(64) k_rotations_and_strains(const SceneDesc *__restr
         const SolidConsts C = solid_consts(S);
         const float4 p4 = S.spos[k], q4 = S.spos0[k];
         const float3 ipos = xyz(p4), ipos0 = xyz(q4);
-        const StencilRows rows(S, S.gridcell[i]);
+        const StencilRows rows(S, S.srow[k]);
         const float4 *__restrict__ spos = S.spos;
         const float4 *__restrict__ spos0 = S.spos0;
         float apq[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
@@ -702,7 +699,7 @@ __global__ void __maxnreg__(64) k_rotations_and_strains(const SceneDesc *__restr
         // the named pass would discard lets the compiler emit a second copy
         // of this kernel without the density sums, whose other sums may
         // then round differently
-        const float value = poly6_density(rho.s, C.h2, C.h, C.mass);
+        const float value = rho.s * C.coef * C.mass;
         S.sdens[k] = value;
         if (with_density) {
             S.density[i] = value;
@@ -734,7 +731,7 @@ __global__ void __maxnreg__(64) k_rotations_and_strains(const SceneDesc *__restr
             auto pass2 = [&](unsigned kk) {
                 if (kk != k) pass2_masked(kk);
             };
-            if (overflow) for_each_neighbour(S, S.gridcell[i], pass2);
+            if (overflow) for_each_neighbour(S, S.srow[k].x, pass2);
             else for_each_masked<true>(S, k, rows, pass2_masked);
             float *st = S.strain + 6 * (size_t)i;
             st[0] = D[0];
@@ -768,7 +765,7 @@ __global__ void k_deformations(const SceneDesc *__restrict__ scenes, BlockMap ma
         const unsigned i = min(S.cellparticles[k], S.pnum - 1);
         const SolidConsts C = solid_consts(S);
         const float3 ipos = xyz(S.spos[k]), ipos0 = xyz(S.spos0[k]);
-        const StencilRows rows(S, S.gridcell[i]);
+        const StencilRows rows(S, S.srow[k]);
         float apq[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
         float aqq[6] = {0, 0, 0, 0, 0, 0};
         unsigned total = 0, count = 0;
@@ -790,7 +787,7 @@ __global__ void k_deformations(const SceneDesc *__restrict__ scenes, BlockMap ma
         // the named pass would discard lets the compiler emit a second copy
         // of this kernel without the density sums, whose other sums may
         // then round differently
-        const float value = poly6_density(rho.s, C.h2, C.h, C.mass);
+        const float value = rho.s * C.coef * C.mass;
         S.sdens[k] = value;
         if (with_density) {
             S.density[i] = value;
@@ -983,9 +980,9 @@ __global__ void __maxnreg__(80) k_forces_solids(const SceneDesc *__restrict__ sc
             solid_pair<COROT, true>(C, I, J, fe_s, fv_s);
         };
         if (MASKED && S.ncand[k] != SPH_NCAND_SCAN)
-            for_each_masked(S, k, StencilRows(S, S.gridcell[i]), visit_masked);
+            for_each_masked(S, k, StencilRows(S, S.srow[k]), visit_masked);
         else
-            for_each_neighbour(S, S.gridcell[i], visit);
+            for_each_neighbour(S, S.srow[k].x, visit);
         const float visc = *S.viscosity;
         const float3 fe = fe_s.get() * 0.5f, fv = fv_s.get() * visc;
         st3(S.force, i, fe + fv);

@@ -95,6 +95,10 @@ struct SceneDesc {
     // exceeds 64 and the force pass must scan
     unsigned *nbmask;
     unsigned *ncand;
+    // written by k_gather for the pair passes after it: per sorted particle
+    // (cell, StencilRows bits), and the scene's ScenePair constants
+    uint2 *srow;
+    float4 *pair_consts;
     // solids: cell-sorted copies for the fused substep's pair passes --
     // rest position (w: body_number bits), stress (6 floats, then
     // mass/density), rotation (3 rows of 4 floats); the velocity copy
@@ -137,6 +141,9 @@ struct RigidWork {
 // Candidate masks: two words for each of the 9 stencil rows.
 #define SPH_MASK_WORDS 18
 #define SPH_NCAND_SCAN 0xffffffffu
+
+// float4s of a scene's pair constants (kernels_common.cuh, ScenePair).
+#define SPH_PAIR_CONSTS 2
 
 // Block map entry: block b of a launch works on `scene`, items
 // [first, first + block size).

@@ -332,6 +332,8 @@ size_t sph_scratch_bytes(const SceneDesc &d) {
            + Arena::align(4)                 // status
            + Arena::align(4ull * SPH_MASK_WORDS * P)  // nbmask
            + Arena::align(4 * P)             // ncand
+           + Arena::align(8 * P)             // srow
+           + Arena::align(16 * SPH_PAIR_CONSTS)
            + Arena::align(4)                 // steps_left
            + solid_bytes(d)
            + rigid_bytes(d);
@@ -357,6 +359,10 @@ void sph_place_scratch(SceneDesc *d, char *base) {
     o += Arena::align(4ull * SPH_MASK_WORDS * P);
     d->ncand = reinterpret_cast<unsigned *>(base + o);
     o += Arena::align(4 * P);
+    d->srow = reinterpret_cast<uint2 *>(base + o);
+    o += Arena::align(8 * P);
+    d->pair_consts = reinterpret_cast<float4 *>(base + o);
+    o += Arena::align(16 * SPH_PAIR_CONSTS);
     d->steps_left = reinterpret_cast<unsigned *>(base + o);
     o += Arena::align(4);
     d->spos0 = d->sstress = d->srot = nullptr;
