@@ -15,20 +15,15 @@ static inline unsigned grid_for(const BlockMap &m, unsigned cap) {
 }
 
 cudaError_t sph_prepare_kernels() {
-    // the staged density pass may use more than the default 48 KB of
-    // dynamic shared memory for large pair blocks
-    int dev = 0, max_optin = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    size_t want = density_smem_bytes(1024);
-    if (max_optin > 0 && want > (size_t)max_optin) want = (size_t)max_optin;
-    cudaError_t e = cudaFuncSetAttribute(k_density<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)want);
+    // the density pass's staging buffers (may exceed the default limit)
+    const int want = (int)sizeof(DensityStage);
+    cudaError_t e = cudaFuncSetAttribute(k_density<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, want);
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_density<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)want);
+        e = cudaFuncSetAttribute(k_density<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, want);
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_density<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)want);
+        e = cudaFuncSetAttribute(k_density<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, want);
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_density<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)want);
+        e = cudaFuncSetAttribute(k_density<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, want);
     return e;
 }
 
@@ -85,7 +80,7 @@ void sph_launch_gather(const Launch &L, bool vel, bool dens, bool solid) {
 }
 
 void sph_launch_density(const Launch &L, bool original, bool mask, bool skip_solids, bool count) {
-    const size_t smem = density_smem_bytes(L.pair_block);
+    const size_t smem = sizeof(DensityStage);
     const unsigned g = grid_for(L.pair_particles, L.grid_cap);
     const int o = original ? 1 : 0, m = mask ? 1 : 0, sk = skip_solids ? 1 : 0;
     if (mask && count) {
@@ -99,7 +94,7 @@ void sph_launch_density(const Launch &L, bool original, bool mask, bool skip_sol
 }
 
 void sph_launch_density_fused(const Launch &L, const Launch *fluids) {
-    const size_t smem = density_smem_bytes(L.pair_block);
+    const size_t smem = sizeof(DensityStage);
     if (fluids && fluids->pair_particles.num)
         k_density<false><<<grid_for(fluids->pair_particles, L.grid_cap), L.pair_block, smem, L.stream>>>(
             L.scenes, fluids->pair_particles, 0, 1, 1);

@@ -19,12 +19,28 @@
 //
 // The stencil is walked as 9 rows (dz outer, dy inner, as the reference's
 // z, y, x loops): cells x-1..x+1 of one (z, y) row are one contiguous range
-// of the cell-sorted order.  Each warp stages its rows in shared memory:
-// for every row the union of its lanes' ranges is copied once with
-// coalesced float4 loads and each lane walks its own range there (lanes of
-// one cell read the same address: a broadcast).  Values, order and
-// arithmetic are those of a direct walk; a union wider than the buffer (a
-// warp that spans two grid rows) is read from global memory instead.
+// of the cell-sorted order.  A block stages the three rows of a z plane in
+// shared memory at a time: per row, the range its particles' rows lie in
+// (from its first and last particle's cell; the block's particles are
+// consecutive in the sort) goes into one array per coordinate, by
+// asynchronous copies that run while the plane before is worked on.
+// A lane then tests four consecutive candidates from three 16-byte loads
+// (lanes of one cell read the same address, a broadcast; the cells' ranges
+// start 8 floats apart, in different banks).
+// A row is taken in two steps:
+//   - near_bits tests 32 candidates without a branch, two per packed
+//     FP32x2 instruction, and collects the signs of r^2 - bound with one
+//     funnel shift per candidate.  Its bound lies 2^-20 above the exact one
+//     (and the smallest normal float, for radii whose squares underflow),
+//     more than the fused sum can differ from the rounded one, so no
+//     neighbour is missed;
+//   - the set bits (about 34 of 216 candidates) are walked in candidate
+//     order with the exact arithmetic of a direct walk: each adds its
+//     density term, and the few that are not within h lose their bit.
+// Values, order and arithmetic of the sums are those of a direct walk,
+// which a row takes whose range does not lie in the staged one (a plane's
+// ranges wider than the buffer, inconsistent host-written tables), or whose
+// particle lies within h of a symmetry plane.
 // The sum is blocked: each stencil row's terms are added in candidate
 // order, and the nine row sums with Kahan compensation (one compensated
 // add per row instead of per neighbour).
@@ -37,13 +53,53 @@
 // candidates; a row of more than 64 marks the particle for a scan
 // (ncand[k] = SPH_NCAND_SCAN).  The stores of one row are one coalesced
 // store per warp.
-// 128 float4s per warp hold a warp's row union (about 48 candidates in a
-// lattice); 256 measured the same and took twice the shared memory.
-#define SPH_STAGE 128
+// SPH_STAGE candidates hold a plane's ranges: about 440 for 128 particles
+// in a lattice of 8 per cell, 820 for 256.
+//
+// Bound: issue slots, 4,118 warp instructions per 32 particles at 1M (the
+// walk 1,411, near_bits 1,423, the rest row bounds, staging and masks)
+// against 5,001 for testing each candidate exactly as it comes, from rows
+// staged per warp: 160 -> 144 us at 1M particles (ncu), 1M-particle substep
+// 362 -> 349 us, mixed scene 519 -> 477 us.
+#define SPH_STAGE 896
 
-__host__ __device__ constexpr size_t density_smem_bytes(unsigned block) {
-    return sizeof(float4) * SPH_STAGE * (block / 32);
+// two buffers, and each row's staged range (first index, padded length)
+struct DensityStage {
+    float xyz[2][3 * SPH_STAGE];
+    uint2 range[9];
+};
+
+// Which of the staged candidates p .. p + 4 ng - 1 (16-byte aligned, ng
+// 1..8) may lie within the bound: candidate p + t at bit 31 - t.  nx, ny,
+// nz: the particle's negated coordinates; nb: the negated bound, each twice.
+// The differences are the exact test's; r^2 - bound is a chain of fused
+// multiply-adds (3 packed operations fewer).  A NaN has its sign clear.
+__device__ __forceinline__ unsigned near_bits(const float *__restrict__ p, unsigned ng, float2 nx, float2 ny, float2 nz,
+                                              float2 nb) {
+    unsigned acc = 0;
+#pragma unroll 1
+    for (unsigned g = 0; g < ng; ++g, p += 4) {
+        const float4 X = *reinterpret_cast<const float4 *>(p);
+        const float4 Y = *reinterpret_cast<const float4 *>(p + SPH_STAGE);
+        const float4 Z = *reinterpret_cast<const float4 *>(p + 2 * SPH_STAGE);
+        auto two = [&](float2 x, float2 y, float2 z) {
+            const float2 dx = __fadd2_rn(x, nx), dy = __fadd2_rn(y, ny), dz = __fadd2_rn(z, nz);
+            const float2 s = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __ffma2_rn(dx, dx, nb)));
+            acc = __funnelshift_l(__float_as_uint(s.x), acc, 1);
+            acc = __funnelshift_l(__float_as_uint(s.y), acc, 1);
+        };
+        two(make_float2(X.x, X.y), make_float2(Y.x, Y.y), make_float2(Z.x, Z.y));
+        two(make_float2(X.z, X.w), make_float2(Y.z, Y.w), make_float2(Z.z, Z.w));
+    }
+    return acc << (32u - 4u * ng);
 }
+
+// Asynchronous 4-byte copy from global to shared memory.
+__device__ __forceinline__ void copy_word_async(float *dst, const float *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // p = (rho - rho0) stiffness (fluids.cl:33-36), rounded as written.
 __device__ __forceinline__ float fluid_pressure(float rho, float rho0, float stiff) {
@@ -53,15 +109,39 @@ __device__ __forceinline__ float fluid_pressure(float rho, float rho0, float sti
 // COUNT: a masked pass that also counts num_neighbours (a named
 // compute_density, whose caller may read the count before the force pass).
 template <bool PLANES, bool MASK, bool COUNT = false>
-__device__ __forceinline__ void density_one(const SceneDesc &S, unsigned n, unsigned item, unsigned lane,
-                                            float4 *__restrict__ wstage, int original) {
-    const bool active = item < n;
-    const unsigned k = item;
-    const unsigned i = active ? min(S.cellparticles[k], S.pnum - 1) : 0u;
+__device__ __forceinline__ void density_block(const SceneDesc &S, unsigned n, unsigned first, DensityStage &stage,
+                                              int original) {
+    const unsigned k = first + threadIdx.x;
+    const bool active = k < n;
     const ScenePair B = scene_pair(S);
     const float h = B.h, h2 = B.h2;
-    const float3 ipos = active ? xyz(S.spos[k]) : make_float3(0.f, 0.f, 0.f);
+    const float4 *__restrict__ spos = S.spos;
+    const unsigned pnum = S.pnum;
+    const StencilRows rows(S, active ? S.srow[k] : make_uint2(0u, 0u));
+    if (threadIdx.x < 9u) {
+        // row r's ranges of the block's particles lie between its first
+        // particle's cell x-1 and its last one's x+1 (by cell index, so past
+        // an end of the grid's row they take in neighbouring rows too)
+        const int r = threadIdx.x;
+        const long long d = (long long)(r / 3 - 1) * rows.layer + (r % 3 - 1) * (long long)rows.R0;
+        const long long c0 = (long long)S.srow[first].x + d - 1,
+                        c1 = (long long)S.srow[min(first + blockDim.x, n) - 1u].x + d + 1;
+        const long long top = (long long)S.num_cells - 1;
+        unsigned b = 0, e = 0;
+        if (c1 >= 0 && c0 <= top) {
+            const unsigned x0 = (unsigned)(c0 < 0 ? 0 : c0), x1 = (unsigned)(c1 > top ? top : c1);
+            b = S.celloffset[x0];
+            e = min(S.celloffset[x1] + S.gridcount[x1], pnum);
+        }
+        const unsigned a = b & ~3u;
+        stage.range[r] = make_uint2(a, b < e ? (min(e - a, (unsigned)SPH_STAGE) + 3u) & ~3u : 0u);
+    }
+    const float3 ipos = active ? xyz(spos[k]) : make_float3(0.f, 0.f, 0.f);
     const NegPoint nip = neg_point(ipos);
+    const float2 nx = make_float2(-ipos.x, -ipos.x), ny = make_float2(-ipos.y, -ipos.y),
+                 nz = make_float2(-ipos.z, -ipos.z);
+    const float wide = __fmaf_rn(B.le, 1.f + 0x1p-20f, 0x1p-126f);
+    const float2 nb = make_float2(-wide, -wide);
     Planes P;
     if (PLANES) {
         load_planes(S, ipos, h, P);
@@ -70,77 +150,153 @@ __device__ __forceinline__ void density_one(const SceneDesc &S, unsigned n, unsi
     Kahan rho;
     unsigned count = 0, total = 0;
     bool overflow = false;
-    const StencilRows rows(S, active ? S.srow[k] : make_uint2(0u, 0u));
-    const float4 *__restrict__ spos = S.spos;
-#pragma unroll 1
-    for (int r = 0; r < 9; ++r) {
-        unsigned b = 0, e = 0;
-        if (active) rows.row(S, r, &b, &e);
-        const unsigned ub = __reduce_min_sync(SPH_FULL_MASK, b < e ? b : 0xffffffffu);
-        const unsigned ue = __reduce_max_sync(SPH_FULL_MASK, b < e ? e : 0u);
-        const bool staged = ub < ue && ue - ub <= SPH_STAGE;
-        if (staged) {
-            __syncwarp();
-            for (unsigned t = lane; t < ue - ub; t += 32) wstage[t] = spos[ub + t];
-            __syncwarp();
+    __syncthreads();
+    // where plane dz's rows start in its buffer; past SPH_STAGE: not staged
+    auto plane_at = [&](int dz, unsigned (&at)[4], unsigned (&ua)[3]) {
+        at[0] = 0;
+#pragma unroll
+        for (int dy = 0; dy < 3; ++dy) {
+            const uint2 g = stage.range[3 * dz + dy];
+            ua[dy] = g.x;
+            at[dy + 1] = at[dy] + g.y;
         }
-        const unsigned len = e - b;
-        // the row's mask in two words, each filled by its own loop below
-        // (a 32-bit shift per neighbour, no test of the candidate's place)
-        unsigned lo = 0, hi = 0;
-        // the row's density terms in candidate order; the row sums are
-        // added with Kahan compensation (blocked summation)
-        float rowsum = 0.f;
-        auto visit = [&](float4 j4, unsigned *word, unsigned bit) {
-            const float r2 = dist2(j4, nip);
-            if (r2 <= B.le) {
-                const float d = fmaxf(h2 - r2, 0.f);
-                rowsum = __fadd_rn(rowsum, d * d * d);
-                // a fused plane-free substep counts in the force pass
-                if (!MASK || PLANES || COUNT) count += r2 <= B.lt;
-                if (MASK && word) *word |= 1u << bit;
-            }
-            if (PLANES && P.imask) {
-                const float3 jpos = xyz(j4);
-                const unsigned jm = plane_jmask(P, jpos, h);
-                // subsets of jm in increasing order: the reference's
-                // plane_bits order restricted to the subsets it keeps
-                for (unsigned sb = (0u - jm) & jm; sb; sb = (sb - jm) & jm) {
-                    float3 ref = jpos;
-                    for (unsigned s2 = 0; s2 < P.count; ++s2)
-                        if (sb & (1u << s2)) ref = reflect3(ref, P.p[s2], P.n[s2]);
-                    const float m2 = norm2(sub3(ref, ipos));
-                    if (m2 <= B.lt) {
-                        const float d = fmaxf(h2 - m2, 0.f);
+    };
+    auto stage_plane = [&](int dz) {
+        unsigned at[4], ua[3];
+        plane_at(dz, at, ua);
+        if (at[3] > SPH_STAGE) return;
+        float *to = stage.xyz[dz & 1];
+#pragma unroll 1
+        for (unsigned t = threadIdx.x; t < at[3]; t += blockDim.x) {
+            const unsigned row0 = t < at[1] ? ua[0] : t < at[2] ? ua[1] - at[1] : ua[2] - at[2];
+            // up to three past the range: any value (capacity bounds it)
+            const float *p = reinterpret_cast<const float *>(spos + min(row0 + t, pnum - 1u));
+            copy_word_async(to + t, p);
+            copy_word_async(to + SPH_STAGE + t, p + 1);
+            copy_word_async(to + 2 * SPH_STAGE + t, p + 2);
+        }
+    };
+    // the exact walk over the staged candidates of a chunk's bits (candidate
+    // src + t at bit 31 - t), in order; returns the bits that are within h
+    auto walk = [&](unsigned m, const float *__restrict__ src, float &rowsum) {
+        unsigned hit = m;
+#pragma unroll 1
+        while (m) {
+            const unsigned t = __clz(m), bit = 0x80000000u >> t;
+            m ^= bit;
+            const float r2 = dist2(make_float4(src[t], src[SPH_STAGE + t], src[2 * SPH_STAGE + t], 0.f), nip);
+            // beyond h by a rounding: h2 - r2 <= 0 adds nothing
+            const float d = fmaxf(h2 - r2, 0.f);
+            rowsum = __fadd_rn(rowsum, d * d * d);
+            if (!MASK || PLANES || COUNT) count += r2 <= B.lt;
+            if (MASK && !(r2 <= B.le)) hit ^= bit;
+        }
+        return hit;
+    };
+    unsigned *mask = S.nbmask + k;
+    stage_plane(0);
+#pragma unroll 1
+    for (int dz = 0; dz < 3; ++dz) {
+        unsigned b[3], e[3], at[4], ua[3];
+#pragma unroll
+        for (int dy = 0; dy < 3; ++dy) {
+            b[dy] = e[dy] = 0;
+            if (active) rows.row(S, 3 * dz + dy, &b[dy], &e[dy]);
+        }
+        plane_at(dz, at, ua);
+        const bool fits = at[3] <= SPH_STAGE;
+        const float *buf = stage.xyz[dz & 1];
+        copies_wait();
+        __syncthreads();  // this plane is staged, and the other buffer is free
+        if (dz < 2) stage_plane(dz + 1);
+        // the plane's rows in turn: [0] of each array, which then moves up
+#pragma unroll 1
+        for (int dy = 0; dy < 3; ++dy) {
+            const unsigned len = e[0] - b[0];
+            // the row's mask in two words
+            unsigned lo = 0, hi = 0;
+            // the row's density terms in candidate order; the row sums are
+            // added with Kahan compensation (blocked summation)
+            float rowsum = 0.f;
+            // (an empty row takes the direct walk, of no candidate)
+            if (fits && b[0] - ua[0] < at[1] - at[0] && e[0] - ua[0] <= at[1] - at[0] && !(PLANES && P.imask)) {
+                // chunks of 32 candidates, from the row's start rounded down
+                // to a multiple of four: candidate c0 + t of the rounded row
+                // is bit 31 - t, and the first `o` belong to the cells before
+                const unsigned o = b[0] & 3u, tot = len ? o + len : 0u;
+                const float *src = buf + at[0] + (b[0] - o - ua[0]);
+                if (tot) {
+                    unsigned m = near_bits(src, min((tot + 3u) >> 2, 8u), nx, ny, nz, nb) & (0xffffffffu >> o);
+                    if (tot < 32u) m &= ~(0xffffffffu >> tot);
+                    m = walk(m, src, rowsum);
+                    if (MASK) lo = __brev(m) >> o;
+                }
+#pragma unroll 1
+                for (unsigned c0 = 32; c0 < tot; c0 += 32) {
+                    const unsigned rem = tot - c0;
+                    unsigned m = near_bits(src + c0, min((rem + 3u) >> 2, 8u), nx, ny, nz, nb);
+                    if (rem < 32u) m &= ~(0xffffffffu >> rem);
+                    m = walk(m, src + c0, rowsum);
+                    if (MASK && c0 < 96u) {
+                        // bit t of the row's mask is candidate b + t
+                        const unsigned long long w = (unsigned long long)__brev(m) << (32u - o);
+                        if (c0 == 32u) {
+                            lo |= (unsigned)w;
+                            hi = (unsigned)(w >> 32);
+                        } else {
+                            hi |= (unsigned)w;
+                        }
+                    }
+                }
+            } else {
+                // bits of `lo` for candidates [0, 32), of `hi` for [32, 64);
+                // a row longer than 64 (the later passes scan it) records
+                // none past 64
+#pragma unroll 1
+                for (unsigned t = 0; t < len; ++t) {
+                    const float4 j4 = spos[b[0] + t];
+                    const float r2 = dist2(j4, nip);
+                    if (r2 <= B.le) {
+                        const float d = fmaxf(h2 - r2, 0.f);
                         rowsum = __fadd_rn(rowsum, d * d * d);
-                        ++count;
+                        // a fused plane-free substep counts in the force pass
+                        if (!MASK || PLANES || COUNT) count += r2 <= B.lt;
+                        if (MASK && t < 32u) lo |= 1u << t;
+                        if (MASK && t >= 32u && t < 64u) hi |= 1u << (t - 32u);
+                    }
+                    if (PLANES && P.imask) {
+                        const float3 jpos = xyz(j4);
+                        const unsigned jm = plane_jmask(P, jpos, h);
+                        // subsets of jm in increasing order: the reference's
+                        // plane_bits order restricted to the subsets it keeps
+                        for (unsigned sb = (0u - jm) & jm; sb; sb = (sb - jm) & jm) {
+                            float3 ref = jpos;
+                            for (unsigned s2 = 0; s2 < P.count; ++s2)
+                                if (sb & (1u << s2)) ref = reflect3(ref, P.p[s2], P.n[s2]);
+                            const float m2 = norm2(sub3(ref, ipos));
+                            if (m2 <= B.lt) {
+                                const float d = fmaxf(h2 - m2, 0.f);
+                                rowsum = __fadd_rn(rowsum, d * d * d);
+                                ++count;
+                            }
+                        }
                     }
                 }
             }
-        };
-        // candidates [0, 32) set bits of `lo`, [32, 64) of `hi`; a row
-        // longer than 64 (the later passes scan it) records none past 64
-        const unsigned n1 = len < 32u ? len : 32u, n2 = len < 64u ? len : 64u;
-        if (staged) {
-            const float4 *src = wstage + (b - ub);
-#pragma unroll 4
-            for (unsigned t = 0; t < n1; ++t) visit(src[t], &lo, t);
-#pragma unroll 4
-            for (unsigned t = n1; t < n2; ++t) visit(src[t], &hi, t - 32u);
-            for (unsigned t = n2; t < len; ++t) visit(src[t], nullptr, 0u);
-        } else {
-            for (unsigned t = 0; t < n1; ++t) visit(spos[b + t], &lo, t);
-            for (unsigned t = n1; t < n2; ++t) visit(spos[b + t], &hi, t - 32u);
-            for (unsigned t = n2; t < len; ++t) visit(spos[b + t], nullptr, 0u);
-        }
-        rho.add(rowsum);
-        if (MASK && active) {
-            const unsigned long long bits = ((unsigned long long)hi << 32) | lo;
-            store_row_mask(S, k, r, len, bits);
-            overflow |= len > 64;
-            total += len;
+            rho.add(rowsum);
+            if (MASK && active) {
+                // store_row_mask's layout
+                mask[0] = lo;
+                if (len > 32u) mask[pnum] = hi;
+                mask += 2 * (size_t)pnum;
+                overflow |= len > 64;
+                total += len;
+            }
+            b[0] = b[1], e[0] = e[1], ua[0] = ua[1], at[0] = at[1], at[1] = at[2];
+            b[1] = b[2], e[1] = e[2], ua[1] = ua[2], at[2] = at[3];
         }
     }
+    const unsigned i = active ? min(S.cellparticles[k], pnum - 1) : 0u;
     if (active) {
         const float value = rho.s * B.coef * *S.mass;
         if (original) {
@@ -176,18 +332,20 @@ __device__ __forceinline__ void density_one(const SceneDesc &S, unsigned n, unsi
 template <bool PLANES, bool COUNT = false>
 __global__ void __launch_bounds__(512, 2)
     k_density(const SceneDesc *__restrict__ scenes, BlockMap map, int original, int want_mask, int skip_solids) {
-    extern __shared__ float4 sm_stage[];
-    float4 *wstage = sm_stage + (threadIdx.x >> 5) * SPH_STAGE;
-    const unsigned lane = threadIdx.x & 31u;
+    extern __shared__ __align__(16) unsigned char sm_stage[];
+    DensityStage &stage = *reinterpret_cast<DensityStage *>(sm_stage);
     SPH_FOR_WORK(map)
     if ((S.num_symmetry_planes != 0) != PLANES) continue;
     // in a fused substep a plane-free solid's first solid pass sums its density
     if (skip_solids && !PLANES && (S.programs & (PROG_COROT | PROG_SVK))) continue;
     const unsigned n = active_count(S);
+    const unsigned first = item - threadIdx.x;
+    if (first >= n) continue;
+    __syncthreads();  // the block's last entry is done with the buffers
     if (want_mask && S.nbmask && (S.programs & PROG_FLUIDS) && !original)
-        density_one<PLANES, true, COUNT>(S, n, item, lane, wstage, original);
+        density_block<PLANES, true, COUNT>(S, n, first, stage, original);
     else
-        density_one<PLANES, false>(S, n, item, lane, wstage, original);
+        density_block<PLANES, false>(S, n, first, stage, original);
     SPH_END_WORK
 }
 
