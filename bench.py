@@ -63,8 +63,8 @@ UNIT = "particle-steps/s"
 PHASE_BYTES = {
     "bin_count": (28, 4),             # find_particle_bins 16 + count 12; zero 4/cell
     "scan": (0, 16),                  # prefix_sum 8 + copy_celloffset_to_backup 8 per cell
-    "insert": (16, 0),                # insert_particles_in_bin_array
-    "gather": (0, 0),                 # no reference counterpart
+    # insert_particles_in_bin_array; the gather has no reference counterpart
+    "insert+gather": (16, 0),
     "density": (24, 8),               # compute_density + one stencil pass over the tables
     "forces_fluids+step": (120, 8),   # compute_forces_fluids 44 + step_forward 76
     # fused solid phases: the first pass also applies the stress law, the

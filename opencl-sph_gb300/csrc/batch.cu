@@ -154,8 +154,7 @@ bool solid_setup(sph_batch *b, BatchScene *sc) {
     L.stream = b->stream;
     L.no_symmetry_planes = sc->desc.num_symmetry_planes == 0;
     sph_launch_init_original_position(L);
-    sph_launch_bins(L);
-    sph_launch_gather(L, false, false);
+    sph_launch_bins_gather(L, false, false);
     sph_launch_density(L, true);
     bool good = sph_check_launch("sph_batch_add(setup)") == cudaSuccess;
     // the host copy must outlive the asynchronous upload
@@ -241,8 +240,7 @@ bool rebuild(sph_batch *b) {
     // branch per material present, joined back
     cudaGraph_t graph = nullptr;
     if (!ok(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal), "batch capture")) return false;
-    sph_launch_bins(A);
-    sph_launch_gather(A, true, false, true);
+    sph_launch_bins_gather(A, true, true);
     // masks for the fluid scenes only; the plane-free solid scenes' blocks
     // are not launched at all
     sph_launch_density_fused(A, b->group[MAT_FLUID].present ? &b->group[MAT_FLUID].L : nullptr);
@@ -939,10 +937,8 @@ extern "C" int sph_batch_profile(sph_batch *b, unsigned reps, float *phase_ms, c
         sph_launch_bin_count(A);
         log.mark("scan");
         sph_launch_scan(A, true);
-        log.mark("insert");
-        sph_launch_insert(A);
-        log.mark("gather");
-        sph_launch_gather(A, true, false, true);
+        log.mark("insert+gather");
+        sph_launch_insert(A, true, true, true);
         log.mark("density");
         sph_launch_density_fused(A, b->group[MAT_FLUID].present ? &b->group[MAT_FLUID].L : nullptr);
         for (int m = 0; m < 3; ++m) {

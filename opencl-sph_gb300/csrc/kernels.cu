@@ -51,16 +51,13 @@ void sph_launch_scan(const Launch &L, bool sums_ready) {
     k_scan_down<<<grid_for(L.scan, L.grid_cap), SPH_SCAN_THREADS, 0, L.stream>>>(L.scenes, L.scan);
 }
 
-void sph_launch_insert(const Launch &L) {
+void sph_launch_insert(const Launch &L, bool gather, bool vel, bool solid) {
     k_scatter<<<wide_grid(L.particles.num, L.grid_cap), L.block, 0, L.stream>>>(L.scenes, L.particles);
-    k_rank_cells<<<wide_grid(L.particles.num, L.grid_cap), L.block, 0, L.stream>>>(L.scenes, L.particles);
-    // crowded cells are rare: a few blocks per scene walk its queue
-    const unsigned gy = L.num_scenes < 65535u ? (L.num_scenes ? L.num_scenes : 1u) : 65535u;
-    // (a batch: 4 blocks of 256 per scene, most of which find no queue)
-    if (L.num_scenes > 1)
-        k_sort_big_cells<<<dim3(4, gy), 256, 0, L.stream>>>(L.scenes, L.num_scenes);
+    const unsigned g = grid_for(L.particles, L.grid_cap);
+    if (gather)
+        k_rank_cells<true><<<g, L.block, 0, L.stream>>>(L.scenes, L.particles, vel ? 1 : 0, solid ? 1 : 0);
     else
-        k_sort_big_cells<<<dim3(32, gy), 1024, 0, L.stream>>>(L.scenes, L.num_scenes);
+        k_rank_cells<false><<<g, L.block, 0, L.stream>>>(L.scenes, L.particles, 0, 0);
 }
 
 void sph_launch_bin_count(const Launch &L) {
@@ -72,6 +69,12 @@ void sph_launch_bins(const Launch &L) {
     sph_launch_bin_count(L);
     sph_launch_scan(L, true);
     sph_launch_insert(L);
+}
+
+void sph_launch_bins_gather(const Launch &L, bool vel, bool solid) {
+    sph_launch_bin_count(L);
+    sph_launch_scan(L, true);
+    sph_launch_insert(L, true, vel, solid);
 }
 
 void sph_launch_gather(const Launch &L, bool vel, bool dens, bool solid) {
@@ -249,14 +252,12 @@ void sph_launch_substep(const Launch &L, SphMaterial mat, PhaseMark mark, void *
     sph_launch_bin_count(L);
     phase("scan");
     sph_launch_scan(L, true);
-    phase("insert");
-    sph_launch_insert(L);
+    phase("insert+gather");
+    sph_launch_insert(L, true, mat == MAT_FLUID || mat == MAT_MIXED, mat != MAT_FLUID);
     if (mat == MAT_MIXED) {
         // fluid and solid particles in one scene (extension): the fluid
         // recipe, with the solids' elastic passes before the force pass,
         // which adds the fluid-solid pair terms and steps every particle
-        phase("gather");
-        sph_launch_gather(L, true, false, true);
         phase("density");
         sph_launch_density(L, false, true, false);
         phase("deformations (solid phase)");
@@ -274,8 +275,6 @@ void sph_launch_substep(const Launch &L, SphMaterial mat, PhaseMark mark, void *
         phase(nullptr);
         return;
     }
-    phase("gather");
-    sph_launch_gather(L, mat == MAT_FLUID, false, mat != MAT_FLUID);
     if (mat == MAT_FLUID || !L.no_symmetry_planes) {
         // a plane-free solid's density is summed by its first solid pass
         phase("density");

@@ -1,5 +1,5 @@
 // kernels_grid.cuh -- neighbour grid on sm_103a: cell hash, counting sort
-// with warp-aggregated atomics, segmented exclusive scan, scatter and a
+// with one atomic per particle, segmented exclusive scan, scatter and a
 // deterministic per-cell order (ascending particle index), plus the gathers
 // that build the cell-sorted float4 copies the pair kernels stream.
 //
@@ -13,11 +13,11 @@
 
 #include "kernels_common.cuh"
 
-// The scatter and the per-cell ranking are chains of dependent loads (work
-// entry -> scene -> gridcell -> celloffset -> the cell's entries), so each
-// of their blocks takes SPH_WIDE consecutive work entries per pass and runs
-// their chains side by side: the loads of all entries are issued before any
-// result is used, and a launch needs a quarter of the blocks.
+// The scatter is a chain of dependent loads (work entry -> scene -> gridcell
+// -> celloffset), so each of its blocks takes SPH_WIDE consecutive work
+// entries per pass and runs their chains side by side: the loads of all
+// entries are issued before any result is used, and a launch needs a quarter
+// of the blocks.
 #define SPH_WIDE 4
 
 struct WideItem {
@@ -83,40 +83,51 @@ __device__ __forceinline__ unsigned cell_of(const SceneDesc &S, float3 p, bool *
 }
 
 // find_particle_bins (common.cl:372-391) fused with count_particles_in_bins
-// (:401-408).  Lanes of a warp that hit the same cell combine into one
-// atomicAdd; each particle keeps its arrival slot within the cell.  (One
-// work entry per block: the wide form measured slower here.)
+// (:401-408).  Each particle keeps its arrival slot within the cell, from
+// one atomic per particle: a chain of dependent accesses bounds the pass,
+// not the counts' atomics in L2, and combining a warp's lanes by cell first
+// with a match instruction took longer than the atomics it saved.  The scan
+// tiles' totals are counted in shared memory first: a few dozen tiles hold
+// a scene of 100,000 particles, and once these are no longer in cell order
+// every lane's atomic went to one of those few words (with the zeroing 29 ->
+// 16 us, and 30 -> 23 us for 1M particles in order).  Looking the totals up
+// in the scan instead, tile by tile, took its time from 8 to 14 us.  A grid
+// of more than SPH_BIN_TILES tiles spreads them enough to add directly.
+// (One work entry per block: the wide form measured slower here.)
+#define SPH_BIN_TILES 512
 __global__ void k_bin_count(const SceneDesc *__restrict__ scenes, BlockMap map, int do_count) {
+    __shared__ unsigned tiles[SPH_BIN_TILES];
     SPH_FOR_WORK(map)
     const unsigned n = active_count(S);
-    const bool valid = item < n;
-    const unsigned lanes = __ballot_sync(SPH_FULL_MASK, valid);
-    if (valid) {
+    if (item - threadIdx.x >= n) continue;
+    const unsigned few = do_count && S.num_scan_blocks <= SPH_BIN_TILES ? S.num_scan_blocks : 0u;
+    if (few) {
+        for (unsigned t = threadIdx.x; t < few; t += blockDim.x) tiles[t] = 0u;
+        __syncthreads();
+    }
+    if (item < n) {
         bool outside;
         const unsigned cell = cell_of(S, ld3(S.position, item), &outside);
+        if (do_count) {
+            if (few) atomicAdd(tiles + cell / SPH_SCAN_TILE, 1u);
+            else atomicAdd(S.scan_sums + cell / SPH_SCAN_TILE, 1u);
+            S.slot[item] = atomicAdd(S.gridcount + cell, 1u);
+        }
         S.gridcell[item] = cell;
         if (outside) atomicOr(S.status, (unsigned)STATUS_OUTSIDE_GRID);
-        if (do_count) {
-            const unsigned peers = __match_any_sync(lanes, cell);
-            const unsigned lane = threadIdx.x & 31u;
-            const unsigned leader = __ffs(peers) - 1;
-            unsigned base = 0;
-            if (lane == leader) base = atomicAdd(S.gridcount + cell, (unsigned)__popc(peers));
-            base = __shfl_sync(peers, base, leader);
-            S.slot[item] = base + __popc(peers & ((1u << lane) - 1u));
-            // the scan tile's total (k_scan_down reads these)
-            const unsigned tile = cell / SPH_SCAN_TILE;
-            const unsigned tpeers = __match_any_sync(lanes, tile);
-            if (lane == (unsigned)(__ffs(tpeers) - 1)) atomicAdd(S.scan_sums + tile, (unsigned)__popc(tpeers));
-        }
+    }
+    if (few) {
+        __syncthreads();
+        for (unsigned t = threadIdx.x; t < few; t += blockDim.x)
+            if (tiles[t]) atomicAdd(S.scan_sums + t, tiles[t]);
+        __syncthreads();  // the next entry clears them
     }
     SPH_END_WORK
 }
 
 // zero_gridcount (common.cl:392-400) for every scene of the launch, one
-// block per scan tile of SPH_SCAN_TILE cells: the counts, the tile's total
-// (which k_bin_count accumulates) and, once per scene, the crowded-cell
-// queue counter.
+// block per scan tile of SPH_SCAN_TILE cells: the counts and the tile's
+// total (which k_bin_count accumulates).
 __global__ void __launch_bounds__(SPH_SCAN_THREADS) k_zero_cells(const SceneDesc *__restrict__ scenes, BlockMap map) {
     for (unsigned vb = blockIdx.x; vb < map.num; vb += gridDim.x) {
         const BlockWork bw = map.work[vb];
@@ -124,10 +135,7 @@ __global__ void __launch_bounds__(SPH_SCAN_THREADS) k_zero_cells(const SceneDesc
         if (scene_idle(S)) continue;
         const unsigned end = min(bw.first + SPH_SCAN_TILE, S.num_cells);
         for (unsigned c = bw.first + threadIdx.x; c < end; c += blockDim.x) S.gridcount[c] = 0u;
-        if (threadIdx.x == 0) {
-            S.scan_sums[bw.first / SPH_SCAN_TILE] = 0u;
-            if (bw.first == 0) S.big_cells[0] = 0u;
-        }
+        if (threadIdx.x == 0) S.scan_sums[bw.first / SPH_SCAN_TILE] = 0u;
     }
 }
 
@@ -135,19 +143,10 @@ __global__ void __launch_bounds__(SPH_SCAN_THREADS) k_zero_cells(const SceneDesc
 // kernels one by one (gridcell already computed).
 __global__ void k_count_only(const SceneDesc *__restrict__ scenes, BlockMap map) {
     SPH_FOR_WORK(map)
-    const unsigned n = active_count(S);
-    const bool valid = item < n;
-    const unsigned lanes = __ballot_sync(SPH_FULL_MASK, valid);
-    if (valid) {
+    if (item < active_count(S)) {
         unsigned cell = S.gridcell[item];
         if (cell >= S.num_cells) cell = S.num_cells - 1;  // host-written garbage
-        const unsigned peers = __match_any_sync(lanes, cell);
-        const unsigned lane = threadIdx.x & 31u;
-        const unsigned leader = __ffs(peers) - 1;
-        unsigned base = 0;
-        if (lane == leader) base = atomicAdd(S.gridcount + cell, (unsigned)__popc(peers));
-        base = __shfl_sync(peers, base, leader);
-        S.slot[item] = base + __popc(peers & ((1u << lane) - 1u));
+        S.slot[item] = atomicAdd(S.gridcount + cell, 1u);
     }
     SPH_END_WORK
 }
@@ -239,11 +238,8 @@ __global__ void __launch_bounds__(SPH_SCAN_THREADS) k_scan_down(const SceneDesc 
 }
 
 // insert_particles_in_bin_array (common.cl:523-529) without atomics: each
-// particle goes to celloffset[cell] + its arrival slot, in arrival order,
-// of an unsorted copy of cellparticles: the first pnum words of the sorted
-// position buffer, which is free until the gather.
-__device__ __forceinline__ unsigned *unsorted_cells(const SceneDesc &S) { return reinterpret_cast<unsigned *>(S.spos); }
-
+// particle and its cell go to place celloffset[cell] + its arrival slot, in
+// arrival order, of the scene's unsorted list.
 __global__ void k_scatter(const SceneDesc *__restrict__ scenes, BlockMap map) {
     SPH_FOR_WIDE(map)
     unsigned cell[SPH_WIDE], slot[SPH_WIDE];
@@ -264,132 +260,82 @@ __global__ void k_scatter(const SceneDesc *__restrict__ scenes, BlockMap map) {
         if (off[j] != 0xffffffffu) {
             const SceneDesc &S = *W[j].S;
             const unsigned dst = off[j] + slot[j];
-            if (dst < S.pnum) unsorted_cells(S)[dst] = W[j].item;
+            if (dst < S.pnum) {
+                S.unsorted[dst] = W[j].item;
+                S.unsorted[S.pnum + dst] = cell[j];
+            }
         }
     SPH_END_WIDE
+}
+
+// Cell-sorted copies of particle i at place k: spos = position (and velocity,
+// density when asked; for solids also the rest position with the body
+// number -- and in a mixed scene SPH_SOLID_PHASE_BIT for a solid-phase
+// particle -- and 1/density0 in the velocity copy's w), so that the pair
+// loops stream float4s.  Also what every pair pass would otherwise work out
+// again in each thread, while this memory-bound work leaves issue slots to
+// spare: the particle's stencil rows (srow) and the scene's constants
+// (write_scene_pair).
+__device__ __forceinline__ void gather_one(const SceneDesc &S, unsigned k, unsigned i, unsigned cell, int with_vel,
+                                           int with_dens, int with_solid) {
+    const float3 p = ld3(S.position, i);
+    const bool solid = with_solid && S.spos0;
+    float3 v = make_float3(0.f, 0.f, 0.f);
+    if (with_vel || solid) v = ld3(S.velocity, i);
+    S.spos[k] = make_float4(p.x, p.y, p.z, 0.f);
+    S.srow[k] = make_uint2(cell, StencilRows(S, cell).bits);
+    if (k == 0) write_scene_pair(S);
+    if (with_vel || solid) S.svel[k] = make_float4(v.x, v.y, v.z, solid ? __frcp_rn(S.density0[i]) : 0.f);
+    if (with_dens) S.sdens[k] = S.density[i];
+    if (solid) {
+        // rest position, and the body number's bits in w
+        const float3 p0 = ld3(S.originalpos, i);
+        unsigned w = S.body_number[i];
+        if (S.phase && S.phase[i]) w |= SPH_SOLID_PHASE_BIT;
+        S.spos0[k] = make_float4(p0.x, p0.y, p0.z, __uint_as_float(w));
+    }
 }
 
 // Canonical order inside each cell: ascending particle index.  One thread
-// per slot of the unsorted copy: its particle's place in the cell is the
-// number of the cell's particles with a smaller index.  Cells of more than
-// SPH_SMALL_CELL particles are copied as they are and queued (by the thread
-// of their first slot) for k_sort_big_cells.
-__global__ void k_rank_cells(const SceneDesc *__restrict__ scenes, BlockMap map) {
-    SPH_FOR_WIDE(map)
-    unsigned x[SPH_WIDE], cell[SPH_WIDE];
-#pragma unroll
-    for (int j = 0; j < SPH_WIDE; ++j) x[j] = W[j].valid ? unsorted_cells(*W[j].S)[W[j].item] : 0xffffffffu;
-#pragma unroll
-    for (int j = 0; j < SPH_WIDE; ++j)
-        cell[j] = W[j].valid && x[j] < W[j].S->pnum ? W[j].S->gridcell[x[j]] : 0xffffffffu;
-    unsigned off[SPH_WIDE], cnt[SPH_WIDE];
-#pragma unroll
-    for (int j = 0; j < SPH_WIDE; ++j) {
-        off[j] = 0u;
-        cnt[j] = 0u;
-        if (W[j].valid && cell[j] < W[j].S->num_cells) {
-            off[j] = W[j].S->celloffset[cell[j]];
-            cnt[j] = W[j].S->gridcount[cell[j]];
-        }
-    }
-#pragma unroll
-    for (int j = 0; j < SPH_WIDE; ++j) {
-        const unsigned item = W[j].item;
+// per entry of the unsorted list: its particle's place in the cell is the
+// number of the cell's particles with a smaller index.  (In a cell of m
+// particles that takes m^2 comparisons; the pair passes test each of them
+// against all others at many times that cost.)  GATHER: a substep, where
+// nothing changes between the order and the pair passes; the particle's
+// sorted copies are written here too.  Bound: latency of the chain entry ->
+// table -> the cell's entries and fields -> stores.  With the scatter 47 ->
+// 33 us at 1M particles, against an order, a sort of crowded cells and a
+// gather in launches of their own (four launches; a 1,000-particle substep
+// 59 -> 55 us).
+template <bool GATHER>
+__global__ void k_rank_cells(const SceneDesc *__restrict__ scenes, BlockMap map, int with_vel, int with_solid) {
+    SPH_FOR_WORK(map)
+    if (item < active_count(S)) {
+        const unsigned x = S.unsorted[item], cell = S.unsorted[S.pnum + item];
         // inconsistent tables come only from host-written garbage: skip
-        if (cnt[j] && off[j] <= item && item - off[j] < cnt[j] && cnt[j] <= W[j].S->pnum - off[j]) {
-            const SceneDesc &S = *W[j].S;
-            if (cnt[j] > SPH_SMALL_CELL) {
-                S.cellparticles[item] = x[j];
-                if (item == off[j]) {
-                    const unsigned k = atomicAdd(S.big_cells, 1u);
-                    S.big_cells[1 + k] = cell[j];
-                }
-            } else {
-                const unsigned *U = unsorted_cells(S) + off[j];
-                unsigned r = 0;
-                for (unsigned a2 = 0; a2 < cnt[j]; ++a2) r += U[a2] < x[j];
-                S.cellparticles[off[j] + r] = x[j];
-            }
-        }
-    }
-    SPH_END_WIDE
-}
-
-// Fallback for crowded cells (e.g. particles clamped into an edge cell):
-// one block bitonic-sorts each queued cell, padded to a power of two, in a
-// scratch region of the sorted-position buffer ([2*off, 2*off + L) of its
-// words, which cannot overlap another cell's region since L < 2*count).
-// grid (blocks per scene, scenes): blockIdx.y is the scene, so a batch of
-// many scenes without crowded cells costs one load per block.
-__global__ void __launch_bounds__(1024) k_sort_big_cells(const SceneDesc *__restrict__ scenes, unsigned num_scenes) {
-    for (unsigned s = blockIdx.y; s < num_scenes; s += gridDim.y) {
-        const SceneDesc &S = scenes[s];
-        if (scene_idle(S)) continue;
-        const unsigned nbig = S.big_cells[0];
-        for (unsigned b = blockIdx.x; b < nbig; b += gridDim.x) {
-            const unsigned cell = S.big_cells[1 + b];
+        if (x < S.pnum && cell < S.num_cells) {
             const unsigned off = S.celloffset[cell], cnt = S.gridcount[cell];
-            if (off > S.pnum || cnt > S.pnum - off) continue;
-            unsigned L = 1;
-            while (L < cnt) L <<= 1;
-            unsigned *buf = reinterpret_cast<unsigned *>(S.spos) + 2u * off;
-            unsigned *seg = S.cellparticles + off;
-            for (unsigned t = threadIdx.x; t < L; t += blockDim.x) buf[t] = t < cnt ? seg[t] : 0xffffffffu;
-            __syncthreads();
-            for (unsigned k = 2; k <= L; k <<= 1) {
-                for (unsigned j = k >> 1; j > 0; j >>= 1) {
-                    for (unsigned t = threadIdx.x; t < L; t += blockDim.x) {
-                        unsigned u = t ^ j;
-                        if (u > t) {
-                            unsigned a = buf[t], c = buf[u];
-                            bool up = (t & k) == 0;
-                            if ((a > c) == up) {
-                                buf[t] = c;
-                                buf[u] = a;
-                            }
-                        }
-                    }
-                    __syncthreads();
-                }
+            if (off <= item && item - off < cnt && cnt <= S.pnum - off) {
+                const unsigned *U = S.unsorted + off;
+                unsigned r = off;
+#pragma unroll 4
+                for (unsigned a = 0; a < cnt; ++a) r += U[a] < x;
+                S.cellparticles[r] = x;
+                if (GATHER) gather_one(S, r, x, cell, with_vel, 0, with_solid);
             }
-            for (unsigned t = threadIdx.x; t < cnt; t += blockDim.x) seg[t] = buf[t];
-            __syncthreads();
         }
     }
+    SPH_END_WORK
 }
 
-// Cell-sorted copies: spos[k] = position[cellparticles[k]] (and velocity,
-// density when asked; for solids also the rest position with the body
-// number -- and in a mixed scene SPH_SOLID_PHASE_BIT for a solid-phase
-// particle -- and 1/density0 in the velocity copy's w).  Gathers once so
-// the pair loops stream float4s.  It also writes what every pair pass would
-// otherwise work out again in each thread, while this memory-bound kernel
-// has issue slots to spare: the particle's stencil rows (srow) and the
-// scene's constants (write_scene_pair).
+// The sorted copies from the fields, for pair kernels called by name.
 __global__ void k_gather(const SceneDesc *__restrict__ scenes, BlockMap map, int with_vel, int with_dens,
                          int with_solid) {
     SPH_FOR_WORK(map)
     if (item < active_count(S)) {
         unsigned i = S.cellparticles[item];
         if (i >= S.pnum) i = 0;  // host-written garbage
-        float3 p = ld3(S.position, i);
-        S.spos[item] = make_float4(p.x, p.y, p.z, 0.f);
-        const unsigned cell = S.gridcell[i];
-        S.srow[item] = make_uint2(cell, StencilRows(S, cell).bits);
-        if (item == 0) write_scene_pair(S);
-        const bool solid = with_solid && S.spos0;
-        if (with_vel || solid) {
-            float3 v = ld3(S.velocity, i);
-            S.svel[item] = make_float4(v.x, v.y, v.z, solid ? __frcp_rn(S.density0[i]) : 0.f);
-        }
-        if (with_dens) S.sdens[item] = S.density[i];
-        if (solid) {
-            // rest position, and the body number's bits in w
-            const float3 p0 = ld3(S.originalpos, i);
-            unsigned w = S.body_number[i];
-            if (S.phase && S.phase[i]) w |= SPH_SOLID_PHASE_BIT;
-            S.spos0[item] = make_float4(p0.x, p0.y, p0.z, __uint_as_float(w));
-        }
+        gather_one(S, item, i, S.gridcell[i], with_vel, with_dens, with_solid);
     }
     SPH_END_WORK
 }

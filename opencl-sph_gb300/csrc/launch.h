@@ -47,12 +47,16 @@ void sph_launch_count(const Launch &L);
 // sums_ready: k_bin_count has added up the tiles' totals (a fused binning);
 // otherwise a pass over the counts does (prefix_sum called by name)
 void sph_launch_scan(const Launch &L, bool sums_ready = false);
-void sph_launch_insert(const Launch &L);  // scatter + per-cell ordering
+// scatter + per-cell ordering; gather: the sorted copies too (vel: with
+// velocities, solid: with the solids' fields)
+void sph_launch_insert(const Launch &L, bool gather = false, bool vel = false, bool solid = false);
 // zero_gridcount + find_particle_bins + count_particles_in_bins in one
 // pass, recording each particle's arrival slot
 void sph_launch_bin_count(const Launch &L);
 // All of compute_particle_bins: zero, bin+count, scan, insert.
 void sph_launch_bins(const Launch &L);
+// The same with the sorted copies (a substep, or a solid's set-up).
+void sph_launch_bins_gather(const Launch &L, bool vel, bool solid);
 // Cell-sorted copies (positions; velocities and densities on request).
 void sph_launch_gather(const Launch &L, bool vel, bool dens, bool solid = false);
 

@@ -2,8 +2,8 @@
 // that cannot allocate device memory.
 //
 // The store path (create_psdata_cuda) owns its scratch: per-particle arrival
-// slots, scan partial sums, the crowded-cell queue and the buffer the
-// crowded-cell sort works in, all carved from one cudaMalloc.  Some callers
+// slots, scan partial sums and the arrival-order list, all carved from one
+// cudaMalloc.  Some callers
 // cannot make that allocation:
 //   - engines and plugin hosts that own all device memory through their
 //     own pool and forbid other allocations in their frame loop;
@@ -35,16 +35,14 @@ constexpr unsigned kBlock = 256;
 constexpr size_t kMaxParticles = SPH_NOALLOC_MAX_PARTICLES;
 constexpr size_t kMaxCells = SPH_NOALLOC_MAX_CELLS;
 constexpr size_t kMaxScanTiles = kMaxCells / SPH_SCAN_TILE;
-constexpr size_t kMaxBig = kMaxParticles / (SPH_SMALL_CELL + 1) + 2;
 
 constexpr size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 // Layout of the scratch array (byte offsets).
 constexpr size_t kSlot = 0;                                                    // u32[n]
-constexpr size_t kSortBuf = kSlot + align256(4 * kMaxParticles);               // u32[2n], crowded-cell sort
-constexpr size_t kScan = kSortBuf + align256(8 * kMaxParticles);               // u32[tiles]
-constexpr size_t kBig = kScan + align256(4 * kMaxScanTiles);                   // u32[1 + queue]
-constexpr size_t kN = kBig + align256(4 * kMaxBig);                            // u32 n
+constexpr size_t kUnsorted = kSlot + align256(4 * kMaxParticles);              // u32[2n], arrival order
+constexpr size_t kScan = kUnsorted + align256(8 * kMaxParticles);              // u32[tiles]
+constexpr size_t kN = kScan + align256(4 * kMaxScanTiles);                     // u32 n
 constexpr size_t kStatus = kN + 256;                                           // u32 status
 constexpr size_t kDesc = kStatus + 256;                                        // SceneDesc
 constexpr size_t kPMap = kDesc + align256(sizeof(SceneDesc));                  // BlockWork per 256 particles
@@ -155,10 +153,9 @@ extern "C" int sph_compute_particle_bins_noalloc(const float *position, unsigned
     d.num_cells = (unsigned)cells;
     d.programs = PROG_COMMON;
     d.slot = reinterpret_cast<unsigned *>(base + kSlot);
-    d.spos = reinterpret_cast<float4 *>(base + kSortBuf);
+    d.unsorted = reinterpret_cast<unsigned *>(base + kUnsorted);
     d.scan_sums = reinterpret_cast<unsigned *>(base + kScan);
     d.num_scan_blocks = (unsigned)((cells + SPH_SCAN_TILE - 1) / SPH_SCAN_TILE);
-    d.big_cells = reinterpret_cast<unsigned *>(base + kBig);
     d.status = reinterpret_cast<unsigned *>(base + kStatus);
     k_noalloc_setup<<<64, 256, 0, s>>>(base, d, n);
 

@@ -33,10 +33,6 @@ enum SphStatus : unsigned {
     STATUS_OUTSIDE_GRID = 1u << 1,    // a particle was binned outside gridbounds
 };
 
-// Cells with more particles than this are ordered by the block-wide
-// fallback sort instead of the per-cell insertion sort.
-#define SPH_SMALL_CELL 32
-
 // ---- one scene on the device ----------------------------------------------
 //
 // Pointers into the scene's device copy of its psdata blob (fields the
@@ -85,7 +81,10 @@ struct SceneDesc {
     float *sdens;             // cell-sorted densities
     unsigned *scan_sums;      // this scene's scan partial sums
     unsigned num_scan_blocks;
-    unsigned *big_cells;      // [0] = count, [1..] = cells above SPH_SMALL_CELL
+    // particles in arrival order within their cells (pnum words), and their
+    // cells (pnum words): between the scatter and the per-cell ranking, in
+    // the memory of the candidate masks, which are recorded later
+    unsigned *unsorted;
     unsigned *status;         // SphStatus bits
     // candidate masks (fluids, fused substep): bit t of stencil row r's
     // 64-bit mask of sorted particle k is set when the row's t-th candidate

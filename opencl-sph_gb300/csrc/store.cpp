@@ -328,7 +328,6 @@ size_t sph_scratch_bytes(const SceneDesc &d) {
            + Arena::align(16 * P)            // svel
            + Arena::align(4 * P)             // sdens
            + Arena::align(4ull * d.num_scan_blocks)
-           + Arena::align(4ull * (d.num_cells + 1))
            + Arena::align(4)                 // status
            + Arena::align(4ull * SPH_MASK_WORDS * P)  // nbmask
            + Arena::align(4 * P)             // ncand
@@ -351,11 +350,9 @@ void sph_place_scratch(SceneDesc *d, char *base) {
     o += Arena::align(4 * P);
     d->scan_sums = reinterpret_cast<unsigned *>(base + o);
     o += Arena::align(4ull * d->num_scan_blocks);
-    d->big_cells = reinterpret_cast<unsigned *>(base + o);
-    o += Arena::align(4ull * (d->num_cells + 1));
     d->status = reinterpret_cast<unsigned *>(base + o);
     o += Arena::align(4);
-    d->nbmask = reinterpret_cast<unsigned *>(base + o);
+    d->nbmask = d->unsorted = reinterpret_cast<unsigned *>(base + o);
     o += Arena::align(4ull * SPH_MASK_WORDS * P);
     d->ncand = reinterpret_cast<unsigned *>(base + o);
     o += Arena::align(4 * P);
