@@ -65,6 +65,7 @@ PHASE_BYTES = {
     "scan": (0, 16),                  # prefix_sum 8 + copy_celloffset_to_backup 8 per cell
     # insert_particles_in_bin_array; the gather has no reference counterpart
     "insert+gather": (16, 0),
+    "grid": (44, 20),                 # the three above, one launch (small scenes)
     "density": (24, 8),               # compute_density + one stencil pass over the tables
     "forces_fluids+step": (120, 8),   # compute_forces_fluids 44 + step_forward 76
     # fused solid phases: the first pass also applies the stress law, the

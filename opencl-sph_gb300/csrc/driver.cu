@@ -294,6 +294,7 @@ Store *create_store(psdata *data, const char *file_list, std::string *err) {
     L.no_symmetry_planes = s->desc.num_symmetry_planes == 0;
     L.has_mixed = s->desc.phase != nullptr;
     L.all_mixed = L.has_mixed;  // one scene per store
+    L.small_grid = sph_small_grid(s->desc.pnum, s->desc.num_cells);
     L.rigid = s->d_rigid;
     L.num_rigid = 0;
     if (!refresh_rigid(s, *data)) {

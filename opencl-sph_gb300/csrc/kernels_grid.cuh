@@ -11,6 +11,8 @@
 // atomic race order).
 #pragma once
 
+#include <cooperative_groups.h>
+
 #include "kernels_common.cuh"
 
 // The scatter is a chain of dependent loads (work entry -> scene -> gridcell
@@ -338,4 +340,88 @@ __global__ void k_gather(const SceneDesc *__restrict__ scenes, BlockMap map, int
         gather_one(S, item, i, S.gridcell[i], with_vel, with_dens, with_solid);
     }
     SPH_END_WORK
+}
+
+// ---- a small scene's grid in one launch -----------------------------------------
+//
+// compute_particle_bins, and with GATHER the sorted copies, of one scene by
+// one thread-block cluster: the phases that are launches of their own for a
+// large scene, with a cluster barrier (hardware, no spinning) between them.
+// A small scene's launches are bound by latency: each starts blocks, reads
+// its work entry and scene and waits for a chain or two of dependent
+// accesses, and the next starts only then.
+// A thread keeps its particles' cells and slots in registers, up to
+// SPH_SMALL_ITEMS of them.
+#define SPH_SMALL_BLOCKS 8
+#define SPH_SMALL_THREADS 512
+#define SPH_SMALL_ITEMS 4
+#define SPH_SMALL_PARTICLES (SPH_SMALL_BLOCKS * SPH_SMALL_THREADS * SPH_SMALL_ITEMS)
+#define SPH_SMALL_CELLS 65536
+
+template <bool GATHER>
+__global__ void __launch_bounds__(SPH_SMALL_THREADS) k_grid_small(const SceneDesc *__restrict__ scenes, int with_vel,
+                                                                  int with_solid) {
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    __shared__ unsigned totals[SPH_SMALL_BLOCKS];
+    const SceneDesc &S = scenes[0];
+    if (scene_idle(S)) return;
+    constexpr unsigned threads = SPH_SMALL_BLOCKS * SPH_SMALL_THREADS;
+    const unsigned rank = cluster.block_rank(), me = rank * SPH_SMALL_THREADS + threadIdx.x;
+    const unsigned n = active_count(S), cells = S.num_cells;
+    for (unsigned c = me; c < cells; c += threads) S.gridcount[c] = 0u;
+    unsigned cell[SPH_SMALL_ITEMS], slot[SPH_SMALL_ITEMS];
+#pragma unroll
+    for (int j = 0; j < SPH_SMALL_ITEMS; ++j) {
+        const unsigned i = me + j * threads;
+        if (i < n) {
+            bool outside;
+            cell[j] = cell_of(S, ld3(S.position, i), &outside);
+            S.gridcell[i] = cell[j];
+            if (outside) atomicOr(S.status, (unsigned)STATUS_OUTSIDE_GRID);
+        }
+    }
+    cluster.sync();  // the counts are zero
+#pragma unroll
+    for (int j = 0; j < SPH_SMALL_ITEMS; ++j)
+        if (me + j * threads < n) slot[j] = atomicAdd(S.gridcount + cell[j], 1u);
+    cluster.sync();  // the counts are final
+    // the scan: a block takes a range of cells, a thread a run of it
+    const unsigned share = (cells + SPH_SMALL_BLOCKS - 1) / SPH_SMALL_BLOCKS;
+    const unsigned run = (share + SPH_SMALL_THREADS - 1) / SPH_SMALL_THREADS;
+    const unsigned end = min(cells, (rank + 1) * share);
+    const unsigned c0 = min(end, rank * share + threadIdx.x * run), c1 = min(end, c0 + run);
+    unsigned sum = 0, total;
+    for (unsigned c = c0; c < c1; ++c) sum += S.gridcount[c];
+    unsigned off = block_exclusive_scan(sum, &total);
+    if (threadIdx.x < SPH_SMALL_BLOCKS) cluster.map_shared_rank(totals, threadIdx.x)[rank] = total;
+    cluster.sync();  // every block's total is in every block
+    for (unsigned b = 0; b < rank; ++b) off += totals[b];
+    for (unsigned c = c0; c < c1; ++c) {
+        S.celloffset[c] = off;
+        off += S.gridcount[c];
+    }
+    cluster.sync();  // the offsets are written
+    unsigned first[SPH_SMALL_ITEMS];
+#pragma unroll
+    for (int j = 0; j < SPH_SMALL_ITEMS; ++j)
+        if (me + j * threads < n) first[j] = S.celloffset[cell[j]];
+#pragma unroll
+    for (int j = 0; j < SPH_SMALL_ITEMS; ++j)
+        if (me + j * threads < n) S.unsorted[first[j] + slot[j]] = me + j * threads;
+    cluster.sync();  // the cells' lists are complete
+#pragma unroll 1
+    for (int j = 0; j < SPH_SMALL_ITEMS; ++j) {
+        const unsigned i = me + j * threads;
+        if (i >= n) break;
+        const unsigned cnt = S.gridcount[cell[0]];
+        const unsigned *U = S.unsorted + first[0];
+        unsigned k = first[0];
+#pragma unroll 4
+        for (unsigned a = 0; a < cnt; ++a) k += U[a] < i;
+        S.cellparticles[k] = i;
+        if (GATHER) gather_one(S, k, i, cell[0], with_vel, 0, with_solid);
+#pragma unroll
+        for (int q = 0; q + 1 < SPH_SMALL_ITEMS; ++q) cell[q] = cell[q + 1], first[q] = first[q + 1];
+    }
 }

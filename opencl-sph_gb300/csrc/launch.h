@@ -31,6 +31,9 @@ struct Launch {
     // every scene of the table is mixed: the plain-fluid instantiations,
     // which skip mixed scenes, are not launched (false is always safe)
     bool all_mixed;
+    // the table is one scene whose grid one cluster builds in one launch
+    // (sph_small_grid; false is always safe)
+    bool small_grid;
 };
 
 // At most this many rigid bodies per launch (the reduction grid's y extent).
@@ -170,6 +173,11 @@ void sph_launch_substep(const Launch &L, SphMaterial mat, PhaseMark mark = nullp
 // the separate stress and step passes for scenes with symmetry planes.
 // `mark` names each phase.
 void sph_launch_solid_passes(const Launch &L, bool corot, PhaseMark mark = nullptr, void *ctx = nullptr);
+
+// Whether one cluster builds the grid of a scene of this size: a rule on the
+// sizes, and that the device can run the cluster (call outside any stream
+// capture, after sph_prepare_kernels).
+bool sph_small_grid(unsigned pnum, unsigned num_cells);
 
 // One-time kernel attributes (call outside any stream capture).
 cudaError_t sph_prepare_kernels();

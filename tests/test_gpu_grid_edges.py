@@ -45,3 +45,23 @@ def test_grid_matches_oracle(n, box, h, crowd):
         m = n if f in ("gridcell", "cellparticles") else a.size
         assert np.array_equal(a.ravel()[:m], b.ravel()[:m]), f
     ps.close()
+
+
+@pytest.mark.parametrize("n,cells_side", [(1, 1), (511, 7), (4096, 40), (4097, 40), (16384, 39), (16384, 41)])
+def test_small_scene_grid_at_its_limits(n, cells_side):
+    """One to four particles a thread, the last size before the launches of
+    a large scene (pnum 16,384 with 39^3 cells) and a grid past the line."""
+    rng = np.random.default_rng(n)
+    h = 0.02
+    box = cells_side * h + 1e-4
+    sc = scenes.wcsph_block(2, 2, 2, h=h, box=(0.0, box), pnum=n)
+    pos = rng.uniform(-0.01, box + 0.01, size=(n, 3))  # some outside
+    sc.init = {"position": pos.astype(np.float32), "n": n}
+    ps = sc.system()
+    o = oracle_of(ps)
+    o.call("compute_particle_bins")
+    ps.compute_particle_bins()
+    ps.sync_device_to_host()
+    for f in ("gridcell", "gridcount", "celloffset", "cellparticles"):
+        assert np.array_equal(ps.get_fields(f)[0].ravel(), o.a[f].ravel()), f
+    ps.close()
