@@ -153,6 +153,7 @@ bool solid_setup(sph_batch *b, BatchScene *sc) {
     L.grid_cap = cap_of(b);
     L.stream = b->stream;
     L.no_symmetry_planes = sc->desc.num_symmetry_planes == 0;
+    L.split_rows = sph_split_rows(sc->desc.pnum);
     sph_launch_init_original_position(L);
     sph_launch_bins_gather(L, false, false);
     sph_launch_density(L, true);
@@ -227,6 +228,9 @@ bool rebuild(sph_batch *b) {
     A.num_rigid = (unsigned)rigid.size();
     A.no_symmetry_planes = std::all_of(descs.begin(), descs.end(),
                                        [](const SceneDesc &d) { return d.num_symmetry_planes == 0; });
+    unsigned long long particles = 0;
+    for (const SceneDesc &d : descs) particles += d.pnum;
+    A.split_rows = sph_split_rows(particles);
     cudaStream_t streams[3] = {b->stream, b->side[0], b->side[1]};
     for (int m = 0; m < 3; ++m) {
         GroupLaunch &G = b->group[m];

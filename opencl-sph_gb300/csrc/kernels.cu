@@ -9,6 +9,8 @@
 #include "kernels_solid.cuh"
 #include "launch.h"
 
+#define SPH_SPLIT_PARTICLES 40000ull
+
 static inline unsigned grid_for(const BlockMap &m, unsigned cap) {
     unsigned g = m.num < cap ? m.num : cap;
     return g ? g : 1;
@@ -34,15 +36,17 @@ static void launch_grid_small(const Launch &L, bool vel, bool solid) {
 }
 
 cudaError_t sph_prepare_kernels() {
-    // the density pass's staging buffers (may exceed the default limit)
-    const int want = (int)sizeof(DensityStage);
-    cudaError_t e = cudaFuncSetAttribute(k_density<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, want);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_density<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, want);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_density<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, want);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_density<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, want);
+    // the density pass's staging buffers may exceed the default limit
+    cudaError_t e = cudaSuccess;
+    auto room = [&](const void *kernel, size_t bytes) {
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    };
+    const size_t whole = sizeof(DensityStage<false>);
+    room((const void *)k_density<false, false>, whole);
+    room((const void *)k_density<true, false>, whole);
+    room((const void *)k_density<false, true>, whole);
+    room((const void *)k_density<true, true>, whole);
     if (SPH_SMALL_BLOCKS > 8) {
         if (e == cudaSuccess)
             e = cudaFuncSetAttribute(k_grid_small<true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
@@ -51,6 +55,14 @@ cudaError_t sph_prepare_kernels() {
     }
     return e;
 }
+
+// Split against whole fluid passes, us a substep with three scenes' substeps
+// overlapping / one scene's alone: 1,000 particles 16.4 / 47.0 -> 14.6 /
+// 41.2, 8,000 17.7 / 53.6 -> 16.0 / 45.1, 25,000 21.9 / 63.7 -> 20.7 / 54.4,
+// 40,000 27.8 / 72.5 -> 27.9 / 65.0, 64,000 27.4 / 66.0 -> 31.1 / 67: from
+// there on the schedulers are full and a block's repeated set-up costs more
+// than its shorter chain saves.
+bool sph_split_rows(unsigned long long particles) { return particles <= SPH_SPLIT_PARTICLES; }
 
 // One cluster against five launches, us a substep with three scenes' substeps
 // overlapping / one scene's alone: 1,000 particles 19.2 / 53.6 -> 16.5 /
@@ -129,38 +141,57 @@ void sph_launch_gather(const Launch &L, bool vel, bool dens, bool solid) {
                                                                           dens ? 1 : 0, solid ? 1 : 0);
 }
 
+// Blocks of a SPLIT launch: each map entry in groups of 32 particles.
+static unsigned split_per(const Launch &L) { return L.pair_block / 32u; }
+static unsigned split_grid(const Launch &L, const BlockMap &m) {
+    const unsigned long long g = (unsigned long long)m.num * split_per(L);
+    return g < L.grid_cap ? (g ? (unsigned)g : 1u) : L.grid_cap;
+}
+
+template <bool PLANES, bool COUNT>
+static void launch_density(const Launch &L, const BlockMap &m, int original, int mask, int skip_solids) {
+    if (L.split_rows)
+        k_density<PLANES, COUNT, true><<<split_grid(L, m), dim3(32, 3), sizeof(DensityStage<true>), L.stream>>>(
+            L.scenes, m, original, mask, skip_solids, split_per(L));
+    else
+        k_density<PLANES, COUNT><<<grid_for(m, L.grid_cap), L.pair_block, sizeof(DensityStage<false>), L.stream>>>(
+            L.scenes, m, original, mask, skip_solids, 1u);
+}
+
 void sph_launch_density(const Launch &L, bool original, bool mask, bool skip_solids, bool count) {
-    const size_t smem = sizeof(DensityStage);
-    const unsigned g = grid_for(L.pair_particles, L.grid_cap);
     const int o = original ? 1 : 0, m = mask ? 1 : 0, sk = skip_solids ? 1 : 0;
+    const BlockMap &map = L.pair_particles;
     if (mask && count) {
-        k_density<false, true><<<g, L.pair_block, smem, L.stream>>>(L.scenes, L.pair_particles, o, m, sk);
-        if (!L.no_symmetry_planes)
-            k_density<true, true><<<g, L.pair_block, smem, L.stream>>>(L.scenes, L.pair_particles, o, m, 0);
+        launch_density<false, true>(L, map, o, m, sk);
+        if (!L.no_symmetry_planes) launch_density<true, true>(L, map, o, m, 0);
         return;
     }
-    k_density<false><<<g, L.pair_block, smem, L.stream>>>(L.scenes, L.pair_particles, o, m, sk);
-    if (!L.no_symmetry_planes) k_density<true><<<g, L.pair_block, smem, L.stream>>>(L.scenes, L.pair_particles, o, m, 0);
+    launch_density<false, false>(L, map, o, m, sk);
+    if (!L.no_symmetry_planes) launch_density<true, false>(L, map, o, m, 0);
 }
 
 void sph_launch_density_fused(const Launch &L, const Launch *fluids) {
-    const size_t smem = sizeof(DensityStage);
-    if (fluids && fluids->pair_particles.num)
-        k_density<false><<<grid_for(fluids->pair_particles, L.grid_cap), L.pair_block, smem, L.stream>>>(
-            L.scenes, fluids->pair_particles, 0, 1, 1);
-    if (!L.no_symmetry_planes)
-        k_density<true><<<grid_for(L.pair_particles, L.grid_cap), L.pair_block, smem, L.stream>>>(
-            L.scenes, L.pair_particles, 0, 1, 0);
+    if (fluids && fluids->pair_particles.num) launch_density<false, false>(L, fluids->pair_particles, 0, 1, 1);
+    if (!L.no_symmetry_planes) launch_density<true, false>(L, L.pair_particles, 0, 1, 0);
+}
+
+template <bool MIXED>
+static void launch_forces_masked(const Launch &L, int step) {
+    const BlockMap &m = L.pair_particles;
+    if (L.split_rows)
+        k_forces_fluids_masked<MIXED, true>
+            <<<split_grid(L, m), dim3(32, 3), 0, L.stream>>>(L.scenes, m, step, split_per(L));
+    else
+        k_forces_fluids_masked<MIXED>
+            <<<grid_for(m, L.grid_cap), L.pair_block, 0, L.stream>>>(L.scenes, m, step, 1u);
 }
 
 void sph_launch_forces_fluids(const Launch &L, bool fuse_step, bool masked) {
     const unsigned g = grid_for(L.pair_particles, L.grid_cap);
     const int step = fuse_step ? 1 : 0;
     if (masked) {
-        if (!L.all_mixed)
-            k_forces_fluids_masked<false><<<g, L.pair_block, 0, L.stream>>>(L.scenes, L.pair_particles, step);
-        if (L.has_mixed)
-            k_forces_fluids_masked<true><<<g, L.pair_block, 0, L.stream>>>(L.scenes, L.pair_particles, step);
+        if (!L.all_mixed) launch_forces_masked<false>(L, step);
+        if (L.has_mixed) launch_forces_masked<true>(L, step);
     } else {
         if (!L.all_mixed) k_forces_fluids<false><<<g, L.pair_block, 0, L.stream>>>(L.scenes, L.pair_particles, step);
         if (L.has_mixed) k_forces_fluids<true><<<g, L.pair_block, 0, L.stream>>>(L.scenes, L.pair_particles, step);

@@ -25,6 +25,14 @@ __device__ __forceinline__ bool scene_idle(const SceneDesc &S) { return S.steps_
         if (scene_idle(S)) continue;                                           \
         const unsigned item = bw_.first + threadIdx.x;
 #define SPH_END_WORK }
+// The same with each map entry in `per` groups of `size` items, one group
+// per pass: `first` is the group's first item.
+#define SPH_FOR_GROUPS(map, per, size)                                         \
+    for (unsigned vb_ = blockIdx.x; vb_ < (map).num * (per); vb_ += gridDim.x) { \
+        const BlockWork bw_ = (map).work[vb_ / (per)];                         \
+        const SceneDesc &S = scenes[bw_.scene];                                \
+        if (scene_idle(S)) continue;                                           \
+        const unsigned first = bw_.first + (size) * (vb_ % (per));
 
 // Active particle count, clamped to the store's capacity so that a bad `n`
 // written from the host can never index past the fields.

@@ -53,20 +53,31 @@
 // candidates; a row of more than 64 marks the particle for a scan
 // (ncand[k] = SPH_NCAND_SCAN).  The stores of one row are one coalesced
 // store per warp.
-// SPH_STAGE candidates hold a plane's ranges: about 440 for 128 particles
-// in a lattice of 8 per cell, 820 for 256.
+// A plane's buffer of 896 candidates holds its ranges: about 440 for 128
+// particles in a lattice of 8 per cell, 820 for 256.
+//
+// SPLIT (small launches): a block is three warps over the same 32 particles,
+// one per z plane, each with a buffer of its own; the nine row sums meet in
+// shared memory and are added in the same order, so the bits are the same.
+// Where there are fewer warps than the schedulers can hold, a warp's own
+// chain of nine rows is the time of the pass.
 //
 // Bound: issue slots, 4,118 warp instructions per 32 particles at 1M (the
 // walk 1,411, near_bits 1,423, the rest row bounds, staging and masks)
 // against 5,001 for testing each candidate exactly as it comes, from rows
 // staged per warp: 160 -> 144 us at 1M particles (ncu), 1M-particle substep
 // 362 -> 349 us, mixed scene 519 -> 477 us.
-#define SPH_STAGE 896
-
-// two buffers, and each row's staged range (first index, padded length)
+//
+// The buffers (two in turn, or one per plane), and each row's staged range
+// (first index, padded length).
+template <bool SPLIT>
 struct DensityStage {
-    float xyz[2][3 * SPH_STAGE];
+    static constexpr unsigned size = SPLIT ? 256 : 896;
+    float xyz[SPLIT ? 3 : 2][3 * size];
     uint2 range[9];
+    float rows[SPLIT ? 9 : 1][32];      // row sums
+    unsigned counts[SPLIT ? 3 : 1][32];
+    unsigned cands[SPLIT ? 3 : 1][32];  // candidates, or SPH_NCAND_SCAN
 };
 
 // Which of the staged candidates p .. p + 4 ng - 1 (16-byte aligned, ng
@@ -74,14 +85,15 @@ struct DensityStage {
 // nz: the particle's negated coordinates; nb: the negated bound, each twice.
 // The differences are the exact test's; r^2 - bound is a chain of fused
 // multiply-adds (3 packed operations fewer).  A NaN has its sign clear.
+template <unsigned STRIDE>
 __device__ __forceinline__ unsigned near_bits(const float *__restrict__ p, unsigned ng, float2 nx, float2 ny, float2 nz,
                                               float2 nb) {
     unsigned acc = 0;
 #pragma unroll 1
     for (unsigned g = 0; g < ng; ++g, p += 4) {
         const float4 X = *reinterpret_cast<const float4 *>(p);
-        const float4 Y = *reinterpret_cast<const float4 *>(p + SPH_STAGE);
-        const float4 Z = *reinterpret_cast<const float4 *>(p + 2 * SPH_STAGE);
+        const float4 Y = *reinterpret_cast<const float4 *>(p + STRIDE);
+        const float4 Z = *reinterpret_cast<const float4 *>(p + 2 * STRIDE);
         auto two = [&](float2 x, float2 y, float2 z) {
             const float2 dx = __fadd2_rn(x, nx), dy = __fadd2_rn(y, ny), dz = __fadd2_rn(z, nz);
             const float2 s = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __ffma2_rn(dx, dx, nb)));
@@ -108,9 +120,11 @@ __device__ __forceinline__ float fluid_pressure(float rho, float rho0, float sti
 
 // COUNT: a masked pass that also counts num_neighbours (a named
 // compute_density, whose caller may read the count before the force pass).
-template <bool PLANES, bool MASK, bool COUNT = false>
-__device__ __forceinline__ void density_block(const SceneDesc &S, unsigned n, unsigned first, DensityStage &stage,
-                                              int original) {
+template <bool PLANES, bool MASK, bool COUNT, bool SPLIT>
+__device__ __forceinline__ void density_block(const SceneDesc &S, unsigned n, unsigned first,
+                                              DensityStage<SPLIT> &stage, int original) {
+    constexpr unsigned STAGE = DensityStage<SPLIT>::size;
+    const unsigned flat = SPLIT ? threadIdx.y * 32u + threadIdx.x : threadIdx.x;
     const unsigned k = first + threadIdx.x;
     const bool active = k < n;
     const ScenePair B = scene_pair(S);
@@ -118,11 +132,11 @@ __device__ __forceinline__ void density_block(const SceneDesc &S, unsigned n, un
     const float4 *__restrict__ spos = S.spos;
     const unsigned pnum = S.pnum;
     const StencilRows rows(S, active ? S.srow[k] : make_uint2(0u, 0u));
-    if (threadIdx.x < 9u) {
+    if (flat < 9u) {
         // row r's ranges of the block's particles lie between its first
         // particle's cell x-1 and its last one's x+1 (by cell index, so past
         // an end of the grid's row they take in neighbouring rows too)
-        const int r = threadIdx.x;
+        const int r = flat;
         const long long d = (long long)(r / 3 - 1) * rows.layer + (r % 3 - 1) * (long long)rows.R0;
         const long long c0 = (long long)S.srow[first].x + d - 1,
                         c1 = (long long)S.srow[min(first + blockDim.x, n) - 1u].x + d + 1;
@@ -134,7 +148,7 @@ __device__ __forceinline__ void density_block(const SceneDesc &S, unsigned n, un
             e = min(S.celloffset[x1] + S.gridcount[x1], pnum);
         }
         const unsigned a = b & ~3u;
-        stage.range[r] = make_uint2(a, b < e ? (min(e - a, (unsigned)SPH_STAGE) + 3u) & ~3u : 0u);
+        stage.range[r] = make_uint2(a, b < e ? (min(e - a, STAGE) + 3u) & ~3u : 0u);
     }
     const float3 ipos = active ? xyz(spos[k]) : make_float3(0.f, 0.f, 0.f);
     const NegPoint nip = neg_point(ipos);
@@ -151,7 +165,7 @@ __device__ __forceinline__ void density_block(const SceneDesc &S, unsigned n, un
     unsigned count = 0, total = 0;
     bool overflow = false;
     __syncthreads();
-    // where plane dz's rows start in its buffer; past SPH_STAGE: not staged
+    // where plane dz's rows start in its buffer; past STAGE: not staged
     auto plane_at = [&](int dz, unsigned (&at)[4], unsigned (&ua)[3]) {
         at[0] = 0;
 #pragma unroll
@@ -164,16 +178,16 @@ __device__ __forceinline__ void density_block(const SceneDesc &S, unsigned n, un
     auto stage_plane = [&](int dz) {
         unsigned at[4], ua[3];
         plane_at(dz, at, ua);
-        if (at[3] > SPH_STAGE) return;
-        float *to = stage.xyz[dz & 1];
+        if (at[3] > STAGE) return;
+        float *to = stage.xyz[SPLIT ? dz : dz & 1];
 #pragma unroll 1
         for (unsigned t = threadIdx.x; t < at[3]; t += blockDim.x) {
             const unsigned row0 = t < at[1] ? ua[0] : t < at[2] ? ua[1] - at[1] : ua[2] - at[2];
             // up to three past the range: any value (capacity bounds it)
             const float *p = reinterpret_cast<const float *>(spos + min(row0 + t, pnum - 1u));
             copy_word_async(to + t, p);
-            copy_word_async(to + SPH_STAGE + t, p + 1);
-            copy_word_async(to + 2 * SPH_STAGE + t, p + 2);
+            copy_word_async(to + STAGE + t, p + 1);
+            copy_word_async(to + 2 * STAGE + t, p + 2);
         }
     };
     // the exact walk over the staged candidates of a chunk's bits (candidate
@@ -184,7 +198,7 @@ __device__ __forceinline__ void density_block(const SceneDesc &S, unsigned n, un
         while (m) {
             const unsigned t = __clz(m), bit = 0x80000000u >> t;
             m ^= bit;
-            const float r2 = dist2(make_float4(src[t], src[SPH_STAGE + t], src[2 * SPH_STAGE + t], 0.f), nip);
+            const float r2 = dist2(make_float4(src[t], src[STAGE + t], src[2 * STAGE + t], 0.f), nip);
             // beyond h by a rounding: h2 - r2 <= 0 adds nothing
             const float d = fmaxf(h2 - r2, 0.f);
             rowsum = __fadd_rn(rowsum, d * d * d);
@@ -193,10 +207,11 @@ __device__ __forceinline__ void density_block(const SceneDesc &S, unsigned n, un
         }
         return hit;
     };
-    unsigned *mask = S.nbmask + k;
-    stage_plane(0);
+    const int dz0 = SPLIT ? (int)threadIdx.y : 0, dz1 = SPLIT ? dz0 + 1 : 3;
+    unsigned *mask = S.nbmask + (size_t)(6 * dz0) * pnum + k;
+    stage_plane(dz0);
 #pragma unroll 1
-    for (int dz = 0; dz < 3; ++dz) {
+    for (int dz = dz0; dz < dz1; ++dz) {
         unsigned b[3], e[3], at[4], ua[3];
 #pragma unroll
         for (int dy = 0; dy < 3; ++dy) {
@@ -204,11 +219,11 @@ __device__ __forceinline__ void density_block(const SceneDesc &S, unsigned n, un
             if (active) rows.row(S, 3 * dz + dy, &b[dy], &e[dy]);
         }
         plane_at(dz, at, ua);
-        const bool fits = at[3] <= SPH_STAGE;
-        const float *buf = stage.xyz[dz & 1];
+        const bool fits = at[3] <= STAGE;
+        const float *buf = stage.xyz[SPLIT ? dz : dz & 1];
         copies_wait();
         __syncthreads();  // this plane is staged, and the other buffer is free
-        if (dz < 2) stage_plane(dz + 1);
+        if (dz + 1 < dz1) stage_plane(dz + 1);
         // the plane's rows in turn: [0] of each array, which then moves up
 #pragma unroll 1
         for (int dy = 0; dy < 3; ++dy) {
@@ -226,7 +241,7 @@ __device__ __forceinline__ void density_block(const SceneDesc &S, unsigned n, un
                 const unsigned o = b[0] & 3u, tot = len ? o + len : 0u;
                 const float *src = buf + at[0] + (b[0] - o - ua[0]);
                 if (tot) {
-                    unsigned m = near_bits(src, min((tot + 3u) >> 2, 8u), nx, ny, nz, nb) & (0xffffffffu >> o);
+                    unsigned m = near_bits<STAGE>(src, min((tot + 3u) >> 2, 8u), nx, ny, nz, nb) & (0xffffffffu >> o);
                     if (tot < 32u) m &= ~(0xffffffffu >> tot);
                     m = walk(m, src, rowsum);
                     if (MASK) lo = __brev(m) >> o;
@@ -234,7 +249,7 @@ __device__ __forceinline__ void density_block(const SceneDesc &S, unsigned n, un
 #pragma unroll 1
                 for (unsigned c0 = 32; c0 < tot; c0 += 32) {
                     const unsigned rem = tot - c0;
-                    unsigned m = near_bits(src + c0, min((rem + 3u) >> 2, 8u), nx, ny, nz, nb);
+                    unsigned m = near_bits<STAGE>(src + c0, min((rem + 3u) >> 2, 8u), nx, ny, nz, nb);
                     if (rem < 32u) m &= ~(0xffffffffu >> rem);
                     m = walk(m, src + c0, rowsum);
                     if (MASK && c0 < 96u) {
@@ -283,7 +298,8 @@ __device__ __forceinline__ void density_block(const SceneDesc &S, unsigned n, un
                     }
                 }
             }
-            rho.add(rowsum);
+            if (SPLIT) stage.rows[3 * dz + dy][threadIdx.x] = rowsum;
+            else rho.add(rowsum);
             if (MASK && active) {
                 // store_row_mask's layout
                 mask[0] = lo;
@@ -294,6 +310,22 @@ __device__ __forceinline__ void density_block(const SceneDesc &S, unsigned n, un
             }
             b[0] = b[1], e[0] = e[1], ua[0] = ua[1], at[0] = at[1], at[1] = at[2];
             b[1] = b[2], e[1] = e[2], ua[1] = ua[2], at[2] = at[3];
+        }
+    }
+    if (SPLIT) {
+        stage.counts[dz0][threadIdx.x] = count;
+        stage.cands[dz0][threadIdx.x] = overflow ? SPH_NCAND_SCAN : total;
+        __syncthreads();
+        if (dz0) return;
+#pragma unroll
+        for (int r = 0; r < 9; ++r) rho.add(stage.rows[r][threadIdx.x]);
+        count = total = 0;
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            const unsigned c = stage.cands[q][threadIdx.x];
+            count += stage.counts[q][threadIdx.x];
+            overflow |= c == SPH_NCAND_SCAN;
+            total += c;
         }
     }
     const unsigned i = active ? min(S.cellparticles[k], pnum - 1) : 0u;
@@ -329,23 +361,24 @@ __device__ __forceinline__ void density_block(const SceneDesc &S, unsigned n, un
 // plane-free loop free of its registers.  COUNT: the masked pass counts
 // num_neighbours too (a named compute_density recording masks); a kernel
 // of its own, so the fused substep's keeps its register allocation.
-template <bool PLANES, bool COUNT = false>
-__global__ void __launch_bounds__(512, 2)
-    k_density(const SceneDesc *__restrict__ scenes, BlockMap map, int original, int want_mask, int skip_solids) {
+// SPLIT: blocks of (32, 3) threads, each map entry `per` of them.
+template <bool PLANES, bool COUNT = false, bool SPLIT = false>
+__global__ void __launch_bounds__(SPLIT ? 96 : 512, SPLIT ? 10 : 2)
+    k_density(const SceneDesc *__restrict__ scenes, BlockMap map, int original, int want_mask, int skip_solids,
+              unsigned per) {
     extern __shared__ __align__(16) unsigned char sm_stage[];
-    DensityStage &stage = *reinterpret_cast<DensityStage *>(sm_stage);
-    SPH_FOR_WORK(map)
+    DensityStage<SPLIT> &stage = *reinterpret_cast<DensityStage<SPLIT> *>(sm_stage);
+    SPH_FOR_GROUPS(map, SPLIT ? per : 1u, 32u)
     if ((S.num_symmetry_planes != 0) != PLANES) continue;
     // in a fused substep a plane-free solid's first solid pass sums its density
     if (skip_solids && !PLANES && (S.programs & (PROG_COROT | PROG_SVK))) continue;
     const unsigned n = active_count(S);
-    const unsigned first = item - threadIdx.x;
     if (first >= n) continue;
     __syncthreads();  // the block's last entry is done with the buffers
     if (want_mask && S.nbmask && (S.programs & PROG_FLUIDS) && !original)
-        density_block<PLANES, true, COUNT>(S, n, first, stage, original);
+        density_block<PLANES, true, COUNT, SPLIT>(S, n, first, stage, original);
     else
-        density_block<PLANES, false>(S, n, first, stage, original);
+        density_block<PLANES, false, false, SPLIT>(S, n, first, stage, original);
     SPH_END_WORK
 }
 
@@ -543,21 +576,36 @@ __global__ void k_forces_fluids(const SceneDesc *__restrict__ scenes, BlockMap m
 // scene leaves to it.
 // At most 64 registers: with the current walk 64 beats 56 (0.1886 ->
 // 0.1859 ms at 1M particles), where the earlier walk ran best at 56.
-template <bool MIXED>
-__global__ void __maxnreg__(64) k_forces_fluids_masked(const SceneDesc *__restrict__ scenes, BlockMap map, int fuse_step) {
-    SPH_FOR_WORK(map)
+// SPLIT as in the density pass: blocks of (32, 3) threads, a warp per z
+// plane, the row sums added in the same order by the first.
+template <bool MIXED, bool SPLIT = false>
+__global__ void __maxnreg__(64)
+    k_forces_fluids_masked(const SceneDesc *__restrict__ scenes, BlockMap map, int fuse_step, unsigned per) {
+    __shared__ float rows_sum[SPLIT ? 9 : 1][3][32];
+    __shared__ unsigned rows_count[SPLIT ? 3 : 1][32];
+    SPH_FOR_GROUPS(map, SPLIT ? per : 1u, 32u)
     if (MIXED && !S.phase) continue;  // the plain instantiation covers those
     if (!MIXED && S.phase) continue;
-    if (item < active_count(S)) {
-        const unsigned k = item;
-        const unsigned i = min(S.cellparticles[k], S.pnum - 1);
-        const FluidI I = fluid_i(S, xyz(S.spos[k]), xyz(S.svel[k]), S.sdens[k]);
-        const StencilRows rows(S, S.srow[k]);
+    const unsigned n = active_count(S);
+    if (SPLIT) {
+        if (first >= n) continue;
+        __syncthreads();  // the block's last entry is done with the sums
+    }
+    const int r0 = SPLIT ? 3 * (int)threadIdx.y : 0, r1 = SPLIT ? r0 + 3 : 9;
+    const unsigned k = first + threadIdx.x;
+    // a block's warps stay together to its end, where their sums meet
+    const bool active = k < n;
+    if (SPLIT || active) {
+        const unsigned kc = SPLIT ? min(k, n - 1u) : k;  // an idle lane repeats the last particle
+        const unsigned i = min(S.cellparticles[kc], S.pnum - 1);
+        const FluidI I = fluid_i(S, xyz(S.spos[kc]), xyz(S.svel[kc]), S.sdens[kc]);
+        const StencilRows rows(S, S.srow[kc]);
         const bool solid_i = mixed_solid<MIXED>(S, i);
         BlockSum3 f;
         unsigned count = 0;  // num_neighbours, which the density pass left to this one
-        if (S.ncand[k] != SPH_NCAND_SCAN) {
-            count = 1;  // k itself (r^2 = 0), whose mask bit the walk clears
+        const bool scan = S.ncand[kc] == SPH_NCAND_SCAN;
+        if (!scan && active) {
+            count = r0 <= 4 && 4 < r1;  // k itself (r^2 = 0), whose mask bit the walk clears
             const float4 *__restrict__ spos = S.spos;
             const float4 *__restrict__ svel = S.svel;
             // two neighbours per iteration: both loads are in flight
@@ -565,14 +613,14 @@ __global__ void __maxnreg__(64) k_forces_fluids_masked(const SceneDesc *__restri
             // the next row's bounds and low mask word are loaded while this
             // row is walked
             unsigned nb, ne;
-            rows.row(S, 0, &nb, &ne);
-            unsigned nlo = S.nbmask[k];
+            rows.row(S, r0, &nb, &ne);
+            unsigned nlo = S.nbmask[(size_t)(2 * r0) * S.pnum + k];
 #pragma unroll 1
-            for (int r = 0; r < 9; ++r) {
+            for (int r = r0; r < r1; ++r) {
                 unsigned b = nb;
                 const unsigned len = ne - nb;
                 unsigned lo = nlo & (len >= 32u ? 0xffffffffu : (1u << len) - 1u);
-                if (r < 8) {
+                if (r + 1 < r1) {
                     rows.row(S, r + 1, &nb, &ne);
                     nlo = S.nbmask[(size_t)(2 * (r + 1)) * S.pnum + k];
                 }
@@ -603,10 +651,29 @@ __global__ void __maxnreg__(64) k_forces_fluids_masked(const SceneDesc *__restri
                         }
                     }
                 }
-                f.end_row();
+                if (SPLIT) {
+                    rows_sum[r][0][threadIdx.x] = f.rxy.x;
+                    rows_sum[r][1][threadIdx.x] = f.rxy.y;
+                    rows_sum[r][2][threadIdx.x] = f.rz;
+                    f = BlockSum3();
+                } else {
+                    f.end_row();
+                }
             }
-        } else {
+        } else if (active && r0 == 0) {
             count = fluid_scan<MIXED>(S, rows.cell, I, f, solid_i);
+        }
+        if (SPLIT) {
+            rows_count[r0 / 3][threadIdx.x] = count;
+            __syncthreads();
+            if (r0 || !active) continue;
+            if (!scan) {
+#pragma unroll
+                for (int r = 0; r < 9; ++r)
+                    f.total.add(make_float3(rows_sum[r][0][threadIdx.x], rows_sum[r][1][threadIdx.x],
+                                            rows_sum[r][2][threadIdx.x]));
+            }
+            count += rows_count[1][threadIdx.x] + rows_count[2][threadIdx.x];
         }
         if (!S.num_symmetry_planes) S.num_neighbours[i] = count;
         fluid_finish(S, i, I, f, fuse_step, mixed_extra<MIXED>(S, i, solid_i));

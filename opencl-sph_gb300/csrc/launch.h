@@ -34,6 +34,9 @@ struct Launch {
     // the table is one scene whose grid one cluster builds in one launch
     // (sph_small_grid; false is always safe)
     bool small_grid;
+    // few particles in all: the pair passes spread a particle's stencil over
+    // three warps (sph_split_rows; either way gives the same bits)
+    bool split_rows;
 };
 
 // At most this many rigid bodies per launch (the reduction grid's y extent).
@@ -178,6 +181,9 @@ void sph_launch_solid_passes(const Launch &L, bool corot, PhaseMark mark = nullp
 // sizes, and that the device can run the cluster (call outside any stream
 // capture, after sph_prepare_kernels).
 bool sph_small_grid(unsigned pnum, unsigned num_cells);
+
+// Whether a launch over this many particles splits the stencil.
+bool sph_split_rows(unsigned long long particles);
 
 // One-time kernel attributes (call outside any stream capture).
 cudaError_t sph_prepare_kernels();

@@ -49,3 +49,24 @@ def test_density_rows_match_oracle(n, per_cell, lattice):
         fused = ps.get_fields("num_neighbours", "density")
         assert np.array_equal(fused[0][:m], count) and np.array_equal(fused[1][:m], dens)
         ps.close()
+
+
+def test_split_and_whole_passes_give_the_same_bits():
+    """A scene alone (its stencils split over three warps) and in a batch
+    whose particles are past the line (whole): the same bits, with rows of
+    every length, a cell above 64 candidates a row and spare capacity."""
+    from sph.batch import Batch
+    for n, per_cell in ((1, 8), (31, 3), (700, 8), (1500, 22), (2500, 60)):
+        sc = cloud(n, per_cell, n)
+        ps = sc.system()
+        ps.update_fused(3)
+        ps.sync_device_to_host()
+        b = Batch()
+        sid = b.add(sc)
+        b.add(scenes.wcsph_block(36, 36, 36, jitter=1e-4, seed=2))
+        b.step(3)
+        got = b.read(sid)
+        for f in ("position", "velocity", "force", "density", "num_neighbours"):
+            assert np.array_equal(got[f], ps.get_fields(f)[0]), f
+        b.close()
+        ps.close()
