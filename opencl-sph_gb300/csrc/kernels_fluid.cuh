@@ -369,7 +369,7 @@ __global__ void __launch_bounds__(SPLIT ? 96 : 512, SPLIT ? 10 : 2)
     extern __shared__ __align__(16) unsigned char sm_stage[];
     DensityStage<SPLIT> &stage = *reinterpret_cast<DensityStage<SPLIT> *>(sm_stage);
     SPH_FOR_GROUPS(map, SPLIT ? per : 1u, 32u)
-    if ((S.num_symmetry_planes != 0) != PLANES) continue;
+    if (has_planes(S) != PLANES) continue;
     // in a fused substep a plane-free solid's first solid pass sums its density
     if (skip_solids && !PLANES && (S.programs & (PROG_COROT | PROG_SVK))) continue;
     const unsigned n = active_count(S);
@@ -675,7 +675,7 @@ __global__ void __maxnreg__(64)
             }
             count += rows_count[1][threadIdx.x] + rows_count[2][threadIdx.x];
         }
-        if (!S.num_symmetry_planes) S.num_neighbours[i] = count;
+        if (!has_planes(S)) S.num_neighbours[i] = count;
         fluid_finish(S, i, I, f, fuse_step, mixed_extra<MIXED>(S, i, solid_i));
     }
     SPH_END_WORK
@@ -716,7 +716,7 @@ __device__ __forceinline__ void integrate(const SceneDesc &S, unsigned i, float3
 __global__ void k_step_forward(const SceneDesc *__restrict__ scenes, BlockMap map, int planes_only) {
     SPH_FOR_WORK(map)
     // a fused substep's plane-free solids were stepped by their force pass
-    if (planes_only && !S.num_symmetry_planes) continue;
+    if (planes_only && !has_planes(S)) continue;
     if (item < active_count(S)) {
         const unsigned i = item;
         integrate(S, i, ld3(S.force, i), ld3(S.velocity, i), ld3(S.position, i));

@@ -247,7 +247,7 @@ __device__ __forceinline__ float3 reflect_bits(const Planes &P, unsigned bits, f
 // tested); k_rotations_and_strains serves the others.
 __global__ void k_rotations_and_strains_planes(const SceneDesc *__restrict__ scenes, BlockMap map) {
     SPH_FOR_WORK(map)
-    if (S.num_symmetry_planes == 0) continue;  // k_rotations_and_strains covers those
+    if (!has_planes(S)) continue;  // k_rotations_and_strains covers those
     if (item < active_count(S)) {
         const unsigned k = item;
         const unsigned i = min(S.cellparticles[k], S.pnum - 1);
@@ -429,7 +429,7 @@ __global__ void k_stresses_corot(const SceneDesc *__restrict__ scenes, BlockMap 
 // symmetry planes; k_deformations serves the others.
 __global__ void k_deformations_planes(const SceneDesc *__restrict__ scenes, BlockMap map) {
     SPH_FOR_WORK(map)
-    if (S.num_symmetry_planes == 0) continue;  // k_deformations covers those
+    if (!has_planes(S)) continue;  // k_deformations covers those
     if (item < active_count(S)) {
         const unsigned k = item;
         const unsigned i = min(S.cellparticles[k], S.pnum - 1);
@@ -503,7 +503,7 @@ __global__ void k_stresses_svk(const SceneDesc *__restrict__ scenes, BlockMap ma
 template <bool COROT>
 __global__ void k_forces_solids_planes(const SceneDesc *__restrict__ scenes, BlockMap map) {
     SPH_FOR_WORK(map)
-    if (S.num_symmetry_planes == 0) continue;  // k_forces_solids covers those
+    if (!has_planes(S)) continue;  // k_forces_solids covers those
     if (item < active_count(S)) {
         const unsigned k = item;
         const unsigned i = min(S.cellparticles[k], S.pnum - 1);
@@ -678,7 +678,7 @@ __device__ __forceinline__ void scan_solid_rows(const SceneDesc &S, unsigned k, 
 __global__ void __maxnreg__(64) k_rotations_and_strains(const SceneDesc *__restrict__ scenes, BlockMap map,
                                                         int with_density, int with_stress) {
     SPH_FOR_WORK(map)
-    if (S.num_symmetry_planes || !S.spos0) continue;  // sorted copies exist with solids.cl
+    if (has_planes(S) || !S.spos0) continue;  // sorted copies exist with solids.cl
     if (item < active_count(S)) {
         const unsigned k = item;
         const unsigned i = min(S.cellparticles[k], S.pnum - 1);
@@ -759,7 +759,7 @@ __global__ void __maxnreg__(64) k_rotations_and_strains(const SceneDesc *__restr
 __global__ void k_deformations(const SceneDesc *__restrict__ scenes, BlockMap map, int with_density,
                                int with_stress) {
     SPH_FOR_WORK(map)
-    if (S.num_symmetry_planes || !S.spos0) continue;  // sorted copies exist with solids.cl
+    if (has_planes(S) || !S.spos0) continue;  // sorted copies exist with solids.cl
     if (item < active_count(S)) {
         const unsigned k = item;
         const unsigned i = min(S.cellparticles[k], S.pnum - 1);
@@ -815,7 +815,7 @@ template <bool COROT>
 __global__ void k_stresses_sorted(const SceneDesc *__restrict__ scenes, BlockMap map, int planes_only) {
     SPH_FOR_WORK(map)
     // a plane-free scene's first pass stored its stresses already
-    if (planes_only && !S.num_symmetry_planes) continue;
+    if (planes_only && !has_planes(S)) continue;
     if (item < active_count(S) && S.sstress) {
         const unsigned k = item;
         const unsigned i = min(S.cellparticles[k], S.pnum - 1);
@@ -952,7 +952,7 @@ __device__ __forceinline__ void solid_pair(const SolidConsts &C, const SolidI &I
 template <bool COROT, bool MASKED>
 __global__ void __maxnreg__(80) k_forces_solids(const SceneDesc *__restrict__ scenes, BlockMap map, int fuse_step) {
     SPH_FOR_WORK(map)
-    if (S.num_symmetry_planes || (MASKED && !S.sstress)) continue;
+    if (has_planes(S) || (MASKED && !S.sstress)) continue;
     if (item < active_count(S)) {
         const unsigned k = item;
         const unsigned i = min(S.cellparticles[k], S.pnum - 1);

@@ -209,3 +209,34 @@ def test_kinematic_bodies():
     for f in ["position", "velocity", "rotation", "body_position", "body_euler_rotation"]:
         assert max_rel(ps.get_fields(f)[0], orc.a[f].reshape(ps.get_fields(f)[0].shape)) <= 1e-5, f
     ps.close()
+
+
+@pytest.mark.parametrize("material", ["corot", "svk"])
+def test_unset_symmetry_planes_change_nothing(material):
+    """A store whose slots for symmetry planes are unset (zero normals) gives
+    the bits of one without slots, named and fused; with a plane set it
+    matches the oracle's images as before (the other tests here)."""
+    def run(slots, fused):
+        sc = scenes.solid_lattice(6, 5, 7, material=material, youngs_modulus=5e4, jitter=1e-4, seed=5, clamp_layers=1)
+        if slots:
+            sc.entries = [("symmetry_planes", "3, 2, 3", "float", None) if e[0] == "symmetry_planes" else e
+                          for e in sc.entries]
+        ps = sc.system()
+        for call in ("init_original_position", None, "compute_original_density"):
+            ps.call_for_all_particles(call) if call else ps.compute_particle_bins()
+        first = "compute_rotations_and_strains" if material == "corot" else "compute_deformations"
+        for _ in range(4):
+            if fused:
+                ps.update_fused(1)
+            else:
+                ps.compute_particle_bins()
+                for call in ("compute_density", first, "compute_stresses", "compute_forces_solids", "step_forward"):
+                    ps.call_for_all_particles(call)
+        ps.sync_device_to_host()
+        out = [np.array(a) for a in ps.get_fields("position", "velocity", "force", "stress", "density",
+                                                  "num_neighbours")]
+        ps.close()
+        return out
+    want = run(False, True)
+    for slots, fused in ((True, True), (True, False), (False, False)):
+        assert all(np.array_equal(a, b) for a, b in zip(run(slots, fused), want)), (slots, fused)
