@@ -2,6 +2,8 @@
 // and the host functions that enqueue them (see launch.h).
 #include <stdio.h>
 
+#include <atomic>
+
 #include "kernels_fluid.cuh"
 #include "kernels_grid.cuh"
 #include "kernels_mixed.cuh"
@@ -74,14 +76,21 @@ bool sph_split_rows(unsigned long long particles) { return particles <= SPH_SPLI
 // largest cluster every configuration runs.
 bool sph_small_grid(unsigned pnum, unsigned num_cells) {
     if (pnum > SPH_SMALL_PARTICLES || num_cells > SPH_SMALL_CELLS) return false;
-    cudaLaunchConfig_t cfg{};
-    cudaLaunchAttribute at[1];
-    small_grid_config(&cfg, at, nullptr);
-    int clusters = 0;
-    const bool ok = cudaOccupancyMaxActiveClusters(&clusters, k_grid_small<true>, &cfg) == cudaSuccess &&
-                    clusters > 0;
-    if (!ok) cudaGetLastError();
-    return ok;
+    // what the device can run, asked once per device (0: not yet, 1: no, 2: yes)
+    static std::atomic<int> known[64];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
+    int v = known[dev].load();
+    if (!v) {
+        cudaLaunchConfig_t cfg{};
+        cudaLaunchAttribute at[1];
+        small_grid_config(&cfg, at, nullptr);
+        int clusters = 0;
+        v = cudaOccupancyMaxActiveClusters(&clusters, k_grid_small<true>, &cfg) == cudaSuccess && clusters > 0 ? 2 : 1;
+        if (v == 1) cudaGetLastError();
+        known[dev].store(v);
+    }
+    return v == 2;
 }
 
 cudaError_t sph_check_launch(const char *what) {
