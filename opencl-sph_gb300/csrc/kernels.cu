@@ -49,6 +49,9 @@ cudaError_t sph_prepare_kernels() {
     room((const void *)k_density<true, false>, whole);
     room((const void *)k_density<false, true>, whole);
     room((const void *)k_density<true, true>, whole);
+    const size_t most = solid_smem_bytes(false, 16);  // pair blocks of 512
+    room((const void *)k_rotations_and_strains<false>, most);
+    room((const void *)k_deformations<false>, most);
     if (SPH_SMALL_BLOCKS > 8) {
         if (e == cudaSuccess)
             e = cudaFuncSetAttribute(k_grid_small<true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
@@ -237,8 +240,14 @@ void sph_launch_init_original_position(const Launch &L) {
 
 void sph_launch_rotations_and_strains(const Launch &L, bool with_density, bool with_stress) {
     const unsigned g = grid_for(L.pair_particles, L.grid_cap);
-    k_rotations_and_strains<<<g, L.pair_block, 0, L.stream>>>(L.scenes, L.pair_particles, with_density ? 1 : 0,
-                                                              with_density && with_stress ? 1 : 0);
+    const unsigned w = L.pair_block / 32u;
+    const int d = with_density ? 1 : 0, st = with_density && with_stress ? 1 : 0;
+    if (L.split_rows)
+        k_rotations_and_strains<true><<<split_grid(L, L.pair_particles), dim3(32, 3), solid_smem_bytes(true, 3),
+                                        L.stream>>>(L.scenes, L.pair_particles, d, st, split_per(L));
+    else
+        k_rotations_and_strains<false><<<g, dim3(32, w), solid_smem_bytes(false, w), L.stream>>>(
+            L.scenes, L.pair_particles, d, st, 1u);
     if (!L.no_symmetry_planes)
         k_rotations_and_strains_planes<<<g, L.pair_block, 0, L.stream>>>(L.scenes, L.pair_particles);
 }
@@ -256,25 +265,36 @@ void sph_launch_stresses(const Launch &L, bool corot, bool sorted, bool planes_o
 
 void sph_launch_deformations(const Launch &L, bool with_density, bool with_stress) {
     const unsigned g = grid_for(L.pair_particles, L.grid_cap);
-    k_deformations<<<g, L.pair_block, 0, L.stream>>>(L.scenes, L.pair_particles, with_density ? 1 : 0,
-                                                     with_density && with_stress ? 1 : 0);
+    const unsigned w = L.pair_block / 32u;
+    const int d = with_density ? 1 : 0, st = with_density && with_stress ? 1 : 0;
+    if (L.split_rows)
+        k_deformations<true><<<split_grid(L, L.pair_particles), dim3(32, 3), solid_smem_bytes(true, 3), L.stream>>>(
+            L.scenes, L.pair_particles, d, st, split_per(L));
+    else
+        k_deformations<false><<<g, dim3(32, w), solid_smem_bytes(false, w), L.stream>>>(L.scenes, L.pair_particles, d,
+                                                                                       st, 1u);
     if (!L.no_symmetry_planes) k_deformations_planes<<<g, L.pair_block, 0, L.stream>>>(L.scenes, L.pair_particles);
 }
 
-void sph_launch_forces_solids(const Launch &L, bool corot, bool masked, bool fuse_step) {
-    const unsigned g = grid_for(L.pair_particles, L.grid_cap);
-    const int step = masked && fuse_step ? 1 : 0;
-    if (corot) {
-        if (masked) k_forces_solids<true, true><<<g, L.pair_block, 0, L.stream>>>(L.scenes, L.pair_particles, step);
-        else k_forces_solids<true, false><<<g, L.pair_block, 0, L.stream>>>(L.scenes, L.pair_particles, 0);
-        if (!L.no_symmetry_planes)
-            k_forces_solids_planes<true><<<g, L.pair_block, 0, L.stream>>>(L.scenes, L.pair_particles);
+template <bool COROT>
+static void launch_forces_solids(const Launch &L, bool masked, int step) {
+    const BlockMap &m = L.pair_particles;
+    const dim3 part(32, 3), whole(32, L.pair_block / 32u);
+    const unsigned gp = split_grid(L, m), g = grid_for(m, L.grid_cap), per = split_per(L);
+    if (L.split_rows) {
+        if (masked) k_forces_solids<COROT, true, true><<<gp, part, solid_force_smem_bytes(3), L.stream>>>(L.scenes, m, step, per);
+        else k_forces_solids<COROT, false, true><<<gp, part, solid_force_smem_bytes(3), L.stream>>>(L.scenes, m, 0, per);
     } else {
-        if (masked) k_forces_solids<false, true><<<g, L.pair_block, 0, L.stream>>>(L.scenes, L.pair_particles, step);
-        else k_forces_solids<false, false><<<g, L.pair_block, 0, L.stream>>>(L.scenes, L.pair_particles, 0);
-        if (!L.no_symmetry_planes)
-            k_forces_solids_planes<false><<<g, L.pair_block, 0, L.stream>>>(L.scenes, L.pair_particles);
+        if (masked) k_forces_solids<COROT, true, false><<<g, whole, solid_force_smem_bytes(whole.y), L.stream>>>(L.scenes, m, step, 1u);
+        else k_forces_solids<COROT, false, false><<<g, whole, solid_force_smem_bytes(whole.y), L.stream>>>(L.scenes, m, 0, 1u);
     }
+    if (!L.no_symmetry_planes) k_forces_solids_planes<COROT><<<g, L.pair_block, 0, L.stream>>>(L.scenes, m);
+}
+
+void sph_launch_forces_solids(const Launch &L, bool corot, bool masked, bool fuse_step) {
+    const int step = masked && fuse_step ? 1 : 0;
+    if (corot) launch_forces_solids<true>(L, masked, step);
+    else launch_forces_solids<false>(L, masked, step);
 }
 
 void sph_launch_solid_passes(const Launch &L, bool corot, PhaseMark mark, void *ctx) {

@@ -301,6 +301,34 @@ struct StencilRows {
     }
 };
 
+// ---- staged candidates ----------------------------------------------------------
+
+// Which of the staged candidates p .. p + 4 ng - 1 (16-byte aligned, ng
+// 1..8) may lie within the bound: candidate p + t at bit 31 - t.  nx, ny,
+// nz: the particle's negated coordinates; nb: the negated bound, each twice.
+// The differences are the exact test's; r^2 - bound is a chain of fused
+// multiply-adds (3 packed operations fewer).  A NaN has its sign clear.
+template <unsigned STRIDE>
+__device__ __forceinline__ unsigned near_bits(const float *__restrict__ p, unsigned ng, float2 nx, float2 ny, float2 nz,
+                                              float2 nb) {
+    unsigned acc = 0;
+#pragma unroll 1
+    for (unsigned g = 0; g < ng; ++g, p += 4) {
+        const float4 X = *reinterpret_cast<const float4 *>(p);
+        const float4 Y = *reinterpret_cast<const float4 *>(p + STRIDE);
+        const float4 Z = *reinterpret_cast<const float4 *>(p + 2 * STRIDE);
+        auto two = [&](float2 x, float2 y, float2 z) {
+            const float2 dx = __fadd2_rn(x, nx), dy = __fadd2_rn(y, ny), dz = __fadd2_rn(z, nz);
+            const float2 s = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __ffma2_rn(dx, dx, nb)));
+            acc = __funnelshift_l(__float_as_uint(s.x), acc, 1);
+            acc = __funnelshift_l(__float_as_uint(s.y), acc, 1);
+        };
+        two(make_float2(X.x, X.y), make_float2(Y.x, Y.y), make_float2(Z.x, Z.y));
+        two(make_float2(X.z, X.w), make_float2(Y.z, Y.w), make_float2(Z.z, Z.w));
+    }
+    return acc << (32u - 4u * ng);
+}
+
 // ---- candidate masks -----------------------------------------------------------
 // The first pair pass of a fused substep records, per stencil row r of
 // sorted particle k, which candidates the later passes need: bit t of the
@@ -310,10 +338,10 @@ struct StencilRows {
 // row exceeds 64 and the later passes must scan.
 
 // Records row r's mask: low word always, high word for rows over 32.
-__device__ __forceinline__ void store_row_mask(const SceneDesc &S, unsigned k, int r, unsigned len,
-                                               unsigned long long bits) {
-    S.nbmask[(size_t)(2 * r) * S.pnum + k] = (unsigned)bits;
-    if (len > 32) S.nbmask[(size_t)(2 * r + 1) * S.pnum + k] = (unsigned)(bits >> 32);
+__device__ __forceinline__ void store_row_mask(const SceneDesc &S, unsigned k, int r, unsigned len, unsigned lo,
+                                               unsigned hi) {
+    S.nbmask[(size_t)(2 * r) * S.pnum + k] = lo;
+    if (len > 32u) S.nbmask[(size_t)(2 * r + 1) * S.pnum + k] = hi;
 }
 
 // Row r's mask as recorded, with bits past the row's end cleared (every
@@ -329,20 +357,21 @@ __device__ __forceinline__ unsigned long long load_row_mask(const SceneDesc &S, 
     return ((unsigned long long)hi << 32) | lo;
 }
 
-// Calls f(kk) for the candidates of particle k's recorded masks, in order.
+// Calls f(kk) for the candidates of particle k's recorded masks in rows
+// [r0, r1), in order.
 // PREFETCH: the next row's bounds and low mask word are loaded while a row
 // is walked (it pays in the corotational pass 2; the solid force passes,
 // at their register cap, run slower with it).
-template <bool PREFETCH = false, class F, class G>
+template <bool PREFETCH = false, class F>
 __device__ __forceinline__ void for_each_masked(const SceneDesc &S, unsigned k, const StencilRows &rows, F &&f,
-                                                G &&row_end) {
+                                                int r0 = 0, int r1 = 9) {
     unsigned nb = 0, ne = 0, nlo = 0;
     if (PREFETCH) {
-        rows.row(S, 0, &nb, &ne);
-        nlo = S.nbmask[k];
+        rows.row(S, r0, &nb, &ne);
+        nlo = S.nbmask[(size_t)(2 * r0) * S.pnum + k];
     }
 #pragma unroll 1
-    for (int r = 0; r < 9; ++r) {
+    for (int r = r0; r < r1; ++r) {
         unsigned b, e;
         unsigned long long mask;
         if (PREFETCH) {
@@ -350,7 +379,7 @@ __device__ __forceinline__ void for_each_masked(const SceneDesc &S, unsigned k, 
             e = ne;
             const unsigned len = e - b;
             const unsigned lo = nlo & (len >= 32u ? 0xffffffffu : (1u << len) - 1u);
-            if (r < 8) {
+            if (r + 1 < r1) {
                 rows.row(S, r + 1, &nb, &ne);
                 nlo = S.nbmask[(size_t)(2 * (r + 1)) * S.pnum + k];
             }
@@ -373,12 +402,7 @@ __device__ __forceinline__ void for_each_masked(const SceneDesc &S, unsigned k, 
                 f(b + t);
             }
         }
-        row_end();
     }
-}
-template <bool PREFETCH = false, class F>
-__device__ __forceinline__ void for_each_masked(const SceneDesc &S, unsigned k, const StencilRows &rows, F &&f) {
-    for_each_masked<PREFETCH>(S, k, rows, f, [] {});
 }
 
 // ---- symmetry planes (the SYMMETRY blocks, e.g. common.cl:647-686) ----------

@@ -80,32 +80,6 @@ struct DensityStage {
     unsigned cands[SPLIT ? 3 : 1][32];  // candidates, or SPH_NCAND_SCAN
 };
 
-// Which of the staged candidates p .. p + 4 ng - 1 (16-byte aligned, ng
-// 1..8) may lie within the bound: candidate p + t at bit 31 - t.  nx, ny,
-// nz: the particle's negated coordinates; nb: the negated bound, each twice.
-// The differences are the exact test's; r^2 - bound is a chain of fused
-// multiply-adds (3 packed operations fewer).  A NaN has its sign clear.
-template <unsigned STRIDE>
-__device__ __forceinline__ unsigned near_bits(const float *__restrict__ p, unsigned ng, float2 nx, float2 ny, float2 nz,
-                                              float2 nb) {
-    unsigned acc = 0;
-#pragma unroll 1
-    for (unsigned g = 0; g < ng; ++g, p += 4) {
-        const float4 X = *reinterpret_cast<const float4 *>(p);
-        const float4 Y = *reinterpret_cast<const float4 *>(p + STRIDE);
-        const float4 Z = *reinterpret_cast<const float4 *>(p + 2 * STRIDE);
-        auto two = [&](float2 x, float2 y, float2 z) {
-            const float2 dx = __fadd2_rn(x, nx), dy = __fadd2_rn(y, ny), dz = __fadd2_rn(z, nz);
-            const float2 s = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __ffma2_rn(dx, dx, nb)));
-            acc = __funnelshift_l(__float_as_uint(s.x), acc, 1);
-            acc = __funnelshift_l(__float_as_uint(s.y), acc, 1);
-        };
-        two(make_float2(X.x, X.y), make_float2(Y.x, Y.y), make_float2(Z.x, Z.y));
-        two(make_float2(X.z, X.w), make_float2(Y.z, Y.w), make_float2(Z.z, Z.w));
-    }
-    return acc << (32u - 4u * ng);
-}
-
 // Asynchronous 4-byte copy from global to shared memory.
 __device__ __forceinline__ void copy_word_async(float *dst, const float *src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)

@@ -199,7 +199,7 @@ __device__ __forceinline__ float3 sym_vec(const float s[6], float3 v) {
 }
 // m += a b^T, one fused multiply-add per entry, written out so that every
 // copy of a sum rounds alike whatever the compiler would contract.
-__device__ __forceinline__ void add_outer(float3 a, float3 b, float m[9]) {
+__device__ __forceinline__ void add_outer(float3 a, float3 b, float *m) {
     m[0] = __fmaf_rn(a.x, b.x, m[0]); m[1] = __fmaf_rn(a.x, b.y, m[1]); m[2] = __fmaf_rn(a.x, b.z, m[2]);
     m[3] = __fmaf_rn(a.y, b.x, m[3]); m[4] = __fmaf_rn(a.y, b.y, m[4]); m[5] = __fmaf_rn(a.y, b.z, m[5]);
     m[6] = __fmaf_rn(a.z, b.x, m[6]); m[7] = __fmaf_rn(a.z, b.y, m[7]); m[8] = __fmaf_rn(a.z, b.z, m[8]);
@@ -601,209 +601,466 @@ __global__ void k_forces_solids_planes(const SceneDesc *__restrict__ scenes, Blo
 // neighbours in the same order with the same arithmetic as a walk over all
 // candidates, so the results are identical; the named force pass (whose
 // masks may be stale) scans.
+//
+// Every sum over the stencil is blocked by z plane: a plane's terms in
+// candidate order, and the three planes' sums in plane order.  So a warp may
+// take its 32 particles' three planes in turn, or (SPLIT, small launches:
+// sph_split_rows) three warps one plane each, with the sums meeting in
+// shared memory; the bits are the same.  A small scene has too few warps to
+// hide a chain of three planes; in a large one the two more set-ups per
+// particle cost more than they hide (on 65,536 corotational particles the
+// split passes take 20% longer).  Blocks are (32, W) threads: W = 3 planes
+// of one group of 32 particles, `per` groups in a map entry, or W groups.
 
-// Pass 1 of the plane-free solid passes over particle k's stencil rows,
-// from the cell-sorted copies.  Each row is taken in chunks of 32
-// candidates, one mask word each: a tight loop over the chunk records the
-// mask bits (|p| <= h or |q| <= h, k itself excluded) and the bits of the
-// chunk's current neighbours (|p| <= h, k itself included).  Then a walk
-// over those neighbours, in candidate order, adds each one's density term
-// (the density pass's blocked sum, in its order: row sums in candidate
-// order, Kahan-added row by row) and for j != i runs sum(p, q, w),
-// w = (h^2 - |p|^2)^3.  The scan loop thus stays free of the sums' work,
-// which otherwise every lane would issue whenever any lane of its warp met
-// a neighbour, and every sum sees the neighbours in the order a plain scan
-// would.  Only a row's first 64 candidates have mask bits; `overflow`
-// records a longer row.
+// A plane's three rows staged by its warp: current and rest positions, one
+// array per coordinate.  About 156 candidates in a lattice of 8 per cell;
+// more room (192, 256) took a batch longer, whose other branches share the
+// SMs' memory.
+#define SPH_SOLID_STAGE 160
+struct SolidPlane {
+    float x[3 * SPH_SOLID_STAGE];   // SPLIT, after the scan: the plane's sums
+    float x0[3 * SPH_SOLID_STAGE];
+};
+// SPLIT: what the planes' warps hand on
+struct SolidParts {
+    float rows[9][32];       // density row sums
+    unsigned counts[3][32];  // neighbours closer than h
+    unsigned cands[3][32];   // candidates, or SPH_NCAND_SCAN
+};
+struct SolidScan {  // a particle's counts over the planes scanned
+    unsigned count = 0, total = 0;
+    bool overflow = false;
+};
+
+// Shared memory of a first pass: a SolidPlane per warp, then (SPLIT) the
+// SolidParts; and of a force pass.
+__host__ __device__ constexpr size_t solid_smem_bytes(bool split, unsigned warps) {
+    return sizeof(SolidPlane) * warps + (split ? sizeof(SolidParts) : 0);
+}
+__host__ __device__ constexpr size_t solid_force_smem_bytes(unsigned warps) { return sizeof(float) * 6 * 32 * warps; }
+
+// Pass 1 over plane dz of particle k's stencil (k of lane threadIdx.x; rows
+// empty for a lane past the scene's end), from the staged copies.  A row is
+// taken in chunks of 32 candidates: near_bits marks those that may be
+// within h now, and within h at rest (more than are, by a rounding at most).
+// A walk over the current ones, in candidate order, tests each exactly, adds
+// its density term (the density pass's blocked sum, in its order) and runs
+// sum(p, q, w), w = (h^2 - |p|^2)^3; k itself and a candidate beyond h by a
+// rounding add zeros.  The few that are near at rest alone are then tested
+// exactly too, and the chunk's mask word is what is left of both, without k
+// itself.  Rows that do not fit the buffer together are staged one by one;
+// one that is wider than the buffer, or whose range does not lie in the
+// staged one (inconsistent host-written tables), tests each candidate from
+// the copies.
+// Only a row's first 64 candidates have mask bits.  row_end(r, sum) takes
+// each row's density sum.
 //
 // The density terms are summed whether or not the caller stores them: a
 // flag tested inside the loops lets the compiler emit one copy of them per
 // value, and copies may contract the sums' products differently, which
 // would break the equality of the named and fused passes.
-template <class Sum>
-__device__ __forceinline__ void scan_solid_rows(const SceneDesc &S, unsigned k, const StencilRows &rows,
-                                                float3 ipos, float3 ipos0, const SolidConsts &C, Kahan &rho,
-                                                unsigned &count, unsigned &total, bool &overflow, Sum &&sum) {
+template <class Sum, class RowEnd>
+__device__ __forceinline__ void scan_solid_plane(const SceneDesc &S, unsigned first, unsigned n, int dz,
+                                                 const StencilRows &rows, float3 ipos, float3 ipos0,
+                                                 const SolidConsts &C, SolidPlane &stage, SolidScan &seen, Sum &&sum,
+                                                 RowEnd &&row_end) {
+    constexpr unsigned STAGE = SPH_SOLID_STAGE;
     const float4 *__restrict__ spos = S.spos;
     const float4 *__restrict__ spos0 = S.spos0;
-    const NegPoint nip = neg_point(ipos), nip0 = neg_point(ipos0);
-#pragma unroll 1
-    for (int r = 0; r < 9; ++r) {
-        unsigned b, e;
-        rows.row(S, r, &b, &e);
-        const unsigned len = e - b;
-        float rowsum = 0.f;  // the row's density terms, as the density pass sums them
-#pragma unroll 1
-        for (unsigned c0 = 0; c0 < len; c0 += 32) {
-            const unsigned cb = b + c0, cn = min(len - c0, 32u);
-            unsigned bits = 0, near = 0;
-#pragma unroll 4
-            for (unsigned t = 0; t < cn; ++t) {
-                const unsigned kk = cb + t;
-                const float r2 = dist2(spos[kk], nip);
-                const float q2 = dist2(spos0[kk], nip0);
-                const unsigned bit = 1u << t;
-                if (r2 <= C.le) near |= bit;
-                if (r2 <= C.le || q2 <= C.le) bits |= bit;
-            }
-            if (k - cb < cn) bits &= ~(1u << (k - cb));  // k itself has no mask bit
-            // mask words 2r and 2r + 1 (store_row_mask's layout)
-            if (c0 < 64) S.nbmask[(size_t)(2 * r + (c0 >> 5)) * S.pnum + k] = bits;
-            while (near) {
-                const unsigned kk = cb + (unsigned)(__ffs(near) - 1);
-                near &= near - 1u;
-                const float3 p = sub3(xyz(spos[kk]), ipos);
-                const float r2 = norm2(p);
-                const float d = fmaxf(C.h2 - r2, 0.f);
-                const float w = d * d * d;
-                rowsum = __fadd_rn(rowsum, w);
-                count += r2 <= C.lt;
-                if (kk != k) sum(p, sub3(xyz(spos0[kk]), ipos0), w);
+    const unsigned lane = threadIdx.x, k = first + lane, pnum = S.pnum;
+    unsigned b[3], e[3], ua[3], at[4];
+    at[0] = 0;
+    {
+        // the rows' ranges of the block's particles (as the density pass)
+        unsigned ra = 0, rl = 0;
+        if (lane < 3u) {
+            const long long d = (long long)(dz - 1) * rows.layer + ((int)lane - 1) * (long long)rows.R0;
+            const long long c0 = (long long)S.srow[first].x + d - 1,
+                            c1 = (long long)S.srow[min(first + 32u, n) - 1u].x + d + 1;
+            const long long top = (long long)S.num_cells - 1;
+            if (c1 >= 0 && c0 <= top) {
+                const unsigned x0 = (unsigned)(c0 < 0 ? 0 : c0), x1 = (unsigned)(c1 > top ? top : c1);
+                const unsigned rb = S.celloffset[x0], re = min(S.celloffset[x1] + S.gridcount[x1], pnum);
+                ra = rb & ~3u;
+                rl = rb < re ? (min(re - ra, STAGE) + 3u) & ~3u : 0u;
             }
         }
-        rho.add(rowsum);
-        overflow |= len > 64;
-        total += len;
+#pragma unroll
+        for (int dy = 0; dy < 3; ++dy) {
+            rows.row(S, 3 * dz + dy, &b[dy], &e[dy]);
+            ua[dy] = __shfl_sync(SPH_FULL_MASK, ra, dy);
+            at[dy + 1] = at[dy] + __shfl_sync(SPH_FULL_MASK, rl, dy);
+        }
+    }
+    const bool fits = at[3] <= STAGE;
+    float *sx = stage.x, *sx0 = stage.x0;
+    auto stage_one = [&](unsigned t, unsigned kk) {
+        kk = min(kk, pnum - 1u);  // up to three past the range: any value
+        const float4 p = spos[kk], q = spos0[kk];
+        sx[t] = p.x, sx[STAGE + t] = p.y, sx[2 * STAGE + t] = p.z;
+        sx0[t] = q.x, sx0[STAGE + t] = q.y, sx0[2 * STAGE + t] = q.z;
+    };
+    if (fits) {
+        __syncwarp();  // the plane before is done with
+#pragma unroll 1
+        for (unsigned t = lane; t < at[3]; t += 32)
+            stage_one(t, t + (t < at[1] ? ua[0] : t < at[2] ? ua[1] - at[1] : ua[2] - at[2]));
+        __syncwarp();
+    }
+    const NegPoint nip = neg_point(ipos), nip0 = neg_point(ipos0);
+    const float wide = __fmaf_rn(C.le, 1.f + 0x1p-20f, 0x1p-126f);
+    const float2 nb = make_float2(-wide, -wide);
+    auto twice = [](float v) { return make_float2(-v, -v); };
+    // the plane's rows in turn: [0] of each array, which then moves up
+#pragma unroll 1
+    for (int dy = 0; dy < 3; ++dy) {
+        const unsigned len = e[0] - b[0];
+        unsigned lo = 0, hi = 0;
+        float rowsum = 0.f;  // the row's density terms, as the density pass sums them
+        auto add = [&](float3 p, float3 q) {
+            const float r2 = norm2(p);
+            const float d = fmaxf(C.h2 - r2, 0.f);
+            const float w = d * d * d;
+            rowsum = __fadd_rn(rowsum, w);
+            seen.count += r2 <= C.lt;
+            sum(p, q, w);
+            return r2 <= C.le;
+        };
+        if (!fits) {
+            __syncwarp();
+#pragma unroll 1
+            for (unsigned t = lane; t < at[1] - at[0]; t += 32) stage_one(t, t + ua[0]);
+            __syncwarp();
+        }
+        if (b[0] - ua[0] < at[1] - at[0] && e[0] - ua[0] <= at[1] - at[0]) {
+            const unsigned o = b[0] & 3u, tot = len ? o + len : 0u, a0 = (fits ? at[0] : 0u) + (b[0] - o - ua[0]);
+#pragma unroll 1
+            for (unsigned c0 = 0; c0 < tot; c0 += 32) {
+                const unsigned rem = tot - c0, ng = min((rem + 3u) >> 2, 8u);
+                const float *px = sx + a0 + c0, *px0 = sx0 + a0 + c0;
+                unsigned valid = c0 ? 0xffffffffu : 0xffffffffu >> o;
+                if (rem < 32u) valid &= ~(0xffffffffu >> rem);
+                unsigned near = near_bits<STAGE>(px, ng, twice(ipos.x), twice(ipos.y), twice(ipos.z), nb) & valid;
+                const unsigned rest =
+                    near_bits<STAGE>(px0, ng, twice(ipos0.x), twice(ipos0.y), twice(ipos0.z), nb) & valid;
+                unsigned w = near;
+#pragma unroll 1
+                while (near) {
+                    const unsigned t = __clz(near), bit = 0x80000000u >> t;
+                    near ^= bit;
+                    if (!add(sub3(make_float3(px[t], px[STAGE + t], px[2 * STAGE + t]), ipos),
+                             sub3(make_float3(px0[t], px0[STAGE + t], px0[2 * STAGE + t]), ipos0)))
+                        w ^= bit;
+                }
+#pragma unroll 1
+                for (unsigned only = rest & ~w; only;) {
+                    const unsigned t = __clz(only), bit = 0x80000000u >> t;
+                    only ^= bit;
+                    if (dist2(make_float4(px0[t], px0[STAGE + t], px0[2 * STAGE + t], 0.f), nip0) <= C.le) w |= bit;
+                }
+                const unsigned self = k - (b[0] - o + c0);
+                if (self < 32u) w &= ~(0x80000000u >> self);  // k itself has no mask bit
+                w = __brev(w);
+                // bit t of the row's mask is candidate b + t
+                if (c0 == 0) {
+                    lo = w >> o;
+                } else if (c0 < 96u) {
+                    const unsigned long long v = (unsigned long long)w << (32u - o);
+                    if (c0 == 32u) {
+                        lo |= (unsigned)v;
+                        hi = (unsigned)(v >> 32);
+                    } else {
+                        hi |= (unsigned)v;
+                    }
+                }
+            }
+        } else {
+#pragma unroll 1
+            for (unsigned t = 0; t < len; ++t) {
+                const float4 p4 = spos[b[0] + t], q4 = spos0[b[0] + t];
+                const bool near = dist2(p4, nip) <= C.le;
+                if (near) add(sub3(xyz(p4), ipos), sub3(xyz(q4), ipos0));
+                if ((near || dist2(q4, nip0) <= C.le) && b[0] + t != k) {
+                    if (t < 32u) lo |= 1u << t;
+                    else if (t < 64u) hi |= 1u << (t - 32u);
+                }
+            }
+        }
+        row_end(3 * dz + dy, rowsum);
+        if (len) store_row_mask(S, k, 3 * dz + dy, len, lo, hi);
+        seen.overflow |= len > 64;
+        seen.total += len;
+        b[0] = b[1], e[0] = e[1], ua[0] = ua[1], at[0] = at[1], at[1] = at[2];
+        b[1] = b[2], e[1] = e[2], ua[1] = ua[2], at[2] = at[3];
     }
 }
 
+// Pass 1 over the planes of this warp: v, the sums that `term(a, p, q, w)`
+// adds a neighbour's term to, and the density's rows.  SPLIT: one plane,
+// whose sums go to shared memory (total_sums adds them up after a barrier);
+// otherwise all three, v their total.
+template <bool SPLIT, int N, class Term>
+__device__ __forceinline__ void scan_solid(const SceneDesc &S, unsigned first, unsigned n, const StencilRows &rows,
+                                           float3 ipos, float3 ipos0, const SolidConsts &C, SolidPlane *stages,
+                                           SolidParts &parts, Kahan &rho, SolidScan &seen, float (&v)[N], Term &&term) {
+    const unsigned lane = threadIdx.x;
+    const int dz0 = SPLIT ? (int)threadIdx.y : 0, dz1 = SPLIT ? dz0 + 1 : 3;
+    SolidPlane &stage = stages[threadIdx.y];
+#pragma unroll 1
+    for (int dz = dz0; dz < dz1; ++dz) {
+        float a[N];
+#pragma unroll
+        for (int c = 0; c < N; ++c) a[c] = 0.f;
+        scan_solid_plane(S, first, n, dz, rows, ipos, ipos0, C, stage, seen,
+                         [&](float3 p, float3 q, float w) { term(a, p, q, w); },
+                         [&](int r, float sum) {
+                             if (SPLIT) parts.rows[r][lane] = sum;
+                             else rho.add(sum);
+                         });
+        if (SPLIT) {
+            __syncwarp();
+#pragma unroll
+            for (int c = 0; c < N; ++c) stage.x[32 * c + lane] = a[c];
+            parts.counts[dz][lane] = seen.count;
+            parts.cands[dz][lane] = seen.overflow ? SPH_NCAND_SCAN : seen.total;
+        } else {
+#pragma unroll
+            for (int c = 0; c < N; ++c) v[c] = dz == dz0 ? a[c] : __fadd_rn(v[c], a[c]);
+        }
+    }
+}
+
+// SPLIT, after a barrier: the planes' sums (from the at-th on) in plane
+// order; and the density rows and counts.
+template <int N>
+__device__ __forceinline__ void total_sums(const SolidPlane *stages, int at, float (&v)[N]) {
+#pragma unroll
+    for (int c = 0; c < N; ++c) {
+        const unsigned o = 32u * (at + c) + threadIdx.x;
+        v[c] = __fadd_rn(__fadd_rn(stages[0].x[o], stages[1].x[o]), stages[2].x[o]);
+    }
+}
+__device__ __forceinline__ void total_rows(const SolidParts &parts, Kahan &rho, SolidScan &seen) {
+    const unsigned lane = threadIdx.x;
+    rho = Kahan();
+    seen = SolidScan();
+#pragma unroll
+    for (int r = 0; r < 9; ++r) rho.add(parts.rows[r][lane]);
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+        seen.count += parts.counts[q][lane];
+        seen.total += parts.cands[q][lane];
+        seen.overflow |= parts.cands[q][lane] == SPH_NCAND_SCAN;
+    }
+}
+
+// The density of pass 1's particle k.  The sorted density copy (scratch) is
+// written either way.
+__device__ __forceinline__ float solid_density(const SceneDesc &S, unsigned i, unsigned k, const SolidConsts &C,
+                                               const Kahan &rho, const SolidScan &seen, int with_density) {
+    const float value = rho.s * C.coef * C.mass;
+    S.ncand[k] = seen.overflow ? SPH_NCAND_SCAN : seen.total;
+    S.sdens[k] = value;
+    if (with_density) {
+        S.density[i] = value;
+        S.num_neighbours[i] = seen.count;
+    }
+    return value;
+}
+
 // compute_rotations_and_strains (solid_corotation.cl:28-195) for
-// plane-free scenes: pass 1 (scan_solid_rows) sums Apq over candidates
+// plane-free scenes: pass 1 (scan_solid_plane) sums Apq over candidates
 // with |p| <= h and records the masks, R = polar(Apq), pass 2 sums D over
 // the masked candidates with |q| <= h.  Body particles keep their rotation and strain
-// (their masks are still recorded).  Also writes the sorted rotation copy.
-// At most 64 registers (about 100 bytes spill to L1): eight 128-thread
-// blocks per SM.  On batched-256, with the packed distance tests: 64 ->
-// 0.581 ms, 72 -> 0.590 ms, 80 -> 0.626 ms.
-__global__ void __maxnreg__(64) k_rotations_and_strains(const SceneDesc *__restrict__ scenes, BlockMap map,
-                                                        int with_density, int with_stress) {
-    SPH_FOR_WORK(map)
+// (their masks are still recorded).
+// SPLIT: the polar factor is one warp's work, beside which the second
+// computes the density.
+// Against a thread per particle that tests each candidate from the copies as
+// it comes (64 registers, 31.9M warp instructions on 65,536 particles; now
+// 27.5M): 78 -> 72 us there and 112 -> 94 us on 101,306 particles (whole, at
+// most 72 registers: 64 -> 98, 80 -> 93 but fewer warps beside a batch's
+// other branches), and 59 -> 28 us on 4,000 (split; 80 registers).
+template <bool SPLIT>
+__global__ void __maxnreg__(SPLIT ? 80 : 72)
+    k_rotations_and_strains(const SceneDesc *__restrict__ scenes, BlockMap map, int with_density, int with_stress,
+                            unsigned per) {
+    extern __shared__ __align__(16) unsigned char sm_solid[];
+    SolidPlane *stages = reinterpret_cast<SolidPlane *>(sm_solid);
+    SolidParts &parts = *reinterpret_cast<SolidParts *>(stages + 3);
+    SPH_FOR_GROUPS(map, per, 32u)
     if (has_planes(S) || !S.spos0) continue;  // sorted copies exist with solids.cl
-    if (item < active_count(S)) {
-        const unsigned k = item;
-        const unsigned i = min(S.cellparticles[k], S.pnum - 1);
-        const SolidConsts C = solid_consts(S);
-        const float4 p4 = S.spos[k], q4 = S.spos0[k];
-        const float3 ipos = xyz(p4), ipos0 = xyz(q4);
-        const StencilRows rows(S, S.srow[k]);
-        const float4 *__restrict__ spos = S.spos;
-        const float4 *__restrict__ spos0 = S.spos0;
-        float apq[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-        unsigned total = 0, count = 0;
-        bool overflow = false;
-        Kahan rho;
-        scan_solid_rows(S, k, rows, ipos, ipos0, C, rho, count, total, overflow,
-                        [&](float3 p, float3 q, float w) { add_outer(p * w, q, apq); });
-        S.ncand[k] = overflow ? SPH_NCAND_SCAN : total;
-        // the sorted density copy (scratch) is written either way: a value
-        // the named pass would discard lets the compiler emit a second copy
-        // of this kernel without the density sums, whose other sums may
-        // then round differently
-        const float value = rho.s * C.coef * C.mass;
-        S.sdens[k] = value;
-        if (with_density) {
-            S.density[i] = value;
-            S.num_neighbours[i] = count;
-        }
-        float R[9];
-        if (__float_as_uint(q4.w) > 0) {
-            // a body particle: rotation and strain stay as they are
-            for (int c = 0; c < 9; ++c) R[c] = S.rotation[9 * (size_t)i + c];
-        } else {
-            for (int c = 0; c < 9; ++c) apq[c] *= C.coef;
-            polar_rotation_fp64(apq, R);
-            for (int c = 0; c < 9; ++c) {
-                S.apq_temp[9 * (size_t)i + c] = apq[c];
-                S.intermediate[9 * (size_t)i + c] = apq[c];
-                S.rotation[9 * (size_t)i + c] = R[c];
+    const unsigned n = active_count(S);
+    const unsigned f = SPLIT ? first : first + 32u * threadIdx.y;  // the warp's group
+    if (f >= n) continue;
+    if (SPLIT) __syncthreads();  // the block's last group is done with the sums
+    const int dz0 = SPLIT ? (int)threadIdx.y : 0, dz1 = SPLIT ? dz0 + 1 : 3;
+    const unsigned k = f + threadIdx.x;
+    const bool active = k < n;
+    const unsigned kc = min(k, n - 1u);
+    const unsigned i = min(S.cellparticles[kc], S.pnum - 1);
+    const SolidConsts C = solid_consts(S);
+    const float4 p4 = S.spos[kc], q4 = S.spos0[kc];
+    const float3 ipos = xyz(p4), ipos0 = xyz(q4);
+    const bool body = __float_as_uint(q4.w) > 0;
+    const StencilRows rows(S, active ? S.srow[k] : make_uint2(0u, 0u));
+    Kahan rho;
+    SolidScan seen;
+    float R[9];
+    float density = 0.f;
+    {
+        float apq[9];
+        scan_solid<SPLIT>(S, f, n, rows, ipos, ipos0, C, stages, parts, rho, seen, apq,
+                          [](float (&a)[9], float3 p, float3 q, float w) { add_outer(p * w, q, a); });
+        if (SPLIT) __syncthreads();
+        if (dz0 == 0) {
+            if (SPLIT) total_sums(stages, 0, apq);
+            else if (active) density = solid_density(S, i, k, C, rho, seen, with_density);
+            if (body) {
+                // a body particle: rotation and strain stay as they are
+                for (int c = 0; c < 9; ++c) R[c] = S.rotation[9 * (size_t)i + c];
+            } else {
+                for (int c = 0; c < 9; ++c) apq[c] *= C.coef;
+                polar_rotation_fp64(apq, R);
+                if (active)
+                    for (int c = 0; c < 9; ++c) {
+                        S.apq_temp[9 * (size_t)i + c] = apq[c];
+                        S.intermediate[9 * (size_t)i + c] = apq[c];
+                        S.rotation[9 * (size_t)i + c] = R[c];
+                    }
             }
-            const float scale = C.mass / S.density0[i];
-            float D[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+            if (SPLIT)
+#pragma unroll
+                for (int c = 0; c < 9; ++c) stages[0].x0[32 * c + threadIdx.x] = R[c];
+        } else if (dz0 == 1) {
+            const bool mine = seen.overflow;
+            total_rows(parts, rho, seen);
+            if (active) {
+                density = solid_density(S, i, k, C, rho, seen, with_density);
+                stages[1].x0[threadIdx.x] = density;
+            }
+            seen.overflow = mine;
+        }
+    }
+    if (SPLIT) {
+        __syncthreads();
+#pragma unroll
+        for (int c = 0; c < 9; ++c) R[c] = stages[0].x0[32 * c + threadIdx.x];
+    }
+    float D[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+    const float4 *__restrict__ spos = S.spos;
+    const float4 *__restrict__ spos0 = S.spos0;
+    const float scale = C.mass / S.density0[i];
+#pragma unroll 1
+    for (int dz = dz0; dz < dz1; ++dz) {
+        float a[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+        if (active && !body) {
             // the masks hold no bit for k itself
             auto pass2_masked = [&](unsigned kk) {
                 const float3 q = sub3(xyz(spos0[kk]), ipos0);
                 const float3 g = spiky_grad(-q, C.h, C.kv, C.le);
                 if (g.x != 0.f || g.y != 0.f || g.z != 0.f) {
                     const float3 u = mat_t_vec(R, sub3(xyz(spos[kk]), ipos)) - q;
-                    add_outer(u * scale, g, D);
+                    add_outer(u * scale, g, a);
                 }
             };
-            auto pass2 = [&](unsigned kk) {
-                if (kk != k) pass2_masked(kk);
-            };
-            if (overflow) for_each_neighbour(S, S.srow[k].x, pass2);
-            else for_each_masked<true>(S, k, rows, pass2_masked);
-            float *st = S.strain + 6 * (size_t)i;
-            st[0] = D[0];
-            st[1] = D[4];
-            st[2] = D[8];
-            st[3] = 0.5f * (D[1] + D[3]);
-            st[4] = 0.5f * (D[2] + D[6]);
-            st[5] = 0.5f * (D[5] + D[7]);
+            if (seen.overflow) {
+                for (int r = 3 * dz; r < 3 * dz + 3; ++r) {
+                    unsigned b, e;
+                    rows.row(S, r, &b, &e);
+                    for (unsigned kk = b; kk < e; ++kk)
+                        if (kk != k) pass2_masked(kk);
+                }
+            } else {
+                for_each_masked<true>(S, k, rows, pass2_masked, 3 * dz, 3 * dz + 3);
+            }
         }
-        if (with_stress && S.sstress) {
-            // compute_stresses for this particle, as k_stresses_sorted<true>
-            // would (a body particle keeps its strain)
-            float e[6], o[6];
-            for (int c = 0; c < 6; ++c) e[c] = S.strain[6 * (size_t)i + c];
-            corot_stress(S, e, o);
-            store_stress(S, i, k, o, __fdiv_rn(C.mass, S.sdens[k]), R, __float_as_uint(q4.w) > 0);
+#pragma unroll
+        for (int c = 0; c < 9; ++c) {
+            if (SPLIT) stages[threadIdx.y].x[32 * c + threadIdx.x] = a[c];
+            else D[c] = dz == dz0 ? a[c] : __fadd_rn(D[c], a[c]);
         }
+    }
+    if (SPLIT) {
+        __syncthreads();
+        if (dz0) continue;
+        total_sums(stages, 0, D);
+        density = stages[1].x0[threadIdx.x];
+    }
+    if (!active) continue;
+    if (!body) {
+        float *st = S.strain + 6 * (size_t)i;
+        st[0] = D[0];
+        st[1] = D[4];
+        st[2] = D[8];
+        st[3] = 0.5f * (D[1] + D[3]);
+        st[4] = 0.5f * (D[2] + D[6]);
+        st[5] = 0.5f * (D[5] + D[7]);
+    }
+    if (with_stress && S.sstress) {
+        // compute_stresses for this particle, as k_stresses_sorted<true>
+        // would (a body particle keeps its strain)
+        float e[6], o[6];
+        for (int c = 0; c < 6; ++c) e[c] = S.strain[6 * (size_t)i + c];
+        corot_stress(S, e, o);
+        store_stress(S, i, k, o, __fdiv_rn(C.mass, density), R, body);
     }
     SPH_END_WORK
 }
 
 // compute_deformations (solid_svk.cl:82-175) for plane-free scenes, from
-// the sorted copies, recording the candidate masks.  No register cap (80):
-// on batched-256 uncapped 0.441 ms, 72 -> 0.446 ms, 64 -> 0.451 ms.
-__global__ void k_deformations(const SceneDesc *__restrict__ scenes, BlockMap map, int with_density,
-                               int with_stress) {
-    SPH_FOR_WORK(map)
+// the sorted copies, recording the candidate masks.  As above: 75 -> 65 us
+// on 101,306 particles, 45 -> 23 us on 32,768 (split).
+template <bool SPLIT>
+__global__ void __maxnreg__(SPLIT ? 80 : 72)
+    k_deformations(const SceneDesc *__restrict__ scenes, BlockMap map, int with_density, int with_stress,
+                   unsigned per) {
+    extern __shared__ __align__(16) unsigned char sm_solid[];
+    SolidPlane *stages = reinterpret_cast<SolidPlane *>(sm_solid);
+    SolidParts &parts = *reinterpret_cast<SolidParts *>(stages + 3);
+    SPH_FOR_GROUPS(map, per, 32u)
     if (has_planes(S) || !S.spos0) continue;  // sorted copies exist with solids.cl
-    if (item < active_count(S)) {
-        const unsigned k = item;
-        const unsigned i = min(S.cellparticles[k], S.pnum - 1);
-        const SolidConsts C = solid_consts(S);
-        const float3 ipos = xyz(S.spos[k]), ipos0 = xyz(S.spos0[k]);
-        const StencilRows rows(S, S.srow[k]);
-        float apq[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-        float aqq[6] = {0, 0, 0, 0, 0, 0};
-        unsigned total = 0, count = 0;
-        bool overflow = false;
-        Kahan rho;
-        scan_solid_rows(S, k, rows, ipos, ipos0, C, rho, count, total, overflow,
-                        [&](float3 p, float3 q, float w) {
-                            add_outer(p * w, q, apq);
-                            const float3 wq = q * w;
-                            aqq[0] = __fmaf_rn(wq.x, q.x, aqq[0]);
-                            aqq[1] = __fmaf_rn(wq.y, q.y, aqq[1]);
-                            aqq[2] = __fmaf_rn(wq.z, q.z, aqq[2]);
-                            aqq[3] = __fmaf_rn(wq.x, q.y, aqq[3]);
-                            aqq[4] = __fmaf_rn(wq.x, q.z, aqq[4]);
-                            aqq[5] = __fmaf_rn(wq.y, q.z, aqq[5]);
-                        });
-        S.ncand[k] = overflow ? SPH_NCAND_SCAN : total;
-        // the sorted density copy (scratch) is written either way: a value
-        // the named pass would discard lets the compiler emit a second copy
-        // of this kernel without the density sums, whose other sums may
-        // then round differently
-        const float value = rho.s * C.coef * C.mass;
-        S.sdens[k] = value;
-        if (with_density) {
-            S.density[i] = value;
-            S.num_neighbours[i] = count;
-        }
-        float inv[6];
-        sym_inverse(aqq, inv);
-        float F[9];
-        mul_as(apq, inv, F);
-        for (int c = 0; c < 9; ++c) S.deformation[9 * (size_t)i + c] = F[c];
-        if (with_stress && S.sstress) {
-            // compute_stresses for this particle, as k_stresses_sorted<false> would
-            float o[6];
-            svk_stress(S, F, o);
-            store_stress(S, i, k, o, __fdiv_rn(C.mass, S.sdens[k]), nullptr, false);
-        }
+    const unsigned n = active_count(S);
+    const unsigned f = SPLIT ? first : first + 32u * threadIdx.y;  // the warp's group
+    if (f >= n) continue;
+    if (SPLIT) __syncthreads();  // the block's last group is done with the sums
+    const unsigned k = f + threadIdx.x;
+    const bool active = k < n;
+    const unsigned kc = min(k, n - 1u);
+    const unsigned i = min(S.cellparticles[kc], S.pnum - 1);
+    const SolidConsts C = solid_consts(S);
+    const float3 ipos = xyz(S.spos[kc]), ipos0 = xyz(S.spos0[kc]);
+    const StencilRows rows(S, active ? S.srow[k] : make_uint2(0u, 0u));
+    Kahan rho;
+    SolidScan seen;
+    float v[15];  // Apq, then Aqq
+    scan_solid<SPLIT>(S, f, n, rows, ipos, ipos0, C, stages, parts, rho, seen, v,
+                      [](float (&a)[15], float3 p, float3 q, float w) {
+                          add_outer(p * w, q, a);
+                          const float3 wq = q * w;
+                          a[9] = __fmaf_rn(wq.x, q.x, a[9]);
+                          a[10] = __fmaf_rn(wq.y, q.y, a[10]);
+                          a[11] = __fmaf_rn(wq.z, q.z, a[11]);
+                          a[12] = __fmaf_rn(wq.x, q.y, a[12]);
+                          a[13] = __fmaf_rn(wq.x, q.z, a[13]);
+                          a[14] = __fmaf_rn(wq.y, q.z, a[14]);
+                      });
+    if (SPLIT) {
+        __syncthreads();
+        if (threadIdx.y) continue;
+        total_sums(stages, 0, v);
+        total_rows(parts, rho, seen);
+    }
+    if (!active) continue;
+    const float density = solid_density(S, i, k, C, rho, seen, with_density);
+    float inv[6], F[9];
+    sym_inverse(v + 9, inv);
+    mul_as(v, inv, F);
+    for (int c = 0; c < 9; ++c) S.deformation[9 * (size_t)i + c] = F[c];
+    if (with_stress && S.sstress) {
+        // compute_stresses for this particle, as k_stresses_sorted<false> would
+        float o[6];
+        svk_stress(S, F, o);
+        store_stress(S, i, k, o, __fdiv_rn(C.mass, density), nullptr, false);
     }
     SPH_END_WORK
 }
@@ -917,7 +1174,9 @@ struct SolidI {
 // The volume factor comes from per-particle reciprocals and the Laplacian's
 // distance from rsqrt, so a pair costs no division or square root.
 // IN_RANGE: the caller walks the first pass's masks, whose candidates
-// passed this range test with the same positions and arithmetic.
+// passed this range test with the same positions and arithmetic (a test
+// here would hold back the loads of the partner's stress until it is done:
+// 43 -> 50 us on 65,536 corotational particles).
 template <bool COROT, bool IN_RANGE = false>
 __device__ __forceinline__ void solid_pair(const SolidConsts &C, const SolidI &II, const SolidSide &J,
                                            Kahan3 &fe_s, Kahan3 &fv_s) {
@@ -946,53 +1205,97 @@ __device__ __forceinline__ void solid_pair(const SolidConsts &C, const SolidI &I
 // walks the masks of the substep's first pair pass, reading the sorted
 // copies; otherwise (a named call) scans every candidate, reading the
 // fields.  Without images the cut-off force equals the force.
-// At most 80 registers (a few bytes spill to L1): six 128-thread blocks per
-// SM instead of five keep more gathers in flight in this latency-bound pass
-// (corotational 0.415 -> 0.383 ms, SVK 0.379 -> 0.344 ms on batched-256).
-template <bool COROT, bool MASKED>
-__global__ void __maxnreg__(80) k_forces_solids(const SceneDesc *__restrict__ scenes, BlockMap map, int fuse_step) {
-    SPH_FOR_WORK(map)
+// Blocks as the first pass's.  A plane's terms are added with Kahan
+// compensation, and the three planes' sums in plane order: in shared memory
+// too, so that the totals hold no registers during the walk (with them in
+// registers 49.2 against 45.1 us on 101,306 SVK particles).
+// At most 80 registers: six 128-thread blocks per SM instead of five keep
+// more gathers in flight in this latency-bound pass.
+template <bool COROT, bool MASKED, bool SPLIT>
+__global__ void __maxnreg__(80)
+    k_forces_solids(const SceneDesc *__restrict__ scenes, BlockMap map, int fuse_step, unsigned per) {
+    extern __shared__ float sums[][6][32];  // per plane (SPLIT), or per warp
+    SPH_FOR_GROUPS(map, per, 32u)
     if (has_planes(S) || (MASKED && !S.sstress)) continue;
-    if (item < active_count(S)) {
-        const unsigned k = item;
-        const unsigned i = min(S.cellparticles[k], S.pnum - 1);
-        const SolidConsts C = solid_consts(S);
-        SolidI I;
-        if (MASKED) side_from_sorted<COROT>(S, k, true, I.side);
-        else side_from_fields<COROT>(S, i, xyz(S.spos[k]), C.mass, I.side);
-        if (COROT) {
-            float R[9];
-            for (int c = 0; c < 9; ++c) R[c] = S.rotation[9 * (size_t)i + c];
-            corot_nmat(R, I.side.s, false, I.M);
-        }
-        Kahan3 fe_s, fv_s;
-        auto visit = [&](unsigned kk) {
-            if (kk == k) return;
-            SolidSide J;
-            if (MASKED) side_from_sorted<COROT>(S, kk, false, J);
-            else side_from_fields<COROT>(S, min(S.cellparticles[kk], S.pnum - 1), xyz(S.spos[kk]), C.mass, J);
-            solid_pair<COROT>(C, I, J, fe_s, fv_s);
-        };
-        // the masks hold neither k itself nor a candidate out of range
-        auto visit_masked = [&](unsigned kk) {
-            SolidSide J;
-            side_from_sorted<COROT>(S, kk, false, J);
-            solid_pair<COROT, true>(C, I, J, fe_s, fv_s);
-        };
-        if (MASKED && S.ncand[k] != SPH_NCAND_SCAN)
-            for_each_masked(S, k, StencilRows(S, S.srow[k]), visit_masked);
-        else
-            for_each_neighbour(S, S.srow[k].x, visit);
-        const float visc = *S.viscosity;
-        const float3 fe = fe_s.get() * 0.5f, fv = fv_s.get() * visc;
-        st3(S.force, i, fe + fv);
-        st3(S.force_elastic, i, fe);
-        st3(S.force_viscous, i, fv);
-        st3(S.cutoff_force, i, fe_s.get() * 0.5f + fv_s.get() * visc);
-        // step_forward for this particle, from the sorted copies of its
-        // position and velocity, which nothing has changed since the gather
-        if (MASKED && fuse_step) integrate(S, i, fe + fv, I.side.vel, I.side.pos);
+    const unsigned n = active_count(S);
+    const unsigned f = SPLIT ? first : first + 32u * threadIdx.y;  // the warp's group
+    if (f >= n) continue;
+    if (SPLIT) __syncthreads();  // the block's last group is done with the sums
+    const int dz0 = SPLIT ? (int)threadIdx.y : 0, dz1 = SPLIT ? dz0 + 1 : 3;
+    const unsigned k = f + threadIdx.x;
+    const bool active = k < n;
+    if (!SPLIT && !active) continue;
+    const unsigned kc = SPLIT ? min(k, n - 1u) : k;
+    const unsigned i = min(S.cellparticles[kc], S.pnum - 1);
+    const SolidConsts C = solid_consts(S);
+    SolidI I;
+    if (MASKED) side_from_sorted<COROT>(S, kc, true, I.side);
+    else side_from_fields<COROT>(S, i, xyz(S.spos[kc]), C.mass, I.side);
+    if (COROT) {
+        float R[9];
+        for (int c = 0; c < 9; ++c) R[c] = S.rotation[9 * (size_t)i + c];
+        corot_nmat(R, I.side.s, false, I.M);
     }
+    float total[6];
+    const StencilRows rows(S, S.srow[kc]);
+    const bool scan = !MASKED || S.ncand[kc] == SPH_NCAND_SCAN;
+#pragma unroll 1
+    for (int dz = dz0; dz < dz1; ++dz) {
+        Kahan3 fe_s, fv_s;
+        if (active) {
+            auto visit = [&](unsigned kk) {
+                SolidSide J;
+                if (MASKED) side_from_sorted<COROT>(S, kk, false, J);
+                else side_from_fields<COROT>(S, min(S.cellparticles[kk], S.pnum - 1), xyz(S.spos[kk]), C.mass, J);
+                solid_pair<COROT>(C, I, J, fe_s, fv_s);
+            };
+            if (scan) {
+                for (int r = 3 * dz; r < 3 * dz + 3; ++r) {
+                    unsigned b, e;
+                    rows.row(S, r, &b, &e);
+                    for (unsigned kk = b; kk < e; ++kk)
+                        if (kk != k) visit(kk);
+                }
+            } else {
+                // the masks hold neither k itself nor a candidate out of range
+                auto visit_masked = [&](unsigned kk) {
+                    SolidSide J;
+                    side_from_sorted<COROT>(S, kk, false, J);
+                    solid_pair<COROT, true>(C, I, J, fe_s, fv_s);
+                };
+                for_each_masked(S, k, rows, visit_masked, 3 * dz, 3 * dz + 3);
+            }
+        }
+        const float v[6] = {fe_s.x.s, fe_s.y.s, fe_s.z.s, fv_s.x.s, fv_s.y.s, fv_s.z.s};
+#pragma unroll
+        for (int c = 0; c < 6; ++c) {
+            if (SPLIT) sums[dz][c][threadIdx.x] = v[c];
+            else {
+                float &t = sums[threadIdx.y][c][threadIdx.x];
+                t = dz == dz0 ? v[c] : __fadd_rn(t, v[c]);
+            }
+        }
+    }
+    if (!SPLIT)
+#pragma unroll
+        for (int c = 0; c < 6; ++c) total[c] = sums[threadIdx.y][c][threadIdx.x];
+    if (SPLIT) {
+        __syncthreads();
+        if (dz0 || !active) continue;
+#pragma unroll
+        for (int c = 0; c < 6; ++c)
+            total[c] = __fadd_rn(__fadd_rn(sums[0][c][threadIdx.x], sums[1][c][threadIdx.x]), sums[2][c][threadIdx.x]);
+    }
+    const float visc = *S.viscosity;
+    const float3 fe_t = make_float3(total[0], total[1], total[2]), fv_t = make_float3(total[3], total[4], total[5]);
+    const float3 fe = fe_t * 0.5f, fv = fv_t * visc;
+    st3(S.force, i, fe + fv);
+    st3(S.force_elastic, i, fe);
+    st3(S.force_viscous, i, fv);
+    st3(S.cutoff_force, i, fe_t * 0.5f + fv_t * visc);
+    // step_forward for this particle, from the sorted copies of its
+    // position and velocity, which nothing has changed since the gather
+    if (MASKED && fuse_step) integrate(S, i, fe + fv, I.side.vel, I.side.pos);
     SPH_END_WORK
 }
 

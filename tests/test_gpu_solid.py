@@ -240,3 +240,39 @@ def test_unset_symmetry_planes_change_nothing(material):
     want = run(False, True)
     for slots, fused in ((True, True), (True, False), (False, False)):
         assert all(np.array_equal(a, b) for a, b in zip(run(slots, fused), want)), (slots, fused)
+
+
+@pytest.mark.parametrize("material", ["corot", "svk"])
+@pytest.mark.parametrize("dims,spacing", [((1, 1, 1), 0.01), ((3, 3, 4), 0.01), ((4, 4, 9), 0.006), ((9, 9, 9), 0.0066),
+                                          ((7, 8, 9), 0.004)])
+def test_solid_rows_split_and_whole(material, dims, spacing):
+    """The first passes' staged rows at their edges -- a lone particle, a
+    last group of one or a few, rows that do not fit the buffer together
+    (about 27 per cell) and rows above 64 candidates (about 125) -- against
+    the oracle, with the stencils split over three warps (the scene alone)
+    and whole (in a batch past the line), which give the same bits."""
+    from sph.batch import Batch
+    sc = scenes.solid_lattice(*dims, spacing=spacing, material=material, youngs_modulus=5e4, jitter=2e-5, seed=3,
+                              clamp_layers=1 if dims[2] > 4 else 0)
+    ps = sc.system()
+    orc = oracle_of(ps)
+    _setup_both(ps, orc)
+    ps.update_fused(3)
+    orc.run(material, 3)
+    ps.sync_device_to_host()
+    n = sc.n
+    if n > 1:  # a lone particle has no stencil to deform (a singular sum)
+        assert rel_err(ps.get_fields("position")[0][:n], orc.a["position"][:n]) <= 1e-5
+        soft = ps.get_fields("body_number")[0][:n] == 0
+        f = "rotation" if material == "corot" else "deformation"
+        assert max_rel(ps.get_fields(f)[0][:n][soft], orc.a[f][:n][soft]) <= 2e-5
+    assert np.array_equal(ps.get_fields("num_neighbours")[0][:n], orc.a["num_neighbours"][:n])
+    b = Batch()
+    sid = b.add(sc)
+    b.add(scenes.wcsph_block(36, 36, 36, jitter=1e-4, seed=2))
+    b.step(3)
+    got = b.read(sid)
+    for f in ("position", "velocity", "force", "stress", "density", "num_neighbours"):
+        assert np.array_equal(got[f], ps.get_fields(f)[0], equal_nan=True), f
+    b.close()
+    ps.close()
