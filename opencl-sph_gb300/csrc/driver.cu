@@ -296,6 +296,7 @@ Store *create_store(psdata *data, const char *file_list, std::string *err) {
     L.all_mixed = L.has_mixed;  // one scene per store
     L.small_grid = sph_small_grid(s->desc.pnum, s->desc.num_cells);
     L.split_rows = sph_split_rows(s->desc.pnum);
+    L.overlap = L.small_grid;
     L.rigid = s->d_rigid;
     L.num_rigid = 0;
     if (!refresh_rigid(s, *data)) {

@@ -13,6 +13,30 @@
 
 #define SPH_SPLIT_PARTICLES 40000ull
 
+// Launches a kernel that begins with follow_previous() (kernels_common.cuh).
+// With L.overlap its blocks may start as the kernel ahead runs out of work,
+// which hides the launch and the blocks' start: a small scene's kernels called
+// by name (three scenes' substeps overlapping / one alone) 20.5 / 56 -> 17.5 /
+// 46.5 us at 8,000 fluid particles, 28.2 / 77.8 -> 21.3 / 57.2 us at 1,539 SVK
+// particles.  Large launches lose by it (65,536 corotational particles 68 ->
+// 96 us): blocks that wait hold the SMs' slots, and start on the split of
+// their memory that the kernel ahead runs with, so only scenes whose grid is
+// one launch overlap (sph_small_grid; 32,768 SVK particles 33 -> 37 us).
+template <class... P, class... A>
+static void sph_launch(const Launch &L, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, A... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = L.stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = L.overlap ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 static inline unsigned grid_for(const BlockMap &m, unsigned cap) {
     unsigned g = m.num < cap ? m.num : cap;
     return g ? g : 1;
@@ -32,8 +56,11 @@ static void small_grid_config(cudaLaunchConfig_t *cfg, cudaLaunchAttribute *at, 
 template <bool GATHER>
 static void launch_grid_small(const Launch &L, bool vel, bool solid) {
     cudaLaunchConfig_t cfg{};
-    cudaLaunchAttribute at[1];
+    cudaLaunchAttribute at[2];
     small_grid_config(&cfg, at, L.stream);
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.numAttrs = L.overlap ? 2 : 1;
     cudaLaunchKernelEx(&cfg, k_grid_small<GATHER>, L.scenes, vel ? 1 : 0, solid ? 1 : 0);
 }
 
@@ -103,35 +130,35 @@ cudaError_t sph_check_launch(const char *what) {
 }
 
 void sph_launch_find_bins(const Launch &L) {
-    k_bin_count<<<grid_for(L.particles, L.grid_cap), L.block, 0, L.stream>>>(L.scenes, L.particles, 0);
+    sph_launch(L, k_bin_count, grid_for(L.particles, L.grid_cap), L.block, 0, L.scenes, L.particles, 0);
 }
 
 void sph_launch_zero_cells(const Launch &L) {
-    k_zero_cells<<<grid_for(L.scan, L.grid_cap), SPH_SCAN_THREADS, 0, L.stream>>>(L.scenes, L.scan);
+    sph_launch(L, k_zero_cells, grid_for(L.scan, L.grid_cap), SPH_SCAN_THREADS, 0, L.scenes, L.scan);
 }
 
 void sph_launch_count(const Launch &L) {
-    k_count_only<<<grid_for(L.particles, L.grid_cap), L.block, 0, L.stream>>>(L.scenes, L.particles);
+    sph_launch(L, k_count_only, grid_for(L.particles, L.grid_cap), L.block, 0, L.scenes, L.particles);
 }
 
 void sph_launch_scan(const Launch &L, bool sums_ready) {
     if (!sums_ready)
-        k_scan_reduce<<<grid_for(L.scan, L.grid_cap), SPH_SCAN_THREADS, 0, L.stream>>>(L.scenes, L.scan);
-    k_scan_down<<<grid_for(L.scan, L.grid_cap), SPH_SCAN_THREADS, 0, L.stream>>>(L.scenes, L.scan);
+        sph_launch(L, k_scan_reduce, grid_for(L.scan, L.grid_cap), SPH_SCAN_THREADS, 0, L.scenes, L.scan);
+    sph_launch(L, k_scan_down, grid_for(L.scan, L.grid_cap), SPH_SCAN_THREADS, 0, L.scenes, L.scan);
 }
 
 void sph_launch_insert(const Launch &L, bool gather, bool vel, bool solid) {
-    k_scatter<<<wide_grid(L.particles.num, L.grid_cap), L.block, 0, L.stream>>>(L.scenes, L.particles);
+    sph_launch(L, k_scatter, wide_grid(L.particles.num, L.grid_cap), L.block, 0, L.scenes, L.particles);
     const unsigned g = grid_for(L.particles, L.grid_cap);
     if (gather)
-        k_rank_cells<true><<<g, L.block, 0, L.stream>>>(L.scenes, L.particles, vel ? 1 : 0, solid ? 1 : 0);
+        sph_launch(L, k_rank_cells<true>, g, L.block, 0, L.scenes, L.particles, vel ? 1 : 0, solid ? 1 : 0);
     else
-        k_rank_cells<false><<<g, L.block, 0, L.stream>>>(L.scenes, L.particles, 0, 0);
+        sph_launch(L, k_rank_cells<false>, g, L.block, 0, L.scenes, L.particles, 0, 0);
 }
 
 void sph_launch_bin_count(const Launch &L) {
     sph_launch_zero_cells(L);
-    k_bin_count<<<grid_for(L.particles, L.grid_cap), L.block, 0, L.stream>>>(L.scenes, L.particles, 1);
+    sph_launch(L, k_bin_count, grid_for(L.particles, L.grid_cap), L.block, 0, L.scenes, L.particles, 1);
 }
 
 void sph_launch_bins(const Launch &L) {
@@ -149,7 +176,7 @@ void sph_launch_bins_gather(const Launch &L, bool vel, bool solid) {
 }
 
 void sph_launch_gather(const Launch &L, bool vel, bool dens, bool solid) {
-    k_gather<<<grid_for(L.particles, L.grid_cap), L.block, 0, L.stream>>>(L.scenes, L.particles, vel ? 1 : 0,
+    sph_launch(L, k_gather, grid_for(L.particles, L.grid_cap), L.block, 0, L.scenes, L.particles, vel ? 1 : 0,
                                                                           dens ? 1 : 0, solid ? 1 : 0);
 }
 
@@ -163,11 +190,9 @@ static unsigned split_grid(const Launch &L, const BlockMap &m) {
 template <bool PLANES, bool COUNT>
 static void launch_density(const Launch &L, const BlockMap &m, int original, int mask, int skip_solids) {
     if (L.split_rows)
-        k_density<PLANES, COUNT, true><<<split_grid(L, m), dim3(32, 3), sizeof(DensityStage<true>), L.stream>>>(
-            L.scenes, m, original, mask, skip_solids, split_per(L));
+        sph_launch(L, k_density<PLANES, COUNT, true>, split_grid(L, m), dim3(32, 3), sizeof(DensityStage<true>), L.scenes, m, original, mask, skip_solids, split_per(L));
     else
-        k_density<PLANES, COUNT><<<grid_for(m, L.grid_cap), L.pair_block, sizeof(DensityStage<false>), L.stream>>>(
-            L.scenes, m, original, mask, skip_solids, 1u);
+        sph_launch(L, k_density<PLANES, COUNT>, grid_for(m, L.grid_cap), L.pair_block, sizeof(DensityStage<false>), L.scenes, m, original, mask, skip_solids, 1u);
 }
 
 void sph_launch_density(const Launch &L, bool original, bool mask, bool skip_solids, bool count) {
@@ -191,11 +216,9 @@ template <bool MIXED>
 static void launch_forces_masked(const Launch &L, int step) {
     const BlockMap &m = L.pair_particles;
     if (L.split_rows)
-        k_forces_fluids_masked<MIXED, true>
-            <<<split_grid(L, m), dim3(32, 3), 0, L.stream>>>(L.scenes, m, step, split_per(L));
+        sph_launch(L, k_forces_fluids_masked<MIXED, true>, split_grid(L, m), dim3(32, 3), 0, L.scenes, m, step, split_per(L));
     else
-        k_forces_fluids_masked<MIXED>
-            <<<grid_for(m, L.grid_cap), L.pair_block, 0, L.stream>>>(L.scenes, m, step, 1u);
+        sph_launch(L, k_forces_fluids_masked<MIXED>, grid_for(m, L.grid_cap), L.pair_block, 0, L.scenes, m, step, 1u);
 }
 
 void sph_launch_forces_fluids(const Launch &L, bool fuse_step, bool masked) {
@@ -205,37 +228,34 @@ void sph_launch_forces_fluids(const Launch &L, bool fuse_step, bool masked) {
         if (!L.all_mixed) launch_forces_masked<false>(L, step);
         if (L.has_mixed) launch_forces_masked<true>(L, step);
     } else {
-        if (!L.all_mixed) k_forces_fluids<false><<<g, L.pair_block, 0, L.stream>>>(L.scenes, L.pair_particles, step);
-        if (L.has_mixed) k_forces_fluids<true><<<g, L.pair_block, 0, L.stream>>>(L.scenes, L.pair_particles, step);
+        if (!L.all_mixed) sph_launch(L, k_forces_fluids<false>, g, L.pair_block, 0, L.scenes, L.pair_particles, step);
+        if (L.has_mixed) sph_launch(L, k_forces_fluids<true>, g, L.pair_block, 0, L.scenes, L.pair_particles, step);
     }
 }
 
 void sph_launch_original_density_mixed(const Launch &L) {
-    k_original_density_mixed<<<grid_for(L.pair_particles, L.grid_cap), L.pair_block, 0, L.stream>>>(
-        L.scenes, L.pair_particles);
+    sph_launch(L, k_original_density_mixed, grid_for(L.pair_particles, L.grid_cap), L.pair_block, 0, L.scenes, L.pair_particles);
 }
 
 void sph_launch_deformations_mixed(const Launch &L, bool masked) {
-    k_deformations_mixed<<<grid_for(L.pair_particles, L.grid_cap), L.pair_block, 0, L.stream>>>(
-        L.scenes, L.pair_particles, masked ? 1 : 0);
+    sph_launch(L, k_deformations_mixed, grid_for(L.pair_particles, L.grid_cap), L.pair_block, 0, L.scenes, L.pair_particles, masked ? 1 : 0);
 }
 
 void sph_launch_forces_solids_mixed(const Launch &L) {
-    k_forces_solids_mixed<<<grid_for(L.pair_particles, L.grid_cap), L.pair_block, 0, L.stream>>>(
-        L.scenes, L.pair_particles);
+    sph_launch(L, k_forces_solids_mixed, grid_for(L.pair_particles, L.grid_cap), L.pair_block, 0, L.scenes, L.pair_particles);
 }
 
 void sph_launch_step_forward(const Launch &L, bool planes_only) {
-    k_step_forward<<<grid_for(L.particles, L.grid_cap), L.block, 0, L.stream>>>(L.scenes, L.particles,
+    sph_launch(L, k_step_forward, grid_for(L.particles, L.grid_cap), L.block, 0, L.scenes, L.particles,
                                                                                 planes_only ? 1 : 0);
 }
 
 void sph_launch_plane_constraints(const Launch &L) {
-    k_plane_constraints<<<grid_for(L.particles, L.grid_cap), L.block, 0, L.stream>>>(L.scenes, L.particles);
+    sph_launch(L, k_plane_constraints, grid_for(L.particles, L.grid_cap), L.block, 0, L.scenes, L.particles);
 }
 
 void sph_launch_init_original_position(const Launch &L) {
-    k_init_original_position<<<grid_for(L.particles, L.grid_cap), L.block, 0, L.stream>>>(L.scenes, L.particles);
+    sph_launch(L, k_init_original_position, grid_for(L.particles, L.grid_cap), L.block, 0, L.scenes, L.particles);
 }
 
 void sph_launch_rotations_and_strains(const Launch &L, bool with_density, bool with_stress) {
@@ -243,23 +263,21 @@ void sph_launch_rotations_and_strains(const Launch &L, bool with_density, bool w
     const unsigned w = L.pair_block / 32u;
     const int d = with_density ? 1 : 0, st = with_density && with_stress ? 1 : 0;
     if (L.split_rows)
-        k_rotations_and_strains<true><<<split_grid(L, L.pair_particles), dim3(32, 3), solid_smem_bytes(true, 3),
-                                        L.stream>>>(L.scenes, L.pair_particles, d, st, split_per(L));
+        sph_launch(L, k_rotations_and_strains<true>, split_grid(L, L.pair_particles), dim3(32, 3), solid_smem_bytes(true, 3), L.scenes, L.pair_particles, d, st, split_per(L));
     else
-        k_rotations_and_strains<false><<<g, dim3(32, w), solid_smem_bytes(false, w), L.stream>>>(
-            L.scenes, L.pair_particles, d, st, 1u);
+        sph_launch(L, k_rotations_and_strains<false>, g, dim3(32, w), solid_smem_bytes(false, w), L.scenes, L.pair_particles, d, st, 1u);
     if (!L.no_symmetry_planes)
-        k_rotations_and_strains_planes<<<g, L.pair_block, 0, L.stream>>>(L.scenes, L.pair_particles);
+        sph_launch(L, k_rotations_and_strains_planes, g, L.pair_block, 0, L.scenes, L.pair_particles);
 }
 
 void sph_launch_stresses(const Launch &L, bool corot, bool sorted, bool planes_only) {
     const unsigned g = grid_for(L.particles, L.grid_cap);
     if (sorted) {
-        if (corot) k_stresses_sorted<true><<<g, L.block, 0, L.stream>>>(L.scenes, L.particles, planes_only ? 1 : 0);
-        else k_stresses_sorted<false><<<g, L.block, 0, L.stream>>>(L.scenes, L.particles, planes_only ? 1 : 0);
+        if (corot) sph_launch(L, k_stresses_sorted<true>, g, L.block, 0, L.scenes, L.particles, planes_only ? 1 : 0);
+        else sph_launch(L, k_stresses_sorted<false>, g, L.block, 0, L.scenes, L.particles, planes_only ? 1 : 0);
     } else {
-        if (corot) k_stresses_corot<<<g, L.block, 0, L.stream>>>(L.scenes, L.particles);
-        else k_stresses_svk<<<g, L.block, 0, L.stream>>>(L.scenes, L.particles);
+        if (corot) sph_launch(L, k_stresses_corot, g, L.block, 0, L.scenes, L.particles);
+        else sph_launch(L, k_stresses_svk, g, L.block, 0, L.scenes, L.particles);
     }
 }
 
@@ -268,12 +286,11 @@ void sph_launch_deformations(const Launch &L, bool with_density, bool with_stres
     const unsigned w = L.pair_block / 32u;
     const int d = with_density ? 1 : 0, st = with_density && with_stress ? 1 : 0;
     if (L.split_rows)
-        k_deformations<true><<<split_grid(L, L.pair_particles), dim3(32, 3), solid_smem_bytes(true, 3), L.stream>>>(
-            L.scenes, L.pair_particles, d, st, split_per(L));
+        sph_launch(L, k_deformations<true>, split_grid(L, L.pair_particles), dim3(32, 3), solid_smem_bytes(true, 3), L.scenes, L.pair_particles, d, st, split_per(L));
     else
-        k_deformations<false><<<g, dim3(32, w), solid_smem_bytes(false, w), L.stream>>>(L.scenes, L.pair_particles, d,
+        sph_launch(L, k_deformations<false>, g, dim3(32, w), solid_smem_bytes(false, w), L.scenes, L.pair_particles, d,
                                                                                        st, 1u);
-    if (!L.no_symmetry_planes) k_deformations_planes<<<g, L.pair_block, 0, L.stream>>>(L.scenes, L.pair_particles);
+    if (!L.no_symmetry_planes) sph_launch(L, k_deformations_planes, g, L.pair_block, 0, L.scenes, L.pair_particles);
 }
 
 template <bool COROT>
@@ -282,13 +299,13 @@ static void launch_forces_solids(const Launch &L, bool masked, int step) {
     const dim3 part(32, 3), whole(32, L.pair_block / 32u);
     const unsigned gp = split_grid(L, m), g = grid_for(m, L.grid_cap), per = split_per(L);
     if (L.split_rows) {
-        if (masked) k_forces_solids<COROT, true, true><<<gp, part, solid_force_smem_bytes(3), L.stream>>>(L.scenes, m, step, per);
-        else k_forces_solids<COROT, false, true><<<gp, part, solid_force_smem_bytes(3), L.stream>>>(L.scenes, m, 0, per);
+        if (masked) sph_launch(L, k_forces_solids<COROT, true, true>, gp, part, solid_force_smem_bytes(3), L.scenes, m, step, per);
+        else sph_launch(L, k_forces_solids<COROT, false, true>, gp, part, solid_force_smem_bytes(3), L.scenes, m, 0, per);
     } else {
-        if (masked) k_forces_solids<COROT, true, false><<<g, whole, solid_force_smem_bytes(whole.y), L.stream>>>(L.scenes, m, step, 1u);
-        else k_forces_solids<COROT, false, false><<<g, whole, solid_force_smem_bytes(whole.y), L.stream>>>(L.scenes, m, 0, 1u);
+        if (masked) sph_launch(L, k_forces_solids<COROT, true, false>, g, whole, solid_force_smem_bytes(whole.y), L.scenes, m, step, 1u);
+        else sph_launch(L, k_forces_solids<COROT, false, false>, g, whole, solid_force_smem_bytes(whole.y), L.scenes, m, 0, 1u);
     }
-    if (!L.no_symmetry_planes) k_forces_solids_planes<COROT><<<g, L.pair_block, 0, L.stream>>>(L.scenes, m);
+    if (!L.no_symmetry_planes) sph_launch(L, k_forces_solids_planes<COROT>, g, L.pair_block, 0, L.scenes, m);
 }
 
 void sph_launch_forces_solids(const Launch &L, bool corot, bool masked, bool fuse_step) {

@@ -15,10 +15,21 @@
 // (fields, grid tables and scratch) untouched.
 __device__ __forceinline__ bool scene_idle(const SceneDesc &S) { return S.steps_left && *S.steps_left == 0u; }
 
+// The start of every kernel that sph_launch (kernels.cu) may start before the
+// kernel ahead of it in the stream has ended: it waits for that end (and for
+// its memory), and only then lets the kernel behind it start in turn, so no
+// more than one launch waits on the SMs.  A launch without that attribute
+// passes straight through.
+__device__ __forceinline__ void follow_previous() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // Iterate the virtual blocks of a segment-aware launch.  Inside the body,
 // `S` is the block's scene and `item` this thread's item index in it.
 // Blocks of idle scenes are skipped (uniformly for the whole block).
 #define SPH_FOR_WORK(map)                                                      \
+    follow_previous();                                                         \
     for (unsigned vb_ = blockIdx.x; vb_ < (map).num; vb_ += gridDim.x) {       \
         const BlockWork bw_ = (map).work[vb_];                                 \
         const SceneDesc &S = scenes[bw_.scene];                                \
@@ -28,6 +39,7 @@ __device__ __forceinline__ bool scene_idle(const SceneDesc &S) { return S.steps_
 // The same with each map entry in `per` groups of `size` items, one group
 // per pass: `first` is the group's first item.
 #define SPH_FOR_GROUPS(map, per, size)                                         \
+    follow_previous();                                                         \
     for (unsigned vb_ = blockIdx.x; vb_ < (map).num * (per); vb_ += gridDim.x) { \
         const BlockWork bw_ = (map).work[vb_ / (per)];                         \
         const SceneDesc &S = scenes[bw_.scene];                                \

@@ -49,6 +49,7 @@ __device__ __forceinline__ void wide_items(const SceneDesc *__restrict__ scenes,
 }
 
 #define SPH_FOR_WIDE(map)                                                                       \
+    follow_previous();                                                                          \
     for (unsigned v0_ = blockIdx.x * SPH_WIDE; v0_ < (map).num; v0_ += gridDim.x * SPH_WIDE) { \
         WideItem W[SPH_WIDE];                                                                   \
         wide_items(scenes, map, v0_, W);
@@ -131,6 +132,7 @@ __global__ void k_bin_count(const SceneDesc *__restrict__ scenes, BlockMap map, 
 // block per scan tile of SPH_SCAN_TILE cells: the counts and the tile's
 // total (which k_bin_count accumulates).
 __global__ void __launch_bounds__(SPH_SCAN_THREADS) k_zero_cells(const SceneDesc *__restrict__ scenes, BlockMap map) {
+    follow_previous();
     for (unsigned vb = blockIdx.x; vb < map.num; vb += gridDim.x) {
         const BlockWork bw = map.work[vb];
         const SceneDesc &S = scenes[bw.scene];
@@ -187,6 +189,7 @@ __device__ __forceinline__ unsigned block_exclusive_scan(unsigned v, unsigned *t
 // Phase 1: each tile's total, from coalesced loads.
 __global__ void __launch_bounds__(SPH_SCAN_THREADS) k_scan_reduce(const SceneDesc *__restrict__ scenes,
                                                                   BlockMap map) {
+    follow_previous();
     for (unsigned vb = blockIdx.x; vb < map.num; vb += gridDim.x) {
         const BlockWork bw = map.work[vb];
         const SceneDesc &S = scenes[bw.scene];
@@ -203,6 +206,7 @@ __global__ void __launch_bounds__(SPH_SCAN_THREADS) k_scan_reduce(const SceneDes
 // Phase 2: each tile adds up the totals of its scene's earlier tiles, then
 // scans its cells through shared memory (coalesced loads and stores).
 __global__ void __launch_bounds__(SPH_SCAN_THREADS) k_scan_down(const SceneDesc *__restrict__ scenes, BlockMap map) {
+    follow_previous();
     __shared__ unsigned tile[SPH_SCAN_TILE];
     constexpr unsigned per = SPH_SCAN_TILE / SPH_SCAN_THREADS;
     for (unsigned vb = blockIdx.x; vb < map.num; vb += gridDim.x) {
@@ -361,6 +365,7 @@ __global__ void k_gather(const SceneDesc *__restrict__ scenes, BlockMap map, int
 template <bool GATHER>
 __global__ void __launch_bounds__(SPH_SMALL_THREADS) k_grid_small(const SceneDesc *__restrict__ scenes, int with_vel,
                                                                   int with_solid) {
+    follow_previous();
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
     __shared__ unsigned totals[SPH_SMALL_BLOCKS];

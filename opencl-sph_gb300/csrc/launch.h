@@ -37,6 +37,9 @@ struct Launch {
     // few particles in all: the pair passes spread a particle's stencil over
     // three warps (sph_split_rows; either way gives the same bits)
     bool split_rows;
+    // small launches that follow each other on one stream: each may start
+    // while the one ahead runs out, and wait for its end on the device
+    bool overlap;
 };
 
 // At most this many rigid bodies per launch (the reduction grid's y extent).
