@@ -29,11 +29,16 @@ static void sph_launch(const Launch &L, void (*kernel)(P...), dim3 grid, dim3 bl
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = L.stream;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute at[2];
     cfg.attrs = at;
-    cfg.numAttrs = L.overlap ? 1 : 0;
+    if (L.overlap) {
+        at[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (L.carveout) {
+        at[cfg.numAttrs].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+        at[cfg.numAttrs++].val.sharedMemCarveout = L.carveout;
+    }
     cudaLaunchKernelEx(&cfg, kernel, P(args)...);
 }
 

@@ -40,6 +40,9 @@ struct Launch {
     // small launches that follow each other on one stream: each may start
     // while the one ahead runs out, and wait for its end on the device
     bool overlap;
+    // kernels of a batch's branches, side by side on the SMs: the split of
+    // the SM's memory they all ask for (percent shared; 0: each its own)
+    int carveout;
 };
 
 // At most this many rigid bodies per launch (the reduction grid's y extent).
