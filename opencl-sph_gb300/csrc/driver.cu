@@ -344,11 +344,11 @@ bool dispatch(Store *s, const char *name) {
     if (k == "insert_particles_in_bin_array") { sph_launch_insert(L); return true; }
     if (k == "compute_density") {
         if ((P & PROG_FLUIDS) && !s->desc.phase && s->desc.nbmask) {
-            // a fluid store: the masked pass (with the count), after a
-            // gather of positions and velocities, so that the next call may
-            // be the masked force pass
+            // a fluid store: the masked pass, after a gather of positions
+            // and velocities, so that the next call may be the masked force
+            // pass
             sph_launch_gather(L, true, false);
-            sph_launch_density(L, false, true, false, true);
+            sph_launch_density(L, false, true);
             s->mask_call = s->calls;
             return true;
         }
@@ -366,7 +366,7 @@ bool dispatch(Store *s, const char *name) {
         if (s->mask_call && s->calls == s->mask_call + 1) {
             // right after the masked compute_density: its sorted copies,
             // pressures, reciprocal densities and masks are current; the
-            // walk gives the scan's bits (and the same neighbour count)
+            // walk gives the scan's bits
             sph_launch_forces_fluids(L, false, true);
             return true;
         }

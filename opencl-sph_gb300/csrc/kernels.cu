@@ -79,8 +79,6 @@ cudaError_t sph_prepare_kernels() {
     const size_t whole = sizeof(DensityStage<false>);
     room((const void *)k_density<false, false>, whole);
     room((const void *)k_density<true, false>, whole);
-    room((const void *)k_density<false, true>, whole);
-    room((const void *)k_density<true, true>, whole);
     const size_t most = solid_smem_bytes(false, 16);  // pair blocks of 512
     room((const void *)k_rotations_and_strains<false>, most);
     room((const void *)k_deformations<false>, most);
@@ -192,29 +190,25 @@ static unsigned split_grid(const Launch &L, const BlockMap &m) {
     return g < L.grid_cap ? (g ? (unsigned)g : 1u) : L.grid_cap;
 }
 
-template <bool PLANES, bool COUNT>
+template <bool PLANES>
 static void launch_density(const Launch &L, const BlockMap &m, int original, int mask, int skip_solids) {
     if (L.split_rows)
-        sph_launch(L, k_density<PLANES, COUNT, true>, split_grid(L, m), dim3(32, 3), sizeof(DensityStage<true>), L.scenes, m, original, mask, skip_solids, split_per(L));
+        sph_launch(L, k_density<PLANES, true>, split_grid(L, m), dim3(32, 3), sizeof(DensityStage<true>), L.scenes, m,
+                   original, mask, skip_solids, split_per(L));
     else
-        sph_launch(L, k_density<PLANES, COUNT>, grid_for(m, L.grid_cap), L.pair_block, sizeof(DensityStage<false>), L.scenes, m, original, mask, skip_solids, 1u);
+        sph_launch(L, k_density<PLANES, false>, grid_for(m, L.grid_cap), L.pair_block, sizeof(DensityStage<false>),
+                   L.scenes, m, original, mask, skip_solids, 1u);
 }
 
-void sph_launch_density(const Launch &L, bool original, bool mask, bool skip_solids, bool count) {
+void sph_launch_density(const Launch &L, bool original, bool mask, bool skip_solids) {
     const int o = original ? 1 : 0, m = mask ? 1 : 0, sk = skip_solids ? 1 : 0;
-    const BlockMap &map = L.pair_particles;
-    if (mask && count) {
-        launch_density<false, true>(L, map, o, m, sk);
-        if (!L.no_symmetry_planes) launch_density<true, true>(L, map, o, m, 0);
-        return;
-    }
-    launch_density<false, false>(L, map, o, m, sk);
-    if (!L.no_symmetry_planes) launch_density<true, false>(L, map, o, m, 0);
+    launch_density<false>(L, L.pair_particles, o, m, sk);
+    if (!L.no_symmetry_planes) launch_density<true>(L, L.pair_particles, o, m, 0);
 }
 
 void sph_launch_density_fused(const Launch &L, const Launch *fluids) {
-    if (fluids && fluids->pair_particles.num) launch_density<false, false>(L, fluids->pair_particles, 0, 1, 1);
-    if (!L.no_symmetry_planes) launch_density<true, false>(L, L.pair_particles, 0, 1, 0);
+    if (fluids && fluids->pair_particles.num) launch_density<false>(L, fluids->pair_particles, 0, 1, 1);
+    if (!L.no_symmetry_planes) launch_density<true>(L, L.pair_particles, 0, 1, 0);
 }
 
 template <bool MIXED>

@@ -183,21 +183,16 @@ struct Kahan3 {
     __device__ __forceinline__ float3 get() const { return make_float3(x.s, y.s, z.s); }
 };
 // Blocked compensated sum of float3 terms: the terms of one stencil row are
-// added in order into a row sum (rounded adds, no compensation), and each
-// row's sum into the total with Kahan compensation.  end_row() closes a row;
-// every walk over a particle's stencil calls it once for each of the nine
-// rows, empty or outside the grid, so that two walks over the same
-// neighbours in the same order give the same bits.
-// The row sum's x and y lanes are one packed FP32x2 add.
+// added in order onto a row sum (one rounding each, no compensation; the x
+// and y lanes packed), and each row's sum into the total with Kahan
+// compensation.  end_row() closes a row; every walk over a particle's
+// stencil calls it once for each of the nine rows, empty or outside the
+// grid, so that two walks over the same neighbours in the same order give
+// the same bits.
 struct BlockSum3 {
     float2 rxy = make_float2(0.f, 0.f);
     float rz = 0.f;
     Kahan3 total;
-    __device__ __forceinline__ void add2(float2 vxy, float vz) {
-        rxy = __fadd2_rn(rxy, vxy);
-        rz = __fadd_rn(rz, vz);
-    }
-    __device__ __forceinline__ void add(float3 v) { add2(make_float2(v.x, v.y), v.z); }
     __device__ __forceinline__ void end_row() {
         total.add(make_float3(rxy.x, rxy.y, rz));
         rxy = make_float2(0.f, 0.f);
@@ -343,11 +338,13 @@ __device__ __forceinline__ unsigned near_bits(const float *__restrict__ p, unsig
 
 // ---- candidate masks -----------------------------------------------------------
 // The first pair pass of a fused substep records, per stencil row r of
-// sorted particle k, which candidates the later passes need: bit t of the
-// row's 64-bit mask is candidate b_r + t; the low word is at
-// nbmask[(2r) * pnum + k], the high word at nbmask[(2r+1) * pnum + k] (only
-// for rows of more than 32 candidates); ncand[k] = SPH_NCAND_SCAN when a
-// row exceeds 64 and the later passes must scan.
+// sorted particle k, which candidates the later passes need: candidate b_r
+// + t is bit 31 - t of the row's low word for t < 32, and bit 63 - t of its
+// high word up to t = 63 (first candidate in the top bit, the order the
+// passes take them in: a leading-zero count finds the next).  The low word
+// is at nbmask[(2r) * pnum + k], the high word at nbmask[(2r+1) * pnum + k]
+// (only for rows of more than 32 candidates); ncand[k] = SPH_NCAND_SCAN when
+// a row exceeds 64 and the later passes must scan.
 
 // Records row r's mask: low word always, high word for rows over 32.
 __device__ __forceinline__ void store_row_mask(const SceneDesc &S, unsigned k, int r, unsigned len, unsigned lo,
@@ -356,17 +353,28 @@ __device__ __forceinline__ void store_row_mask(const SceneDesc &S, unsigned k, i
     if (len > 32u) S.nbmask[(size_t)(2 * r + 1) * S.pnum + k] = hi;
 }
 
-// Row r's mask as recorded, with bits past the row's end cleared (every
-// visited index stays inside [b, e)).
-__device__ __forceinline__ unsigned long long load_row_mask(const SceneDesc &S, unsigned k, int r, unsigned len) {
-    unsigned lo = S.nbmask[(size_t)(2 * r) * S.pnum + k];
-    lo &= len >= 32 ? 0xffffffffu : (1u << len) - 1u;
-    unsigned hi = 0;
-    if (len > 32) {
-        hi = S.nbmask[(size_t)(2 * r + 1) * S.pnum + k];
-        hi &= len >= 64 ? 0xffffffffu : (1u << (len - 32)) - 1u;
-    }
-    return ((unsigned long long)hi << 32) | lo;
+// Bits of the candidates [0, len) of a mask word.
+__device__ __forceinline__ unsigned first_bits(unsigned len) {
+    return len >= 32u ? 0xffffffffu : ~(0xffffffffu >> len);
+}
+
+// A row's mask words as recorded, with bits past the row's end cleared
+// (every visited index stays inside [b, e)).
+struct RowMask {
+    unsigned lo, hi;
+};
+__device__ __forceinline__ RowMask load_row_mask(const SceneDesc &S, unsigned k, int r, unsigned len) {
+    RowMask m;
+    m.lo = S.nbmask[(size_t)(2 * r) * S.pnum + k] & first_bits(len);
+    m.hi = len > 32u ? S.nbmask[(size_t)(2 * r + 1) * S.pnum + k] & first_bits(len - 32u) : 0u;
+    return m;
+}
+
+// The next candidate of a mask word, taken out of it.
+__device__ __forceinline__ unsigned take_first(unsigned &m) {
+    const unsigned t = (unsigned)__clz((int)m);
+    m ^= 0x80000000u >> t;
+    return t;
 }
 
 // Calls f(kk) for the candidates of particle k's recorded masks in rows
@@ -385,35 +393,25 @@ __device__ __forceinline__ void for_each_masked(const SceneDesc &S, unsigned k, 
 #pragma unroll 1
     for (int r = r0; r < r1; ++r) {
         unsigned b, e;
-        unsigned long long mask;
+        RowMask mask;
         if (PREFETCH) {
             b = nb;
             e = ne;
             const unsigned len = e - b;
-            const unsigned lo = nlo & (len >= 32u ? 0xffffffffu : (1u << len) - 1u);
+            mask.lo = nlo & first_bits(len);
             if (r + 1 < r1) {
                 rows.row(S, r + 1, &nb, &ne);
                 nlo = S.nbmask[(size_t)(2 * (r + 1)) * S.pnum + k];
             }
-            unsigned hi = 0;
-            if (len > 32u) {
-                hi = S.nbmask[(size_t)(2 * r + 1) * S.pnum + k];
-                hi &= len >= 64u ? 0xffffffffu : (1u << (len - 32u)) - 1u;
-            }
-            mask = ((unsigned long long)hi << 32) | lo;
+            mask.hi = len > 32u ? S.nbmask[(size_t)(2 * r + 1) * S.pnum + k] & first_bits(len - 32u) : 0u;
         } else {
             rows.row(S, r, &b, &e);
             mask = load_row_mask(S, k, r, e - b);
         }
-        // the row's two mask words in turn, with 32-bit bit scans
+        // the row's two mask words in turn
 #pragma unroll 1
-        for (unsigned w = 0, m = (unsigned)mask; w < 2; ++w, m = (unsigned)(mask >> 32), b += 32) {
-            while (m) {
-                const unsigned t = (unsigned)(__ffs(m) - 1);
-                m &= m - 1u;
-                f(b + t);
-            }
-        }
+        for (unsigned w = 0, m = mask.lo; w < 2; ++w, m = mask.hi, b += 32)
+            while (m) f(b + take_first(m));
     }
 }
 

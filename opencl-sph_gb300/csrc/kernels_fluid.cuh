@@ -47,12 +47,9 @@
 //
 // With `want_mask` (fused fluid substeps, where positions cannot change
 // before the force pass) each fluid particle also records, per row, which
-// candidates lie within h: bit t of row r's 64-bit mask is candidate
-// b_r + t.  The low word goes to nbmask[(2r) * pnum + k], the high word to
-// nbmask[(2r+1) * pnum + k] only when the row holds more than 32
-// candidates; a row of more than 64 marks the particle for a scan
-// (ncand[k] = SPH_NCAND_SCAN).  The stores of one row are one coalesced
-// store per warp.
+// candidates lie within h (kernels_common.cuh, candidate masks).  The stores
+// of one row are one coalesced store per warp.  num_neighbours is the number
+// of set bits, less the few candidates at exactly h.
 // A plane's buffer of 896 candidates holds its ranges: about 440 for 128
 // particles in a lattice of 8 per cell, 820 for 256.
 //
@@ -92,9 +89,7 @@ __device__ __forceinline__ float fluid_pressure(float rho, float rho0, float sti
     return __fmul_rn(__fsub_rn(rho, rho0), stiff);
 }
 
-// COUNT: a masked pass that also counts num_neighbours (a named
-// compute_density, whose caller may read the count before the force pass).
-template <bool PLANES, bool MASK, bool COUNT, bool SPLIT>
+template <bool PLANES, bool MASK, bool SPLIT>
 __device__ __forceinline__ void density_block(const SceneDesc &S, unsigned n, unsigned first,
                                               DensityStage<SPLIT> &stage, int original) {
     constexpr unsigned STAGE = DensityStage<SPLIT>::size;
@@ -170,15 +165,21 @@ __device__ __forceinline__ void density_block(const SceneDesc &S, unsigned n, un
         unsigned hit = m;
 #pragma unroll 1
         while (m) {
-            const unsigned t = __clz(m), bit = 0x80000000u >> t;
-            m ^= bit;
+            const unsigned t = take_first(m);
             const float r2 = dist2(make_float4(src[t], src[STAGE + t], src[2 * STAGE + t], 0.f), nip);
             // beyond h by a rounding: h2 - r2 <= 0 adds nothing
             const float d = fmaxf(h2 - r2, 0.f);
             rowsum = __fadd_rn(rowsum, d * d * d);
-            if (!MASK || PLANES || COUNT) count += r2 <= B.lt;
-            if (MASK && !(r2 <= B.le)) hit ^= bit;
+            if (!(r2 <= B.lt)) {
+                // at h, or beyond by a rounding: not counted
+                --count;
+                if (!(r2 <= B.le)) {
+                    hit ^= 0x80000000u >> t;
+                    ++count;
+                }
+            }
         }
+        count += __popc(hit);
         return hit;
     };
     const int dz0 = SPLIT ? (int)threadIdx.y : 0, dz1 = SPLIT ? dz0 + 1 : 3;
@@ -218,7 +219,7 @@ __device__ __forceinline__ void density_block(const SceneDesc &S, unsigned n, un
                     unsigned m = near_bits<STAGE>(src, min((tot + 3u) >> 2, 8u), nx, ny, nz, nb) & (0xffffffffu >> o);
                     if (tot < 32u) m &= ~(0xffffffffu >> tot);
                     m = walk(m, src, rowsum);
-                    if (MASK) lo = __brev(m) >> o;
+                    lo = m << o;
                 }
 #pragma unroll 1
                 for (unsigned c0 = 32; c0 < tot; c0 += 32) {
@@ -226,15 +227,12 @@ __device__ __forceinline__ void density_block(const SceneDesc &S, unsigned n, un
                     unsigned m = near_bits<STAGE>(src + c0, min((rem + 3u) >> 2, 8u), nx, ny, nz, nb);
                     if (rem < 32u) m &= ~(0xffffffffu >> rem);
                     m = walk(m, src + c0, rowsum);
-                    if (MASK && c0 < 96u) {
-                        // bit t of the row's mask is candidate b + t
-                        const unsigned long long w = (unsigned long long)__brev(m) << (32u - o);
-                        if (c0 == 32u) {
-                            lo |= (unsigned)w;
-                            hi = (unsigned)(w >> 32);
-                        } else {
-                            hi |= (unsigned)w;
-                        }
+                    // candidate b + t at bit 31 - t of the row's mask
+                    if (c0 == 32u) {
+                        lo |= __funnelshift_l(m, 0u, o);
+                        hi = m << o;
+                    } else if (c0 == 64u) {
+                        hi |= __funnelshift_l(m, 0u, o);
                     }
                 }
             } else {
@@ -248,10 +246,9 @@ __device__ __forceinline__ void density_block(const SceneDesc &S, unsigned n, un
                     if (r2 <= B.le) {
                         const float d = fmaxf(h2 - r2, 0.f);
                         rowsum = __fadd_rn(rowsum, d * d * d);
-                        // a fused plane-free substep counts in the force pass
-                        if (!MASK || PLANES || COUNT) count += r2 <= B.lt;
-                        if (MASK && t < 32u) lo |= 1u << t;
-                        if (MASK && t >= 32u && t < 64u) hi |= 1u << (t - 32u);
+                        count += r2 <= B.lt;
+                        if (MASK && t < 32u) lo |= 0x80000000u >> t;
+                        if (MASK && t >= 32u && t < 64u) hi |= 0x80000000u >> (t - 32u);
                     }
                     if (PLANES && P.imask) {
                         const float3 jpos = xyz(j4);
@@ -309,7 +306,7 @@ __device__ __forceinline__ void density_block(const SceneDesc &S, unsigned n, un
             S.density0[i] = value;
         } else {
             S.density[i] = value;
-            if (!MASK || PLANES || COUNT) S.num_neighbours[i] = count;
+            S.num_neighbours[i] = count;
             S.sdens[k] = value;
         }
         if (MASK) {
@@ -332,11 +329,9 @@ __device__ __forceinline__ void density_block(const SceneDesc &S, unsigned n, un
 
 // Two instantiations, each skipping the other's scenes: the plane variant
 // (launched only when some scene has symmetry planes) keeps the common
-// plane-free loop free of its registers.  COUNT: the masked pass counts
-// num_neighbours too (a named compute_density recording masks); a kernel
-// of its own, so the fused substep's keeps its register allocation.
+// plane-free loop free of its registers.
 // SPLIT: blocks of (32, 3) threads, each map entry `per` of them.
-template <bool PLANES, bool COUNT = false, bool SPLIT = false>
+template <bool PLANES, bool SPLIT = false>
 __global__ void __launch_bounds__(SPLIT ? 96 : 512, SPLIT ? 10 : 2)
     k_density(const SceneDesc *__restrict__ scenes, BlockMap map, int original, int want_mask, int skip_solids,
               unsigned per) {
@@ -350,9 +345,9 @@ __global__ void __launch_bounds__(SPLIT ? 96 : 512, SPLIT ? 10 : 2)
     if (first >= n) continue;
     __syncthreads();  // the block's last entry is done with the buffers
     if (want_mask && S.nbmask && (S.programs & PROG_FLUIDS) && !original)
-        density_block<PLANES, true, COUNT, SPLIT>(S, n, first, stage, original);
+        density_block<PLANES, true, SPLIT>(S, n, first, stage, original);
     else
-        density_block<PLANES, false, false, SPLIT>(S, n, first, stage, original);
+        density_block<PLANES, false, SPLIT>(S, n, first, stage, original);
     SPH_END_WORK
 }
 
@@ -388,7 +383,7 @@ struct FluidI {
     float2 nxy, nvxy;  // -ipos and -ivel's x, y lanes (the packed differences)
     float inv_rhoi, pi, h, rho0, stiff;
     float vk, pk;  // visc kv and -kv / 2, the pair term's constant factors
-    float lt, le;
+    float le;
 };
 
 __device__ __forceinline__ FluidI fluid_i(const SceneDesc &S, float3 ipos, float3 ivel, float rhoi) {
@@ -400,7 +395,6 @@ __device__ __forceinline__ FluidI fluid_i(const SceneDesc &S, float3 ipos, float
     I.inv_rhoi = rcp_approx(rhoi);
     const ScenePair B = scene_pair(S);
     I.h = B.h;
-    I.lt = B.lt;
     I.le = B.le;
     I.rho0 = *S.restdens;
     I.stiff = *S.stiffness;
@@ -410,26 +404,41 @@ __device__ __forceinline__ FluidI fluid_i(const SceneDesc &S, float3 ipos, float
     return I;
 }
 
+// 1/sqrt(x) of a normal x from the special-function unit (rsqrtf without
+// its scaling of denormals).
+__device__ __forceinline__ float rsqrt_normal(float x) {
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
 // One neighbour's pressure + viscosity term (fluids.cl:37-56), added to f,
 // from the neighbour's pressure pj and reciprocal density inv_rhoj.  Every
-// rounding is pinned, so the scan and the mask walk produce the same sum.
+// rounding is pinned, so the scan and the mask walk produce the same sum,
+// and a pair's two terms are opposite to the last bit.  (Taking the factors
+// common to all terms out of them and adding with fused multiply-adds saves
+// a tenth of the instructions, but the terms are then rounded with their
+// sums: the momentum of a free mixed scene drifted 4.6 times as far.)
 // Distinct particles at exactly zero distance (and i itself) contribute
-// nothing.  Returns r^2 (the neighbour count's test).  IN_RANGE: the caller
-// walks the density pass's masks, whose candidates passed r^2 <= le with
-// the same positions and arithmetic, so that test is not repeated.
+// nothing.  IN_RANGE: the caller walks the density pass's masks, whose
+// candidates passed r^2 <= le with the same positions and arithmetic, so
+// that test is not repeated.
 template <bool IN_RANGE = false>
-__device__ __forceinline__ float fluid_pair_p(const FluidI &I, float pi, float3 jpos, float3 jvel, float pj,
-                                              float inv_rhoj, BlockSum3 &f) {
+__device__ __forceinline__ void fluid_pair_p(const FluidI &I, float pi, float3 jpos, float3 jvel, float pj,
+                                             float inv_rhoj, BlockSum3 &f) {
     // d = x_j - x_i and r^2 as sub3 and norm2 compute them, the x and y
     // lanes in packed FP32x2 instructions (each lane rounded alike)
     const float2 dxy = __fadd2_rn(make_float2(jpos.x, jpos.y), I.nxy);
     const float dz = __fsub_rn(jpos.z, I.ipos.z);
     const float2 sq = __fmul2_rn(dxy, dxy);
     const float r2 = __fadd_rn(__fadd_rn(sq.x, sq.y), __fmul_rn(dz, dz));
-    if ((!IN_RANGE && !(r2 <= I.le)) || r2 == 0.f) return r2;
-    const float rinv = rsqrtf(r2);
-    const float dist = __fmul_rn(r2, rinv);
-    const float din = __fsub_rn(I.h, dist);
+    if (!IN_RANGE && !(r2 <= I.le)) return;
+    float rinv = rsqrt_normal(r2);
+    if (r2 < 0x1p-126f) {  // zero or denormal
+        if (r2 == 0.f) return;
+        rinv = rsqrtf(r2);
+    }
+    const float din = __fsub_rn(I.h, __fmul_rn(r2, rinv));
     const float inv_didj = __fmul_rn(I.inv_rhoi, inv_rhoj);
     const float vterm = __fmul_rn(din, I.vk);
     const float pterm = __fmul_rn(__fmul_rn(__fmul_rn(__fmul_rn(__fadd_rn(pi, pj), I.pk), rinv), din), din);
@@ -439,14 +448,8 @@ __device__ __forceinline__ float fluid_pair_p(const FluidI &I, float pi, float3 
     const float rvz = __fsub_rn(jvel.z, I.ivel.z);
     const float2 fxy = __fmul2_rn(__ffma2_rn(dxy, make_float2(pterm, pterm), __fmul2_rn(rvxy, make_float2(vterm, vterm))),
                                   make_float2(inv_didj, inv_didj));
-    f.add2(fxy, __fmul_rn(__fmaf_rn(dz, pterm, __fmul_rn(rvz, vterm)), inv_didj));
-    return r2;
-}
-
-template <bool IN_RANGE = false>
-__device__ __forceinline__ float fluid_pair(const FluidI &I, float3 jpos, float3 jvel, float pj, float inv_rhoj,
-                                            BlockSum3 &f) {
-    return fluid_pair_p<IN_RANGE>(I, I.pi, jpos, jvel, pj, inv_rhoj, f);
+    f.rxy = __fadd2_rn(f.rxy, fxy);
+    f.rz = __fadd_rn(f.rz, __fmul_rn(__fmaf_rn(dz, pterm, __fmul_rn(rvz, vterm)), inv_didj));
 }
 
 // The end of a fluid particle's force pass: mass, cube band, store, step.
@@ -479,49 +482,37 @@ __device__ __forceinline__ float3 mixed_extra(const SceneDesc &S, unsigned i, bo
 }
 // One neighbour of the masked force walk, from its position (pressure in
 // w) and velocity (reciprocal density in w, negated for a mixed scene's
-// solid particle); adds to the neighbour count.
+// solid particle).
 template <bool MIXED>
-__device__ __forceinline__ void walk_pair(const FluidI &I, bool solid_i, float4 p, float4 v, BlockSum3 &f,
-                                          unsigned &count) {
+__device__ __forceinline__ void walk_pair(const FluidI &I, bool solid_i, float4 p, float4 v, BlockSum3 &f) {
     if (MIXED) {
         const bool solid_j = v.w < 0.f;
-        if (solid_i && solid_j) {
-            count += norm2(sub3(xyz(p), I.ipos)) <= I.lt;
-            return;
-        }
-        if (solid_i || solid_j) {
-            count += fluid_pair_p<true>(I, fmaxf(I.pi, 0.f), xyz(p), xyz(v), fmaxf(p.w, 0.f), fabsf(v.w), f) <=
-                     I.lt;
-            return;
-        }
+        if (solid_i && solid_j) return;
+        if (solid_i || solid_j)
+            return fluid_pair_p<true>(I, fmaxf(I.pi, 0.f), xyz(p), xyz(v), fmaxf(p.w, 0.f), fabsf(v.w), f);
     }
-    count += fluid_pair<true>(I, xyz(p), xyz(v), p.w, v.w, f) <= I.lt;
+    fluid_pair_p<true>(I, I.pi, xyz(p), xyz(v), p.w, v.w, f);
 }
 
 // The stencil scan: every candidate of the 27 cells, in the reference's
-// order; returns the count of candidates closer than h (j = i included).
+// order.
 template <bool MIXED>
-__device__ __forceinline__ unsigned fluid_scan(const SceneDesc &S, unsigned cell, const FluidI &I, BlockSum3 &f,
-                                               bool solid_i) {
+__device__ __forceinline__ void fluid_scan(const SceneDesc &S, unsigned cell, const FluidI &I, BlockSum3 &f,
+                                           bool solid_i) {
     const float4 *__restrict__ spos = S.spos;
     const float4 *__restrict__ svel = S.svel;
     const float *__restrict__ sdens = S.sdens;
-    unsigned count = 0;
     for_each_neighbour(S, cell, [&](unsigned kk) {
         const bool solid_j = MIXED && S.phase[min(S.cellparticles[kk], S.pnum - 1)] != 0u;
-        if (solid_i && solid_j) {
-            count += norm2(sub3(xyz(spos[kk]), I.ipos)) <= I.lt;
-            return;
-        }
+        if (solid_i && solid_j) return;
         const float rho = sdens[kk];
         float pi = I.pi, pj = fluid_pressure(rho, I.rho0, I.stiff);
         if (MIXED && (solid_i || solid_j)) {
             pi = fmaxf(pi, 0.f);
             pj = fmaxf(pj, 0.f);
         }
-        count += fluid_pair_p(I, pi, xyz(spos[kk]), xyz(svel[kk]), pj, rcp_approx(rho), f) <= I.lt;
+        fluid_pair_p(I, pi, xyz(spos[kk]), xyz(svel[kk]), pj, rcp_approx(rho), f);
     }, [&] { f.end_row(); });
-    return count;
 }
 
 template <bool MIXED>
@@ -545,18 +536,19 @@ __global__ void k_forces_fluids(const SceneDesc *__restrict__ scenes, BlockMap m
 // recorded, row by row and two neighbours at a time, reading each
 // neighbour's position with its pressure in w and its velocity with its
 // reciprocal density in w (two float4 loads).  Lanes whose masks overflowed
-// scan the stencil.  It also counts num_neighbours (the candidates closer
-// than h, j = i included), which the fused density pass of a plane-free
-// scene leaves to it.
-// At most 64 registers: with the current walk 64 beats 56 (0.1886 ->
-// 0.1859 ms at 1M particles), where the earlier walk ran best at 56.
+// scan the stencil.
+// Bound: latency of the gathers (issue slots 64% used; 2 neighbours in
+// flight a thread, 32 warps an SM).  Masks whose first candidate is the top
+// bit (one leading-zero count finds the next), no count of neighbours here
+// and a reciprocal root without denormals' scaling: 132.9M -> 117.1M warp
+// instructions, 162 -> 153 us at 1M particles.
+// At most 64 registers (56: 175 against 168 us with the step at 1M, 72: 174).
 // SPLIT as in the density pass: blocks of (32, 3) threads, a warp per z
-// plane, the row sums added in the same order by the first.
+// plane, the row sums added in the same order by the first; 72 registers.
 template <bool MIXED, bool SPLIT = false>
-__global__ void __maxnreg__(64)
+__global__ void __maxnreg__(SPLIT ? 72 : 64)
     k_forces_fluids_masked(const SceneDesc *__restrict__ scenes, BlockMap map, int fuse_step, unsigned per) {
     __shared__ float rows_sum[SPLIT ? 9 : 1][3][32];
-    __shared__ unsigned rows_count[SPLIT ? 3 : 1][32];
     SPH_FOR_GROUPS(map, SPLIT ? per : 1u, 32u)
     if (MIXED && !S.phase) continue;  // the plain instantiation covers those
     if (!MIXED && S.phase) continue;
@@ -576,10 +568,8 @@ __global__ void __maxnreg__(64)
         const StencilRows rows(S, S.srow[kc]);
         const bool solid_i = mixed_solid<MIXED>(S, i);
         BlockSum3 f;
-        unsigned count = 0;  // num_neighbours, which the density pass left to this one
         const bool scan = S.ncand[kc] == SPH_NCAND_SCAN;
         if (!scan && active) {
-            count = r0 <= 4 && 4 < r1;  // k itself (r^2 = 0), whose mask bit the walk clears
             const float4 *__restrict__ spos = S.spos;
             const float4 *__restrict__ svel = S.svel;
             // two neighbours per iteration: both loads are in flight
@@ -593,35 +583,31 @@ __global__ void __maxnreg__(64)
             for (int r = r0; r < r1; ++r) {
                 unsigned b = nb;
                 const unsigned len = ne - nb;
-                unsigned lo = nlo & (len >= 32u ? 0xffffffffu : (1u << len) - 1u);
+                unsigned lo = nlo & first_bits(len);
                 if (r + 1 < r1) {
                     rows.row(S, r + 1, &nb, &ne);
                     nlo = S.nbmask[(size_t)(2 * (r + 1)) * S.pnum + k];
                 }
-                unsigned hi = 0;
-                if (len > 32u) {
-                    hi = S.nbmask[(size_t)(2 * r + 1) * S.pnum + k];
-                    hi &= len >= 64u ? 0xffffffffu : (1u << (len - 32u)) - 1u;
+                unsigned hi = len > 32u ? S.nbmask[(size_t)(2 * r + 1) * S.pnum + k] & first_bits(len - 32u) : 0u;
+                // k itself (row 4, its own cell's) adds no force
+                if (r == 4) {
+                    const unsigned self = k - b;
+                    if (self < 32u) lo &= ~(0x80000000u >> self);
+                    else if (self < 64u) hi &= ~(0x80000000u >> (self - 32u));
                 }
-                unsigned long long mask = ((unsigned long long)hi << 32) | lo;
-                // k itself (row 4, its own cell's) adds no force and is
-                // counted above
-                if (r == 4 && k - b < 64u) mask &= ~(1ull << (k - b));
-                // the row's two mask words in turn, with 32-bit bit scans
+                // the row's two mask words in turn
 #pragma unroll 1
-                for (unsigned w = 0, m = (unsigned)mask; w < 2; ++w, m = (unsigned)(mask >> 32), b += 32) {
+                for (unsigned w = 0, m = lo; w < 2; ++w, m = hi, b += 32) {
                     while (m) {
-                        const unsigned t1 = (unsigned)(__ffs(m) - 1);
-                        m &= m - 1u;
+                        const unsigned t1 = take_first(m);
                         const float4 p1 = spos[b + t1], v1 = svel[b + t1];
                         if (m) {
-                            const unsigned t2 = (unsigned)(__ffs(m) - 1);
-                            m &= m - 1u;
+                            const unsigned t2 = take_first(m);
                             const float4 p2 = spos[b + t2], v2 = svel[b + t2];
-                            walk_pair<MIXED>(I, solid_i, p1, v1, f, count);
-                            walk_pair<MIXED>(I, solid_i, p2, v2, f, count);
+                            walk_pair<MIXED>(I, solid_i, p1, v1, f);
+                            walk_pair<MIXED>(I, solid_i, p2, v2, f);
                         } else {
-                            walk_pair<MIXED>(I, solid_i, p1, v1, f, count);
+                            walk_pair<MIXED>(I, solid_i, p1, v1, f);
                         }
                     }
                 }
@@ -635,10 +621,9 @@ __global__ void __maxnreg__(64)
                 }
             }
         } else if (active && r0 == 0) {
-            count = fluid_scan<MIXED>(S, rows.cell, I, f, solid_i);
+            fluid_scan<MIXED>(S, rows.cell, I, f, solid_i);
         }
         if (SPLIT) {
-            rows_count[r0 / 3][threadIdx.x] = count;
             __syncthreads();
             if (r0 || !active) continue;
             if (!scan) {
@@ -647,9 +632,7 @@ __global__ void __maxnreg__(64)
                     f.total.add(make_float3(rows_sum[r][0][threadIdx.x], rows_sum[r][1][threadIdx.x],
                                             rows_sum[r][2][threadIdx.x]));
             }
-            count += rows_count[1][threadIdx.x] + rows_count[2][threadIdx.x];
         }
-        if (!has_planes(S)) S.num_neighbours[i] = count;
         fluid_finish(S, i, I, f, fuse_step, mixed_extra<MIXED>(S, i, solid_i));
     }
     SPH_END_WORK

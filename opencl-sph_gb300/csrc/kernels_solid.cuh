@@ -746,32 +746,26 @@ __device__ __forceinline__ void scan_solid_plane(const SceneDesc &S, unsigned fi
                 unsigned w = near;
 #pragma unroll 1
                 while (near) {
-                    const unsigned t = __clz(near), bit = 0x80000000u >> t;
-                    near ^= bit;
+                    const unsigned t = take_first(near), bit = 0x80000000u >> t;
                     if (!add(sub3(make_float3(px[t], px[STAGE + t], px[2 * STAGE + t]), ipos),
                              sub3(make_float3(px0[t], px0[STAGE + t], px0[2 * STAGE + t]), ipos0)))
                         w ^= bit;
                 }
 #pragma unroll 1
                 for (unsigned only = rest & ~w; only;) {
-                    const unsigned t = __clz(only), bit = 0x80000000u >> t;
-                    only ^= bit;
+                    const unsigned t = take_first(only), bit = 0x80000000u >> t;
                     if (dist2(make_float4(px0[t], px0[STAGE + t], px0[2 * STAGE + t], 0.f), nip0) <= C.le) w |= bit;
                 }
                 const unsigned self = k - (b[0] - o + c0);
                 if (self < 32u) w &= ~(0x80000000u >> self);  // k itself has no mask bit
-                w = __brev(w);
-                // bit t of the row's mask is candidate b + t
+                // candidate b + t at bit 31 - t of the row's mask
                 if (c0 == 0) {
-                    lo = w >> o;
-                } else if (c0 < 96u) {
-                    const unsigned long long v = (unsigned long long)w << (32u - o);
-                    if (c0 == 32u) {
-                        lo |= (unsigned)v;
-                        hi = (unsigned)(v >> 32);
-                    } else {
-                        hi |= (unsigned)v;
-                    }
+                    lo = w << o;
+                } else if (c0 == 32u) {
+                    lo |= __funnelshift_l(w, 0u, o);
+                    hi = w << o;
+                } else if (c0 == 64u) {
+                    hi |= __funnelshift_l(w, 0u, o);
                 }
             }
         } else {
@@ -781,8 +775,8 @@ __device__ __forceinline__ void scan_solid_plane(const SceneDesc &S, unsigned fi
                 const bool near = dist2(p4, nip) <= C.le;
                 if (near) add(sub3(xyz(p4), ipos), sub3(xyz(q4), ipos0));
                 if ((near || dist2(q4, nip0) <= C.le) && b[0] + t != k) {
-                    if (t < 32u) lo |= 1u << t;
-                    else if (t < 64u) hi |= 1u << (t - 32u);
+                    if (t < 32u) lo |= 0x80000000u >> t;
+                    else if (t < 64u) hi |= 0x80000000u >> (t - 32u);
                 }
             }
         }

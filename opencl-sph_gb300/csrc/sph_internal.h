@@ -86,12 +86,9 @@ struct SceneDesc {
     // the memory of the candidate masks, which are recorded later
     unsigned *unsorted;
     unsigned *status;         // SphStatus bits
-    // candidate masks (fluids, fused substep): bit t of stencil row r's
-    // 64-bit mask of sorted particle k is set when the row's t-th candidate
-    // lies within h; low word at nbmask[(2r) * pnum + k], high word at
-    // nbmask[(2r+1) * pnum + k] (written only for rows of more than 32
-    // candidates); ncand[k] = candidate count, or SPH_NCAND_SCAN when a row
-    // exceeds 64 and the force pass must scan
+    // candidate masks (kernels_common.cuh), SPH_MASK_WORDS words a particle;
+    // ncand[k] = candidate count, or SPH_NCAND_SCAN when a row exceeds 64 and
+    // the later passes must scan
     unsigned *nbmask;
     unsigned *ncand;
     // written by k_gather for the pair passes after it: per sorted particle
