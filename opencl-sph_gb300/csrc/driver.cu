@@ -391,12 +391,17 @@ bool dispatch(Store *s, const char *name) {
         else sph_launch_density(L, true);
         return true;
     }
+    auto clear_list = [&] {
+        return cuda_ok(cudaMemsetAsync(s->desc.solid_list, 0, 4, s->stream), "solid-phase list");
+    };
     if (mixed && k == "compute_deformations") {
+        if (!clear_list()) return false;
         sph_launch_gather(L, false, false, true);
         sph_launch_deformations_mixed(L, false);
         return true;
     }
     if (mixed && k == "compute_forces_solids") {
+        if (!clear_list()) return false;
         sph_launch_gather(L, false, false, true);
         sph_launch_forces_solids_mixed(L);
         return true;

@@ -2,6 +2,7 @@
 // and the host functions that enqueue them (see launch.h).
 #include <stdio.h>
 
+#include <algorithm>
 #include <atomic>
 
 #include "kernels_fluid.cuh"
@@ -236,12 +237,23 @@ void sph_launch_original_density_mixed(const Launch &L) {
     sph_launch(L, k_original_density_mixed, grid_for(L.pair_particles, L.grid_cap), L.pair_block, 0, L.scenes, L.pair_particles);
 }
 
-void sph_launch_deformations_mixed(const Launch &L, bool masked) {
-    sph_launch(L, k_deformations_mixed, grid_for(L.pair_particles, L.grid_cap), L.pair_block, 0, L.scenes, L.pair_particles, masked ? 1 : 0);
+// Blocks over the solid-phase list, whose length only the device knows: a
+// fixed number at most, which loop over what is left of it.
+#define SPH_LIST_BLOCK 128u
+static unsigned solid_grid(const Launch &L) {
+    const unsigned most = (L.particles.num * L.block + SPH_LIST_BLOCK - 1u) / SPH_LIST_BLOCK;
+    const unsigned cap = std::min(L.grid_cap, 152u * 16u);
+    return most < cap ? (most ? most : 1u) : cap;
 }
 
-void sph_launch_forces_solids_mixed(const Launch &L) {
-    sph_launch(L, k_forces_solids_mixed, grid_for(L.pair_particles, L.grid_cap), L.pair_block, 0, L.scenes, L.pair_particles);
+void sph_launch_deformations_mixed(const Launch &L, bool masked, bool with_stress) {
+    sph_launch(L, k_deformations_mixed, solid_grid(L), SPH_LIST_BLOCK, 0, L.scenes, masked ? 1 : 0,
+               with_stress ? 1 : 0);
+}
+
+void sph_launch_forces_solids_mixed(const Launch &L, bool sorted) {
+    if (sorted) sph_launch(L, k_forces_solids_mixed<true>, solid_grid(L), SPH_LIST_BLOCK, 0, L.scenes);
+    else sph_launch(L, k_forces_solids_mixed<false>, solid_grid(L), SPH_LIST_BLOCK, 0, L.scenes);
 }
 
 void sph_launch_step_forward(const Launch &L, bool planes_only) {
@@ -390,11 +402,9 @@ void sph_launch_substep(const Launch &L, SphMaterial mat, PhaseMark mark, void *
         phase("density");
         sph_launch_density(L, false, true, false);
         phase("deformations (solid phase)");
-        sph_launch_deformations_mixed(L, true);
-        phase("stresses (solid phase)");
-        sph_launch_stresses(L, false);
+        sph_launch_deformations_mixed(L, true, true);
         phase("forces_solids (solid phase)");
-        sph_launch_forces_solids_mixed(L);
+        sph_launch_forces_solids_mixed(L, true);
         phase("forces_fluids+step");
         sph_launch_forces_fluids(L, true, true);
         if (L.num_rigid) {

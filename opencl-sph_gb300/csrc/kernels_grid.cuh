@@ -129,8 +129,9 @@ __global__ void k_bin_count(const SceneDesc *__restrict__ scenes, BlockMap map, 
 }
 
 // zero_gridcount (common.cl:392-400) for every scene of the launch, one
-// block per scan tile of SPH_SCAN_TILE cells: the counts and the tile's
-// total (which k_bin_count accumulates).
+// block per scan tile of SPH_SCAN_TILE cells: the counts, the tile's total
+// (which k_bin_count accumulates) and, once per scene, the length of the
+// solid-phase list (which the gather makes).
 __global__ void __launch_bounds__(SPH_SCAN_THREADS) k_zero_cells(const SceneDesc *__restrict__ scenes, BlockMap map) {
     follow_previous();
     for (unsigned vb = blockIdx.x; vb < map.num; vb += gridDim.x) {
@@ -139,7 +140,10 @@ __global__ void __launch_bounds__(SPH_SCAN_THREADS) k_zero_cells(const SceneDesc
         if (scene_idle(S)) continue;
         const unsigned end = min(bw.first + SPH_SCAN_TILE, S.num_cells);
         for (unsigned c = bw.first + threadIdx.x; c < end; c += blockDim.x) S.gridcount[c] = 0u;
-        if (threadIdx.x == 0) S.scan_sums[bw.first / SPH_SCAN_TILE] = 0u;
+        if (threadIdx.x == 0) {
+            S.scan_sums[bw.first / SPH_SCAN_TILE] = 0u;
+            if (bw.first == 0 && S.solid_list) S.solid_list[0] = 0u;
+        }
     }
 }
 
@@ -297,7 +301,16 @@ __device__ __forceinline__ void gather_one(const SceneDesc &S, unsigned k, unsig
         // rest position, and the body number's bits in w
         const float3 p0 = ld3(S.originalpos, i);
         unsigned w = S.body_number[i];
-        if (S.phase && S.phase[i]) w |= SPH_SOLID_PHASE_BIT;
+        if (S.phase && S.phase[i]) {
+            w |= SPH_SOLID_PHASE_BIT;
+            // the lanes here together append their places to the list
+            namespace cg = cooperative_groups;
+            const cg::coalesced_group g = cg::coalesced_threads();
+            unsigned at = 0;
+            if (g.thread_rank() == 0) at = atomicAdd(S.solid_list, g.size());
+            at = g.shfl(at, 0) + g.thread_rank();
+            if (at < S.pnum) S.solid_list[1 + at] = k;
+        }
         S.spos0[k] = make_float4(p0.x, p0.y, p0.z, __uint_as_float(w));
     }
 }
@@ -375,6 +388,7 @@ __global__ void __launch_bounds__(SPH_SMALL_THREADS) k_grid_small(const SceneDes
     const unsigned rank = cluster.block_rank(), me = rank * SPH_SMALL_THREADS + threadIdx.x;
     const unsigned n = active_count(S), cells = S.num_cells;
     for (unsigned c = me; c < cells; c += threads) S.gridcount[c] = 0u;
+    if (me == 0 && S.solid_list) S.solid_list[0] = 0u;
     unsigned cell[SPH_SMALL_ITEMS], slot[SPH_SMALL_ITEMS];
 #pragma unroll
     for (int j = 0; j < SPH_SMALL_ITEMS; ++j) {

@@ -59,24 +59,54 @@ __device__ __forceinline__ bool solid_partner(float4 q4, unsigned kk, unsigned k
     return kk != k && (__float_as_uint(q4.w) & SPH_SOLID_PHASE_BIT) != 0u;
 }
 
-// f(kk, p4, q4) for particle k's stencil candidates in the reference's
-// order, with the candidate's sorted position and rest position loaded at
-// the top of each step: the row loop is unrolled by 4, so four candidates'
-// loads are in flight before the first one's tests (the solid particles of
-// a mixed scene are too few warps to hide the latency otherwise).
-template <class F>
-__device__ __forceinline__ void for_each_candidate_sorted(const SceneDesc &S, uint2 srow, F &&f) {
-    const StencilRows rows(S, srow);
+// f(kk) for particle k's solid partners kk != k that are within h now, or (REST) at rest, in the reference's order, from the sorted
+// copies: 32 candidates at a time are tested first, exactly and without the
+// work of f, which every lane would otherwise issue whenever any lane of its
+// warp met a partner.
+template <bool REST, class F>
+__device__ __forceinline__ void for_each_partner(const SceneDesc &S, unsigned k, const StencilRows &rows, float3 ipos,
+                                                 float3 ipos0, float le, F &&f) {
     const float4 *__restrict__ spos = S.spos;
     const float4 *__restrict__ spos0 = S.spos0;
+    const NegPoint nip = neg_point(ipos), nip0 = neg_point(ipos0);
 #pragma unroll 1
     for (int r = 0; r < 9; ++r) {
         unsigned b, e;
         rows.row(S, r, &b, &e);
+#pragma unroll 1
+        for (; b < e; b += 32u) {
+            const unsigned cn = min(e - b, 32u);
+            unsigned m = 0;
 #pragma unroll 4
-        for (unsigned kk = b; kk < e; ++kk) f(kk, spos[kk], spos0[kk]);
+            for (unsigned t = 0; t < cn; ++t) {
+                const float4 p = spos[b + t], q = spos0[b + t];
+                const bool in = dist2(p, nip) <= le || (REST && dist2(q, nip0) <= le);
+                if (in && solid_partner(q, b + t, k)) m |= 0x80000000u >> t;
+            }
+#pragma unroll 1
+            while (m) f(b + take_first(m));
+        }
     }
 }
+
+// The solid passes of a mixed scene run over the list of its solid-phase
+// particles (a few percent of a large scene), a thread each, not over every
+// particle.  Mixed scenes run as stores of their own: one scene.
+// Against a thread per particle of the whole scene: deformations with the
+// stresses 38 + 12 -> 37 us, forces 97 -> 82 us for 32,768 solid particles
+// among 1,085,513; the substep 577 -> 550 us, three scenes overlapping 464 -> 433.
+// (Three warps per 32 of them, one per z plane, halve both times, but their
+// sums are then added in another order, and the stresses of an undeformed
+// solid are nothing but the rounding of such sums.)
+#define SPH_FOR_SOLIDS(S, k)                                                                     \
+    follow_previous();                                                                           \
+    const SceneDesc &S = scenes[0];                                                              \
+    if (!S.phase || !S.spos0) return;                                                            \
+    const unsigned solids_ = min(S.solid_list[0], S.pnum);                                       \
+    for (unsigned g_ = blockIdx.x * blockDim.x + threadIdx.x; g_ < solids_;                      \
+         g_ += gridDim.x * blockDim.x) {                                                         \
+        const unsigned k = min(S.solid_list[1 + g_], S.pnum - 1u);
+#define SPH_END_SOLIDS }
 
 // compute_deformations (solid_svk.cl:82-175) of a mixed scene's solid
 // particles over their solid neighbours: F = Apq Aqq^-1 with
@@ -85,50 +115,50 @@ __device__ __forceinline__ void for_each_candidate_sorted(const SceneDesc &S, ui
 // fused substep, after the density pass of the same positions): walks the
 // density pass's candidate masks, which hold exactly the candidates with
 // |p| <= h, in candidate order, so the sums are those of the scan (which a
-// named call runs).
-__global__ void k_deformations_mixed(const SceneDesc *__restrict__ scenes, BlockMap map, int masked) {
-    SPH_FOR_WORK(map)
-    if (!S.phase || !S.spos0) continue;
-    if (item < active_count(S)) {
-        const unsigned k = item;
-        const float4 k0 = S.spos0[k];
-        if (__float_as_uint(k0.w) & SPH_SOLID_PHASE_BIT) {
-            const unsigned i = min(S.cellparticles[k], S.pnum - 1);
-            const SolidConsts C = solid_consts(S);
-            const float3 ipos = xyz(S.spos[k]);
-            const float3 ipos0 = xyz(k0);
-            float apq[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-            float aqq[6] = {0, 0, 0, 0, 0, 0};
-            auto visit = [&](unsigned kk, float4 p4, float4 q4) {
-                if (!solid_partner(q4, kk, k)) return;
-                const float3 p = sub3(xyz(p4), ipos);
-                const float r2 = norm2(p);
-                if (!(r2 <= C.le)) return;
-                const float d = fmaxf(C.h2 - r2, 0.f);
-                const float w = d * d * d;
-                const float3 q = sub3(xyz(q4), ipos0);
-                add_outer(p * w, q, apq);
-                const float3 wq = q * w;
-                aqq[0] = __fmaf_rn(wq.x, q.x, aqq[0]);
-                aqq[1] = __fmaf_rn(wq.y, q.y, aqq[1]);
-                aqq[2] = __fmaf_rn(wq.z, q.z, aqq[2]);
-                aqq[3] = __fmaf_rn(wq.x, q.y, aqq[3]);
-                aqq[4] = __fmaf_rn(wq.x, q.z, aqq[4]);
-                aqq[5] = __fmaf_rn(wq.y, q.z, aqq[5]);
-            };
-            if (masked && S.ncand[k] != SPH_NCAND_SCAN)
-                for_each_masked(S, k, StencilRows(S, S.srow[k]),
-                                [&](unsigned kk) { visit(kk, S.spos[kk], S.spos0[kk]); });
-            else
-                for_each_candidate_sorted(S, S.srow[k], visit);
-            float inv[6];
-            sym_inverse(aqq, inv);
-            float F[9];
-            mul_as(apq, inv, F);
-            for (int c = 0; c < 9; ++c) S.deformation[9 * (size_t)i + c] = F[c];
-        }
+// named call runs).  `with_stress`: also compute_stresses for the particle,
+// as k_stresses_svk would, and the sorted copy of the stress with density0
+// beside it.
+__global__ void k_deformations_mixed(const SceneDesc *__restrict__ scenes, int masked, int with_stress) {
+    SPH_FOR_SOLIDS(S, k)
+    const unsigned i = min(S.cellparticles[k], S.pnum - 1);
+    const SolidConsts C = solid_consts(S);
+    const float3 ipos = xyz(S.spos[k]);
+    const float3 ipos0 = xyz(S.spos0[k]);
+    float a[15] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};  // Apq, then Aqq
+    auto add = [&](float4 p4, float4 q4) {
+        const float3 p = sub3(xyz(p4), ipos);
+        const float d = fmaxf(C.h2 - norm2(p), 0.f);
+        const float w = d * d * d;
+        const float3 q = sub3(xyz(q4), ipos0);
+        add_outer(p * w, q, a);
+        const float3 wq = q * w;
+        a[9] = __fmaf_rn(wq.x, q.x, a[9]);
+        a[10] = __fmaf_rn(wq.y, q.y, a[10]);
+        a[11] = __fmaf_rn(wq.z, q.z, a[11]);
+        a[12] = __fmaf_rn(wq.x, q.y, a[12]);
+        a[13] = __fmaf_rn(wq.x, q.z, a[13]);
+        a[14] = __fmaf_rn(wq.y, q.z, a[14]);
+    };
+    const StencilRows rows(S, S.srow[k]);
+    if (masked && S.ncand[k] != SPH_NCAND_SCAN)
+        for_each_masked(S, k, rows, [&](unsigned kk) {
+            const float4 q4 = S.spos0[kk];
+            if (solid_partner(q4, kk, k)) add(S.spos[kk], q4);
+        });
+    else
+        for_each_partner<false>(S, k, rows, ipos, ipos0, C.le, [&](unsigned kk) { add(S.spos[kk], S.spos0[kk]); });
+    float inv[6], F[9];
+    sym_inverse(a + 9, inv);
+    mul_as(a, inv, F);
+    for (int c = 0; c < 9; ++c) S.deformation[9 * (size_t)i + c] = F[c];
+    if (with_stress) {
+        float o[6];
+        svk_stress(S, F, o);
+        for (int c = 0; c < 6; ++c) S.stress[6 * (size_t)i + c] = o[c];
+        S.sstress[2 * (size_t)k] = make_float4(o[0], o[1], o[2], o[3]);
+        S.sstress[2 * (size_t)k + 1] = make_float4(o[4], o[5], S.density0[i], 0.f);
     }
-    SPH_END_WORK
+    SPH_END_SOLIDS
 }
 
 // compute_forces_solids (solid_svk.cl:182-367) of a mixed scene's solid
@@ -138,53 +168,60 @@ __global__ void k_deformations_mixed(const SceneDesc *__restrict__ scenes, Block
 // force, force_elastic, force_viscous and cutoff_force (no symmetry
 // planes: the cut-off force is the whole force); the fluid force pass then
 // adds the particle's fluid pair terms and steps it.  The candidate tests
-// read the sorted copies (gathered with the rest positions); the fields of
-// j are read for the neighbours only.
-__global__ void k_forces_solids_mixed(const SceneDesc *__restrict__ scenes, BlockMap map) {
-    SPH_FOR_WORK(map)
-    if (!S.phase || !S.spos0) continue;
-    if (item < active_count(S)) {
-        const unsigned k = item;
-        const float4 k0 = S.spos0[k];
-        if (__float_as_uint(k0.w) & SPH_SOLID_PHASE_BIT) {
-            const unsigned i = min(S.cellparticles[k], S.pnum - 1);
-            const SolidConsts C = solid_consts(S);
-            const float3 ipos = xyz(S.spos[k]);
-            const float3 ivel = ld3(S.velocity, i);
-            const float3 ipos0 = xyz(k0);
-            float si[6];
-            for (int c = 0; c < 6; ++c) si[c] = S.stress[6 * (size_t)i + c];
-            const float rho0i = S.density0[i];
-            Kahan3 fe_s, fv_s;
-            for_each_candidate_sorted(S, S.srow[k], [&](unsigned kk, float4 p4, float4 q4) {
-                if (!solid_partner(q4, kk, k)) return;
-                const float3 jpos = xyz(p4);
-                const float3 x = sub3(ipos0, xyz(q4));
-                const float r2 = norm2(sub3(jpos, ipos));
-                if (!(norm2(x) <= C.le || r2 <= C.le)) return;
-                const unsigned j = min(S.cellparticles[kk], S.pnum - 1);
-                const float3 jvel = ld3(S.velocity, j);
-                const float vivj = C.mass * C.mass / rho0i / S.density0[j];
-                const float mrj = C.mass / S.density[j];
-                float sj[6];
-                for (int c = 0; c < 6; ++c) sj[c] = S.stress[6 * (size_t)j + c];
-                const float3 gx = spiky_grad(x, C.h, C.kv, C.le);
-                const float3 f_ji = sym_vec(si, gx) * (-vivj);
-                const bool jbody = (__float_as_uint(q4.w) & ~SPH_SOLID_PHASE_BIT) != 0u;
-                const float3 f_ij = jbody ? -f_ji : sym_vec(sj, -gx) * (-vivj);
-                const float3 fe = f_ij - f_ji;
-                const float lap = r2 <= C.le ? C.kv * (C.h - sqrtf(r2)) : 0.f;
-                const float3 fv = (jvel - ivel) * (mrj * lap);
-                fe_s.add(fe);
-                fv_s.add(fv);
-            });
-            const float visc = S.solid_viscosity ? *S.solid_viscosity : *S.viscosity;
-            const float3 fe = fe_s.get() * 0.5f, fv = fv_s.get() * visc;
-            st3(S.force, i, fe + fv);
-            st3(S.force_elastic, i, fe);
-            st3(S.force_viscous, i, fv);
-            st3(S.cutoff_force, i, fe + fv);
+// read the sorted copies (gathered with the rest positions); a neighbour's
+// velocity, densities and stress come from its sorted copies too in a fused
+// substep (SORTED: those of the density pass and of k_deformations_mixed),
+// from the fields in a named call, the same values.
+template <bool SORTED>
+__global__ void k_forces_solids_mixed(const SceneDesc *__restrict__ scenes) {
+    SPH_FOR_SOLIDS(S, k)
+    const unsigned i = min(S.cellparticles[k], S.pnum - 1);
+    const SolidConsts C = solid_consts(S);
+    const float3 ipos = xyz(S.spos[k]);
+    const float3 ivel = ld3(S.velocity, i);
+    const float3 ipos0 = xyz(S.spos0[k]);
+    float si[6];
+    for (int c = 0; c < 6; ++c) si[c] = S.stress[6 * (size_t)i + c];
+    const float rho0i = S.density0[i];
+    Kahan3 fe_s, fv_s;
+    auto visit = [&](unsigned kk) {
+        const float4 q4 = S.spos0[kk];
+        const float3 jpos = xyz(S.spos[kk]);
+        const float3 x = sub3(ipos0, xyz(q4));
+        const float r2 = norm2(sub3(jpos, ipos));
+        float3 jvel;
+        float sj[6], rho0j, rhoj;
+        if (SORTED) {
+            const float4 s0 = S.sstress[2 * (size_t)kk], s1 = S.sstress[2 * (size_t)kk + 1];
+            jvel = xyz(S.svel[kk]);
+            rhoj = S.sdens[kk];
+            sj[0] = s0.x, sj[1] = s0.y, sj[2] = s0.z, sj[3] = s0.w, sj[4] = s1.x, sj[5] = s1.y;
+            rho0j = s1.z;
+        } else {
+            const unsigned j = min(S.cellparticles[kk], S.pnum - 1);
+            jvel = ld3(S.velocity, j);
+            rho0j = S.density0[j];
+            rhoj = S.density[j];
+            for (int c = 0; c < 6; ++c) sj[c] = S.stress[6 * (size_t)j + c];
         }
-    }
-    SPH_END_WORK
+        const float vivj = C.mass * C.mass / rho0i / rho0j;
+        const float mrj = C.mass / rhoj;
+        const float3 gx = spiky_grad(x, C.h, C.kv, C.le);
+        const float3 f_ji = sym_vec(si, gx) * (-vivj);
+        const bool jbody = (__float_as_uint(q4.w) & ~SPH_SOLID_PHASE_BIT) != 0u;
+        const float3 f_ij = jbody ? -f_ji : sym_vec(sj, -gx) * (-vivj);
+        const float3 fe = f_ij - f_ji;
+        const float lap = r2 <= C.le ? C.kv * (C.h - sqrtf(r2)) : 0.f;
+        const float3 fv = (jvel - ivel) * (mrj * lap);
+        fe_s.add(fe);
+        fv_s.add(fv);
+    };
+    for_each_partner<true>(S, k, StencilRows(S, S.srow[k]), ipos, ipos0, C.le, visit);
+    const float visc = S.solid_viscosity ? *S.solid_viscosity : *S.viscosity;
+    const float3 fe = fe_s.get() * 0.5f, fv = fv_s.get() * visc;
+    st3(S.force, i, fe + fv);
+    st3(S.force_elastic, i, fe);
+    st3(S.force_viscous, i, fv);
+    st3(S.cutoff_force, i, fe + fv);
+    SPH_END_SOLIDS
 }

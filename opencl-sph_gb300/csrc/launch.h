@@ -105,8 +105,11 @@ void sph_launch_forces_solids(const Launch &L, bool corot, bool masked = false, 
 // elastic pair forces of the solid particles over their solid neighbours
 // (the force pass of fluids.cl then adds the fluid-solid pair terms).
 void sph_launch_original_density_mixed(const Launch &L);
-void sph_launch_deformations_mixed(const Launch &L, bool masked);
-void sph_launch_forces_solids_mixed(const Launch &L);
+// (over the solid-phase list of a gather with `solid`, which appends to it:
+// the list is cleared before, by the binning or by the caller)
+void sph_launch_deformations_mixed(const Launch &L, bool masked, bool with_stress = false);
+// sorted: a fused substep, after the passes that fill the sorted copies
+void sph_launch_forces_solids_mixed(const Launch &L, bool sorted = false);
 
 void sph_launch_set_body_position(const Launch &L, unsigned body, const float pos[3]);
 void sph_launch_set_body_rotation(const Launch &L, unsigned body, const float euler[3]);

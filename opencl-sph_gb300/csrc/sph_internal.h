@@ -100,6 +100,9 @@ struct SceneDesc {
     // mass/density), rotation (3 rows of 4 floats); the velocity copy
     // carries 1/density0 in w
     float4 *spos0, *sstress, *srot;
+    // mixed scenes: the number of solid-phase particles and their places in
+    // the sort, in no particular order; made by the gather
+    unsigned *solid_list;
     // batched form only (null otherwise): substeps this scene still takes;
     // at 0 every kernel skips the scene, SPH_STEPS_UNLIMITED never expires
     unsigned *steps_left;

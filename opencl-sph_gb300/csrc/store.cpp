@@ -321,6 +321,10 @@ static size_t solid_bytes(const SceneDesc &d) {
     return Arena::align(16ull * d.pnum) + Arena::align(32ull * d.pnum) + Arena::align(48ull * d.pnum);
 }
 
+// A scene with fluid and solid particles (its `phase` field tells them
+// apart).
+static bool mixed(const SceneDesc &d) { return (d.programs & PROG_FLUIDS) && (d.programs & PROG_SVK); }
+
 size_t sph_scratch_bytes(const SceneDesc &d) {
     size_t P = d.pnum;
     return Arena::align(4 * P)               // slot
@@ -334,6 +338,7 @@ size_t sph_scratch_bytes(const SceneDesc &d) {
            + Arena::align(8 * P)             // srow
            + Arena::align(16 * SPH_PAIR_CONSTS)
            + Arena::align(4)                 // steps_left
+           + (mixed(d) ? Arena::align(4 * (P + 1)) : 0)  // solid_list
            + solid_bytes(d)
            + rigid_bytes(d);
 }
@@ -362,6 +367,11 @@ void sph_place_scratch(SceneDesc *d, char *base) {
     o += Arena::align(16 * SPH_PAIR_CONSTS);
     d->steps_left = reinterpret_cast<unsigned *>(base + o);
     o += Arena::align(4);
+    d->solid_list = nullptr;
+    if (mixed(*d)) {
+        d->solid_list = reinterpret_cast<unsigned *>(base + o);
+        o += Arena::align(4 * (P + 1));
+    }
     d->spos0 = d->sstress = d->srot = nullptr;
     if (d->programs & PROG_SOLIDS) {
         d->spos0 = reinterpret_cast<float4 *>(base + o);

@@ -138,3 +138,32 @@ def test_mixed_scene_conserves_momentum():
     assert abs(pc[1] - pc0[1]) > 0.5 * abs(pc0[1]) and abs(pb[0] - pb0[0]) > 0.5 * abs(pb0[0])
     assert ps.status() == 0
     ps.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("fluid,cube", [((3, 2, 3), (1, 1, 1)), ((6, 4, 6), (3, 3, 3)), ((8, 4, 8), (5, 4, 5)),
+                                        ((26, 26, 26), (9, 9, 9))])
+def test_mixed_solid_list_sizes(fluid, cube):
+    """One solid particle, fewer than a group of 32, a few groups with a
+    remainder, and a scene past the one-launch grid: named kernels give the
+    fused substeps' bits, and the solids match the oracle."""
+    sc = scenes.fluid_solid_scene(fluid=fluid, cube=cube, box=(0.0, 0.6), jitter=1e-4, seed=9, gravity=(0.0, 0.0, 0.0))
+    a, b = sc.system(), sc.system()
+    setup(a)
+    setup(b)
+    o = oracle_of(a)
+    o.setup_solid()
+    a.update_fused(4)
+    for _ in range(4):
+        named_substep(b)
+    o.run("mixed", 4)
+    a.sync_device_to_host()
+    b.sync_device_to_host()
+    n = sc.n
+    # (a lone solid particle's deformation gradient is a singular sum: NaN)
+    for f in ("position", "velocity", "force", "stress", "density"):
+        assert np.array_equal(a.get_fields(f)[0][:n], b.get_fields(f)[0][:n], equal_nan=True), f
+    if np.prod(cube) > 1:
+        assert rel_err(a.get_fields("position")[0][:n], o.a["position"][:n]) <= 1e-5
+    a.close()
+    b.close()
