@@ -499,12 +499,9 @@ void sph_launch_record(const RecordPlan &p, cudaStream_t stream) {
     k_record_tick<<<1, 1, 0, stream>>>(p);
 }
 
-// Segment copy: block row y copies segment y, in 16-byte words where both
-// ends allow, else 4-byte words, else bytes (a grid-stride loop each).
-__global__ void k_copy_segments(const CopySeg *__restrict__ segs, unsigned first) {
-    const CopySeg g = segs[first + blockIdx.y];
-    const size_t stride = (size_t)gridDim.x * blockDim.x;
-    const size_t t0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+// Segment copy by `stride` threads, of which this is thread t0: in 16-byte
+// words where both ends allow, else 4-byte words, else bytes.
+__device__ __forceinline__ void copy_segment(const CopySeg &g, size_t t0, size_t stride) {
     const uintptr_t align = (uintptr_t)g.src | (uintptr_t)g.dst;
     size_t done = 0;
     if ((((uintptr_t)g.src ^ (uintptr_t)g.dst) & 15u) == 0) {
@@ -529,23 +526,22 @@ __global__ void k_copy_segments(const CopySeg *__restrict__ segs, unsigned first
     for (size_t c = done + t0; c < g.bytes; c += stride) g.dst[c] = g.src[c];
 }
 
-// One block copies a few small segments, in 4-byte words where both ends
-// are 4-byte aligned, else bytes.
+// Block row y copies segment y.
+__global__ void k_copy_segments(const CopySeg *__restrict__ segs, unsigned first) {
+    copy_segment(segs[first + blockIdx.y], (size_t)blockIdx.x * blockDim.x + threadIdx.x,
+                 (size_t)gridDim.x * blockDim.x);
+}
 __global__ void k_copy_inline(InlineSegs segs) {
-    for (unsigned q = 0; q < segs.count && q < SPH_INLINE_SEGS; ++q) {
-        const CopySeg g = segs.seg[q];
-        if ((((uintptr_t)g.src | (uintptr_t)g.dst | (uintptr_t)g.bytes) & 3u) == 0) {
-            const unsigned *s = reinterpret_cast<const unsigned *>(g.src);
-            unsigned *d = reinterpret_cast<unsigned *>(g.dst);
-            for (size_t w = threadIdx.x; w < g.bytes / 4; w += blockDim.x) d[w] = s[w];
-        } else {
-            for (size_t c = threadIdx.x; c < g.bytes; c += blockDim.x) g.dst[c] = g.src[c];
-        }
-    }
+    if (blockIdx.y < SPH_INLINE_SEGS)
+        copy_segment(segs.seg[blockIdx.y], (size_t)blockIdx.x * blockDim.x + threadIdx.x,
+                     (size_t)gridDim.x * blockDim.x);
 }
 
 void sph_launch_copy_inline(const InlineSegs &segs, cudaStream_t stream) {
-    k_copy_inline<<<1, 256, 0, stream>>>(segs);
+    // a block per 16 KB: four 16-byte words a thread
+    unsigned long long top = 1;
+    for (unsigned q = 0; q < segs.count; ++q) top = segs.seg[q].bytes > top ? segs.seg[q].bytes : top;
+    k_copy_inline<<<dim3((unsigned)((top + 16383) / 16384), segs.count), 256, 0, stream>>>(segs);
 }
 
 void sph_launch_copy_segments(const CopySeg *segs, unsigned count, unsigned long long max_bytes,
