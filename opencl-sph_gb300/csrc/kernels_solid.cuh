@@ -206,14 +206,16 @@ __device__ __forceinline__ void add_outer(float3 a, float3 b, float *m) {
 }
 
 // Spiky gradient dir(d) * -45/(pi h^6) * (h - |d|)^2, zero beyond h
-// (applyKernelGradient, common.cl:81-87); kv = 45/(pi h^6).
+// (applyKernelGradient, common.cl:81-87); kv = 45/(pi h^6).  Without a
+// branch, which would hold back the loads after it.
 __device__ __forceinline__ float3 spiky_grad(float3 d, float h, float kv, float le) {
-    float r2 = norm2(d);
-    if (!(r2 <= le) || r2 == 0.f) return make_float3(0.f, 0.f, 0.f);
-    float rinv = rsqrtf(r2);
+    const float r2 = norm2(d);
+    const bool in = r2 <= le && r2 != 0.f;
+    const float rinv = rsqrtf(r2);
     const float din = __fsub_rn(h, __fmul_rn(r2, rinv));
     const float s = -kv * din * din * rinv;
-    return d * s;
+    const float3 g = d * s;
+    return make_float3(in ? g.x : 0.f, in ? g.y : 0.f, in ? g.z : 0.f);
 }
 
 struct SolidConsts {
@@ -871,7 +873,7 @@ __device__ __forceinline__ float solid_density(const SceneDesc &S, unsigned i, u
 // computes the density.
 // Against a thread per particle that tests each candidate from the copies as
 // it comes (64 registers, 31.9M warp instructions on 65,536 particles; now
-// 27.5M): 78 -> 72 us there and 112 -> 94 us on 101,306 particles (whole, at
+// 27.5M): 78 -> 65 us there and 112 -> 89 us on 101,306 particles (whole, at
 // most 72 registers: 64 -> 98, 80 -> 93 but fewer warps beside a batch's
 // other branches), and 59 -> 28 us on 4,000 (split; 80 registers).
 template <bool SPLIT>
@@ -949,13 +951,17 @@ __global__ void __maxnreg__(SPLIT ? 80 : 72)
         float a[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
         if (active && !body) {
             // the masks hold no bit for k itself
-            auto pass2_masked = [&](unsigned kk) {
-                const float3 q = sub3(xyz(spos0[kk]), ipos0);
+            // the test selects: as a branch it held back the load of p4 and
+            // the next candidates' (72 -> 65 us)
+            auto pass2_pair = [&](float4 q4, float4 p4) {
+                const float3 q = sub3(xyz(q4), ipos0);
                 const float3 g = spiky_grad(-q, C.h, C.kv, C.le);
-                if (g.x != 0.f || g.y != 0.f || g.z != 0.f) {
-                    const float3 u = mat_t_vec(R, sub3(xyz(spos[kk]), ipos)) - q;
-                    add_outer(u * scale, g, a);
-                }
+                const bool in = g.x != 0.f || g.y != 0.f || g.z != 0.f;
+                const float3 u = (mat_t_vec(R, sub3(xyz(p4), ipos)) - q) * scale;
+                add_outer(make_float3(in ? u.x : 0.f, in ? u.y : 0.f, in ? u.z : 0.f), g, a);
+            };
+            auto pass2_masked = [&](unsigned kk) {
+                pass2_pair(spos0[kk], spos[kk]);
             };
             if (seen.overflow) {
                 for (int r = 3 * dz; r < 3 * dz + 3; ++r) {
