@@ -94,19 +94,17 @@ PHASE_BYTES = {
 # the dominant phase's kernel, from one ncu capture of that kernel alone
 # (one launch after two warm-up substeps, `bench.py --quick --steps 2
 # --warmup 3` of the same workload), taken with the register caps and
-# kernels of this source: k_rotations_and_strains at 64 registers (its
-# spills add DRAM traffic), k_deformations uncapped (80), the solid force
-# passes at 80, the fluid force pass at 64; the density and fluid force passes with their sums blocked per cell
-# row; distance tests and the fluid pair term in packed FP32x2 instructions.
+# kernels of this source: the solid first passes at 72 registers, the solid
+# force passes at 80, the fluid force pass at 64.
 MEASURED_TRAFFIC = {
-    ("wcsph-1m", "density"): 45.20e6,                           # k_density<false>
-    ("wcsph-1m", "forces_fluids+step"): 116.82e6,               # k_forces_fluids_masked<false>
-    ("batched-256", "density"): 262.97e6,                       # k_density<false> (masks, pressure, 1/density too)
-    ("batched-256", "fluid forces+step"): 365.65e6,             # k_forces_fluids_masked<false>
-    ("batched-256", "corotational rotations"): 285.09e6,        # k_rotations_and_strains (with the stress law)
-    ("batched-256", "corotational forces+step"): 241.63e6,      # k_forces_solids<1, 1> (with the step)
-    ("batched-256", "svk deformations"): 105.53e6,              # k_deformations (with the stress law)
-    ("batched-256", "svk forces+step"): 161.73e6,               # k_forces_solids<0, 1> (with the step)
+    ("wcsph-1m", "density"): 60.09e6,                           # k_density<0, 0>
+    ("wcsph-1m", "forces_fluids+step"): 120.14e6,               # k_forces_fluids_masked<0, 0>
+    ("batched-256", "density"): 289.29e6,                       # k_density<0, 0> (masks, counts, pressure, 1/density too)
+    ("batched-256", "fluid forces+step"): 368.96e6,             # k_forces_fluids_masked<0, 0>
+    ("batched-256", "corotational rotations"): 256.55e6,        # k_rotations_and_strains<0> (with the stress law)
+    ("batched-256", "corotational forces+step"): 245.92e6,      # k_forces_solids<1, 1, 0> (with the step)
+    ("batched-256", "svk deformations"): 131.24e6,              # k_deformations<0> (with the stress law)
+    ("batched-256", "svk forces+step"): 165.05e6,               # k_forces_solids<0, 1, 0> (with the step)
 }
 
 # Warp instructions per launch of the same kernels (ncu
@@ -114,14 +112,14 @@ MEASURED_TRAFFIC = {
 # live phase time they give the issue rate, against 4 warp instructions per
 # SM per clock.
 MEASURED_INST = {
-    ("wcsph-1m", "density"): 169.65e6,
-    ("wcsph-1m", "forces_fluids+step"): 141.36e6,
-    ("batched-256", "density"): 430.89e6,
-    ("batched-256", "fluid forces+step"): 363.75e6,
-    ("batched-256", "corotational rotations"): 454.02e6,
-    ("batched-256", "corotational forces+step"): 260.60e6,
-    ("batched-256", "svk deformations"): 347.92e6,
-    ("batched-256", "svk forces+step"): 259.39e6,
+    ("wcsph-1m", "density"): 136.75e6,
+    ("wcsph-1m", "forces_fluids+step"): 117.07e6,
+    ("batched-256", "density"): 353.23e6,
+    ("batched-256", "fluid forces+step"): 300.70e6,
+    ("batched-256", "corotational rotations"): 404.82e6,
+    ("batched-256", "corotational forces+step"): 258.01e6,
+    ("batched-256", "svk deformations"): 301.05e6,
+    ("batched-256", "svk forces+step"): 251.40e6,
 }
 
 

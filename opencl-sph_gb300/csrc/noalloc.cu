@@ -12,7 +12,7 @@
 // sph_compute_particle_bins_noalloc serves them: the caller passes its own
 // device buffers for the inputs and outputs, and the scratch comes from one
 // file-scope device array of fixed size, below.  Every GPU that loads this
-// library holds that array (about 12.3 MB) until the process exits.
+// library holds that array (about 12.2 MiB) until the process exits.
 //
 // The array is shared by every call on a device and keeps the previous
 // call's contents; everything that must start at zero is cleared at the
