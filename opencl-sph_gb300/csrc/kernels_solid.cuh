@@ -1177,7 +1177,11 @@ struct SolidI {
 // passed this range test with the same positions and arithmetic (a test
 // here would hold back the loads of the partner's stress until it is done:
 // 43 -> 50 us on 65,536 corotational particles).
-template <bool COROT, bool IN_RANGE = false>
+// FEW: a split launch, whose few warps wait for their loads: an SVK pair
+// works out both kinds of partner and selects, without a branch (substep of
+// 32,768 particles 32.5 -> 30.7 us; whole launches lose by the work, 101,306
+// particles 75.1 -> 76.1).
+template <bool COROT, bool IN_RANGE = false, bool FEW = false>
 __device__ __forceinline__ void solid_pair(const SolidConsts &C, const SolidI &II, const SolidSide &J,
                                            Kahan3 &fe_s, Kahan3 &fv_s) {
     const SolidSide &I = II.side;
@@ -1192,7 +1196,12 @@ __device__ __forceinline__ void solid_pair(const SolidConsts &C, const SolidI &I
         fe = J.body ? (mat3_vec(J.N, sym_vec(I.s, gx)) + mi) * vivj : (mat3_vec(J.N, gx) + mi) * vivj;
     } else {
         const float3 si = sym_vec(I.s, gx);
-        fe = J.body ? si * (2.f * vivj) : (sym_vec(J.s, gx) + si) * vivj;
+        if (FEW) {
+            const float3 both = (sym_vec(J.s, gx) + si) * vivj, own = si * (2.f * vivj);
+            fe = make_float3(J.body ? own.x : both.x, J.body ? own.y : both.y, J.body ? own.z : both.z);
+        } else {
+            fe = J.body ? si * (2.f * vivj) : (sym_vec(J.s, gx) + si) * vivj;
+        }
     }
     const float dist = r2 > 0.f ? __fmul_rn(r2, rsqrtf(r2)) : 0.f;
     const float lap = r2 <= C.le ? C.kv * (C.h - dist) : 0.f;
@@ -1261,7 +1270,7 @@ __global__ void __maxnreg__(80)
                 auto visit_masked = [&](unsigned kk) {
                     SolidSide J;
                     side_from_sorted<COROT>(S, kk, false, J);
-                    solid_pair<COROT, true>(C, I, J, fe_s, fv_s);
+                    solid_pair<COROT, true, SPLIT>(C, I, J, fe_s, fv_s);
                 };
                 for_each_masked(S, k, rows, visit_masked, 3 * dz, 3 * dz + 3);
             }
