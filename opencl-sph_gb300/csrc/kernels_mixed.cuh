@@ -93,8 +93,8 @@ __device__ __forceinline__ void for_each_partner(const SceneDesc &S, unsigned k,
 // particles (a few percent of a large scene), a thread each, not over every
 // particle.  Mixed scenes run as stores of their own: one scene.
 // Against a thread per particle of the whole scene: deformations with the
-// stresses 38 + 12 -> 37 us, forces 97 -> 82 us for 32,768 solid particles
-// among 1,085,513; the substep 577 -> 550 us, three scenes overlapping 464 -> 433.
+// stresses 38 + 12 -> 29 us, forces 97 -> 82 us for 32,768 solid particles
+// among 1,085,513; the substep 577 -> 542 us, three scenes overlapping 464 -> 431.
 // (Three warps per 32 of them, one per z plane, halve both times, but their
 // sums are then added in another order, and the stresses of an undeformed
 // solid are nothing but the rounding of such sums.)
@@ -125,11 +125,14 @@ __global__ void k_deformations_mixed(const SceneDesc *__restrict__ scenes, int m
     const float3 ipos = xyz(S.spos[k]);
     const float3 ipos0 = xyz(S.spos0[k]);
     float a[15] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};  // Apq, then Aqq
-    auto add = [&](float4 p4, float4 q4) {
+    // a candidate that is no partner adds zeros (its rest position may be
+    // anything): as a branch the test held back the loads after it
+    auto add = [&](float4 p4, float4 q4, bool partner) {
         const float3 p = sub3(xyz(p4), ipos);
         const float d = fmaxf(C.h2 - norm2(p), 0.f);
-        const float w = d * d * d;
-        const float3 q = sub3(xyz(q4), ipos0);
+        const float w = partner ? d * d * d : 0.f;
+        const float3 qj = sub3(xyz(q4), ipos0);
+        const float3 q = make_float3(partner ? qj.x : 0.f, partner ? qj.y : 0.f, partner ? qj.z : 0.f);
         add_outer(p * w, q, a);
         const float3 wq = q * w;
         a[9] = __fmaf_rn(wq.x, q.x, a[9]);
@@ -142,11 +145,11 @@ __global__ void k_deformations_mixed(const SceneDesc *__restrict__ scenes, int m
     const StencilRows rows(S, S.srow[k]);
     if (masked && S.ncand[k] != SPH_NCAND_SCAN)
         for_each_masked(S, k, rows, [&](unsigned kk) {
-            const float4 q4 = S.spos0[kk];
-            if (solid_partner(q4, kk, k)) add(S.spos[kk], q4);
+            const float4 q4 = S.spos0[kk], p4 = S.spos[kk];
+            add(p4, q4, solid_partner(q4, kk, k));
         });
     else
-        for_each_partner<false>(S, k, rows, ipos, ipos0, C.le, [&](unsigned kk) { add(S.spos[kk], S.spos0[kk]); });
+        for_each_partner<false>(S, k, rows, ipos, ipos0, C.le, [&](unsigned kk) { add(S.spos[kk], S.spos0[kk], true); });
     float inv[6], F[9];
     sym_inverse(a + 9, inv);
     mul_as(a, inv, F);

@@ -167,3 +167,29 @@ def test_mixed_solid_list_sizes(fluid, cube):
         assert rel_err(a.get_fields("position")[0][:n], o.a["position"][:n]) <= 1e-5
     a.close()
     b.close()
+
+
+@pytest.mark.gpu
+def test_mixed_fluid_rest_positions_are_not_read():
+    """A fluid particle's rest position may hold anything: the masked
+    deformation pass, which loads it beside its solid partners', adds nothing
+    from it."""
+    def run(junk):
+        ps = scenes.fluid_solid_scene(fluid=(6, 4, 6), cube=(4, 4, 4), box=(0.0, 0.6), jitter=1e-4, seed=9).system()
+        setup(ps)
+        ps.sync_device_to_host()
+        rest, phase = ps.get_fields("originalpos", "phase")
+        fluid = np.asarray(phase) == 0
+        rest[fluid] = junk if junk is not None else rest[fluid]
+        ps.sync_fields_host_to_device("originalpos")
+        ps.update_fused(3)
+        ps.sync_device_to_host()
+        out = [np.array(a) for a in ps.get_fields("position", "velocity", "force", "stress", "deformation")]
+        ps.close()
+        return out, fluid
+    want, fluid = run(None)
+    for junk in (np.nan, np.inf, 3e38):
+        got, _ = run(junk)
+        for a, b in zip(got, want):
+            assert np.array_equal(a, b, equal_nan=True), junk
+    assert np.isfinite(want[3][~fluid]).all()
