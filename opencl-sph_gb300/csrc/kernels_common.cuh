@@ -157,7 +157,6 @@ __device__ __forceinline__ bool has_planes(const SceneDesc &S) {
     return S.num_symmetry_planes != 0u && __float_as_uint(S.pair_consts[1].z) != 0u;
 }
 
-// Kahan-compensated float accumulator.
 // 1/x from the special-function unit (rcp.approx.ftz.f32: at most 1 ulp
 // from the rounded reciprocal, denormals flushed).  One instruction in place
 // of the IEEE-rounded reciprocal's sequence; deterministic, so every walk of
@@ -168,6 +167,7 @@ __device__ __forceinline__ float rcp_approx(float x) {
     return r;
 }
 
+// Kahan-compensated float accumulator.
 struct Kahan {
     float s = 0.f, c = 0.f;
     __device__ __forceinline__ void add(float x) {
@@ -181,6 +181,23 @@ struct Kahan3 {
     Kahan x, y, z;
     __device__ __forceinline__ void add(float3 v) { x.add(v.x); y.add(v.y); z.add(v.z); }
     __device__ __forceinline__ float3 get() const { return make_float3(x.s, y.s, z.s); }
+};
+// Parts of a sum, each with what its own compensation holds back: the parts
+// are added with the exact rounding error of each addition (the two-sum of
+// Knuth, TAOCP vol. 2, 4.2.2), so the total is rounded once, whatever
+// cancels between them.
+struct CompensatedSum {
+    float s, lo;
+    __device__ __forceinline__ CompensatedSum(float s_, float lo_) : s(s_), lo(lo_) {}
+    __device__ __forceinline__ explicit CompensatedSum(const Kahan &k) : s(k.s), lo(-k.c) {}
+    __device__ __forceinline__ void add(const CompensatedSum &o) {
+        const float t = __fadd_rn(s, o.s);
+        const float b = __fsub_rn(t, s);
+        const float err = __fadd_rn(__fsub_rn(s, __fsub_rn(t, b)), __fsub_rn(o.s, b));
+        lo = __fadd_rn(__fadd_rn(lo, o.lo), err);
+        s = t;
+    }
+    __device__ __forceinline__ float get() const { return __fadd_rn(s, lo); }
 };
 // Blocked compensated sum of float3 terms: the terms of one stencil row are
 // added in order onto a row sum (one rounding each, no compensation; the x

@@ -639,7 +639,7 @@ struct SolidScan {  // a particle's counts over the planes scanned
 __host__ __device__ constexpr size_t solid_smem_bytes(bool split, unsigned warps) {
     return sizeof(SolidPlane) * warps + (split ? sizeof(SolidParts) : 0);
 }
-__host__ __device__ constexpr size_t solid_force_smem_bytes(unsigned warps) { return sizeof(float) * 6 * 32 * warps; }
+__host__ __device__ constexpr size_t solid_force_smem_bytes(unsigned warps) { return sizeof(float) * 12 * 32 * warps; }
 
 // Pass 1 over plane dz of particle k's stencil (k of lane threadIdx.x; rows
 // empty for a lane past the scene's end), from the staged copies.  A row is
@@ -1215,15 +1215,18 @@ __device__ __forceinline__ void solid_pair(const SolidConsts &C, const SolidI &I
 // copies; otherwise (a named call) scans every candidate, reading the
 // fields.  Without images the cut-off force equals the force.
 // Blocks as the first pass's.  A plane's terms are added with Kahan
-// compensation, and the three planes' sums in plane order: in shared memory
-// too, so that the totals hold no registers during the walk (with them in
-// registers 49.2 against 45.1 us on 101,306 SVK particles).
+// compensation, and the three planes' sums with their compensations and the
+// exact errors of adding them (CompensatedSum): near equilibrium the two
+// outer planes' sums are large and opposite, and what was dropped between
+// them would be most of the error of the small force that remains.  The
+// totals are kept in shared memory, so that they hold no registers during
+// the walk.
 // At most 80 registers: six 128-thread blocks per SM instead of five keep
 // more gathers in flight in this latency-bound pass.
 template <bool COROT, bool MASKED, bool SPLIT>
 __global__ void __maxnreg__(80)
     k_forces_solids(const SceneDesc *__restrict__ scenes, BlockMap map, int fuse_step, unsigned per) {
-    extern __shared__ float sums[][6][32];  // per plane (SPLIT), or per warp
+    extern __shared__ float sums[][12][32];  // per plane (SPLIT), or per warp: six sums, then their low parts
     SPH_FOR_GROUPS(map, per, 32u)
     if (has_planes(S) || (MASKED && !S.sstress)) continue;
     const unsigned n = active_count(S);
@@ -1275,25 +1278,32 @@ __global__ void __maxnreg__(80)
                 for_each_masked(S, k, rows, visit_masked, 3 * dz, 3 * dz + 3);
             }
         }
-        const float v[6] = {fe_s.x.s, fe_s.y.s, fe_s.z.s, fv_s.x.s, fv_s.y.s, fv_s.z.s};
+        const Kahan v[6] = {fe_s.x, fe_s.y, fe_s.z, fv_s.x, fv_s.y, fv_s.z};
+        float (&to)[12][32] = sums[SPLIT ? dz : (int)threadIdx.y];
 #pragma unroll
         for (int c = 0; c < 6; ++c) {
-            if (SPLIT) sums[dz][c][threadIdx.x] = v[c];
-            else {
-                float &t = sums[threadIdx.y][c][threadIdx.x];
-                t = dz == dz0 ? v[c] : __fadd_rn(t, v[c]);
+            CompensatedSum t(v[c]);
+            if (!SPLIT && dz != dz0) {
+                t = CompensatedSum(to[c][threadIdx.x], to[6 + c][threadIdx.x]);
+                t.add(CompensatedSum(v[c]));
             }
+            to[c][threadIdx.x] = t.s;
+            to[6 + c][threadIdx.x] = t.lo;
         }
     }
-    if (!SPLIT)
-#pragma unroll
-        for (int c = 0; c < 6; ++c) total[c] = sums[threadIdx.y][c][threadIdx.x];
     if (SPLIT) {
         __syncthreads();
         if (dz0 || !active) continue;
+    }
 #pragma unroll
-        for (int c = 0; c < 6; ++c)
-            total[c] = __fadd_rn(__fadd_rn(sums[0][c][threadIdx.x], sums[1][c][threadIdx.x]), sums[2][c][threadIdx.x]);
+    for (int c = 0; c < 6; ++c) {
+        auto part = [&](unsigned q) { return CompensatedSum(sums[q][c][threadIdx.x], sums[q][6 + c][threadIdx.x]); };
+        CompensatedSum t = part(SPLIT ? 0u : threadIdx.y);
+        if (SPLIT) {
+            t.add(part(1));
+            t.add(part(2));
+        }
+        total[c] = t.get();
     }
     const float visc = *S.viscosity;
     const float3 fe_t = make_float3(total[0], total[1], total[2]), fv_t = make_float3(total[3], total[4], total[5]);
