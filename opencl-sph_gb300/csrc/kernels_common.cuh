@@ -170,8 +170,10 @@ __device__ __forceinline__ float rcp_approx(float x) {
 // Kahan-compensated float accumulator.
 struct Kahan {
     float s = 0.f, c = 0.f;
-    __device__ __forceinline__ void add(float x) {
-        float y = __fsub_rn(x, c);
+    __device__ __forceinline__ void add(float x) { add_rounded(__fsub_rn(x, c)); }
+    // a b, rounded with its addition
+    __device__ __forceinline__ void add_product(float a, float b) { add_rounded(__fmaf_rn(a, b, -c)); }
+    __device__ __forceinline__ void add_rounded(float y) {
         float t = __fadd_rn(s, y);
         c = __fsub_rn(__fsub_rn(t, s), y);
         s = t;
@@ -180,12 +182,17 @@ struct Kahan {
 struct Kahan3 {
     Kahan x, y, z;
     __device__ __forceinline__ void add(float3 v) { x.add(v.x); y.add(v.y); z.add(v.z); }
+    __device__ __forceinline__ void add_product(float3 v, float w) {
+        x.add_product(v.x, w);
+        y.add_product(v.y, w);
+        z.add_product(v.z, w);
+    }
     __device__ __forceinline__ float3 get() const { return make_float3(x.s, y.s, z.s); }
 };
 // Parts of a sum, each with what its own compensation holds back: the parts
 // are added with the exact rounding error of each addition (the two-sum of
-// Knuth, TAOCP vol. 2, 4.2.2), so the total is rounded once, whatever
-// cancels between them.
+// Knuth, TAOCP vol. 2, 4.2.2), so the total is rounded once, with its factor,
+// whatever cancels between them.
 struct CompensatedSum {
     float s, lo;
     __device__ __forceinline__ CompensatedSum(float s_, float lo_) : s(s_), lo(lo_) {}
@@ -197,7 +204,8 @@ struct CompensatedSum {
         lo = __fadd_rn(__fadd_rn(lo, o.lo), err);
         s = t;
     }
-    __device__ __forceinline__ float get() const { return __fadd_rn(s, lo); }
+    // the sum times a factor
+    __device__ __forceinline__ float times(float w) const { return __fmaf_rn(s, w, __fmul_rn(lo, w)); }
 };
 // Blocked compensated sum of float3 terms: the terms of one stencil row are
 // added in order onto a row sum (one rounding each, no compensation; the x

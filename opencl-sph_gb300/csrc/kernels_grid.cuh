@@ -281,7 +281,7 @@ __global__ void k_scatter(const SceneDesc *__restrict__ scenes, BlockMap map) {
 // Cell-sorted copies of particle i at place k: spos = position (and velocity,
 // density when asked; for solids also the rest position with the body
 // number -- and in a mixed scene SPH_SOLID_PHASE_BIT for a solid-phase
-// particle -- and 1/density0 in the velocity copy's w), so that the pair
+// particle -- and mass/density0 in the velocity copy's w), so that the pair
 // loops stream float4s.  Also what every pair pass would otherwise work out
 // again in each thread, while this memory-bound work leaves issue slots to
 // spare: the particle's stencil rows (srow) and the scene's constants
@@ -295,7 +295,7 @@ __device__ __forceinline__ void gather_one(const SceneDesc &S, unsigned k, unsig
     S.spos[k] = make_float4(p.x, p.y, p.z, 0.f);
     S.srow[k] = make_uint2(cell, StencilRows(S, cell).bits);
     if (k == 0) write_scene_pair(S);
-    if (with_vel || solid) S.svel[k] = make_float4(v.x, v.y, v.z, solid ? __frcp_rn(S.density0[i]) : 0.f);
+    if (with_vel || solid) S.svel[k] = make_float4(v.x, v.y, v.z, solid ? __fdiv_rn(*S.mass, S.density0[i]) : 0.f);
     if (with_dens) S.sdens[k] = S.density[i];
     if (solid) {
         // rest position, and the body number's bits in w

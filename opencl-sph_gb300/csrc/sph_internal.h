@@ -98,7 +98,7 @@ struct SceneDesc {
     // solids: cell-sorted copies for the fused substep's pair passes --
     // rest position (w: body_number bits), stress (6 floats, then
     // mass/density), rotation (3 rows of 4 floats); the velocity copy
-    // carries 1/density0 in w
+    // carries mass/density0 in w
     float4 *spos0, *sstress, *srot;
     // mixed scenes: the number of solid-phase particles and their places in
     // the sort, in no particular order; made by the gather

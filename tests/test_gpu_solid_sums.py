@@ -44,3 +44,55 @@ def test_equilibrium_forces_keep_the_sums_compensation(material, dims):
     ps.close()
     rms = np.sqrt(np.mean(left)) * 2.0 ** 24
     assert rms <= 0.14, rms
+
+
+# A store whose plane slots are unset takes the plane-free pair term; with a
+# plane set that no particle is near, the plane variant's, whose volume
+# factor is divided out and whose distance is a correctly rounded root.  The
+# plane-free term must round no more.  One scene's ratio of the two errors
+# against 64 bits varies by 0.085 with the mantissas that its spacing and
+# density give the volumes, so the geometric mean over 24 scenes has a
+# standard error of 0.017; the bound is two of them above 1.
+@pytest.mark.parametrize("material", ["corot", "svk"])
+def test_plane_free_pair_term_rounds_no_more_than_the_divided_one(material):
+    from oracle.oracle import OracleScene
+    from sph import bindings as bnd
+    first = "compute_rotations_and_strains" if material == "corot" else "compute_deformations"
+    fields = ("force_elastic", "force_viscous")
+    ratios = {f: [] for f in fields}
+    for q in range(24):
+        errors = {}
+        for plane in (False, True):
+            d = 0.01 * (1 + 0.047 * q)
+            sc = scenes.solid_lattice(12, 12, 12, spacing=d, h=2 * d, density=1000.0 * 1.037 ** q, material=material,
+                                      youngs_modulus=5e4, jitter=0.04 * d, seed=5 + q, clamp_layers=q % 2)
+            sc.entries = [("symmetry_planes", "3, 2, 3", "float", None) if e[0] == "symmetry_planes" else e
+                          for e in sc.entries]
+            ps = sc.system()
+            n = sc.n
+            ps.call_for_all_particles("init_original_position")
+            ps.compute_particle_bins()
+            ps.call_for_all_particles("compute_original_density")
+            rng = np.random.default_rng(3 + q)
+            x = ps.get_fields("position")[0][:n] + rng.uniform(-1, 1, size=(n, 3)) * d * (0.1 if q % 2 else 1e-3)
+            ps.set_fields(position=x.astype(np.float32), velocity=rng.normal(0, 0.1, (n, 3)).astype(np.float32))
+            if plane:
+                sp = np.zeros((3, 2, 3), np.float32)
+                sp[0, 0, 1], sp[0, 1, 1] = -50.0, 1.0
+                ps.set_fields(symmetry_planes=sp)
+            ps.compute_particle_bins()
+            for call in ("compute_density", first, "compute_stresses"):
+                ps.call_for_all_particles(call)
+            ps.sync_device_to_host()
+            o = OracleScene(bnd.store_views(ps.psdata), "f64", nthreads=4)
+            o.call("compute_particle_bins")
+            o.call("compute_forces_solids_" + material)
+            ps.call_for_all_particles("compute_forces_solids")
+            ps.sync_device_to_host()
+            for f in fields:
+                errors[f, plane] = np.sqrt(np.mean((ps.get_fields(f)[0][:n] - o.a[f].reshape(-1, 3)[:n]) ** 2))
+            ps.close()
+        for f in fields:
+            ratios[f].append(np.log(errors[f, False] / errors[f, True]))
+    for f in fields:
+        assert np.exp(np.mean(ratios[f])) <= 1.035, (f, np.exp(np.mean(ratios[f])))
