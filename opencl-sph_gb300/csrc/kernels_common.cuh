@@ -19,7 +19,11 @@ __device__ __forceinline__ bool scene_idle(const SceneDesc &S) { return S.steps_
 // kernel ahead of it in the stream has ended: it waits for that end (and for
 // its memory), and only then lets the kernel behind it start in turn, so no
 // more than one launch waits on the SMs.  A launch without that attribute
-// passes straight through.
+// passes straight through.  A waiting kernel is on the SMs while the one
+// ahead still writes, so such kernels read with ordinary loads: the
+// non-coherent ones (__ldg, const __restrict__ parameters) are only for
+// memory that nothing writes while the kernel lives, which here is the scene
+// table and the block maps.
 __device__ __forceinline__ void follow_previous() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -260,16 +264,16 @@ __device__ __forceinline__ void for_each_neighbour(const SceneDesc &S, unsigned 
     const unsigned cx = rem - cy * R0;
     const unsigned x0 = cx > 0 ? cx - 1 : 0;
     const unsigned x1 = cx + 1 < R0 ? cx + 1 : R0 - 1;
-    const unsigned *__restrict__ off = S.celloffset;
-    const unsigned *__restrict__ cnt = S.gridcount;
+    const unsigned *off = S.celloffset;
+    const unsigned *cnt = S.gridcount;
     for (int dz = -1; dz <= 1; ++dz) {
         int z = (int)cz + dz;
         for (int dy = -1; dy <= 1; ++dy) {
             int y = (int)cy + dy;
             if (z >= 0 && z < (int)R2 && y >= 0 && y < (int)R1) {
                 unsigned row = (unsigned)z * layer + (unsigned)y * R0;
-                unsigned b = __ldg(off + row + x0);
-                unsigned e = __ldg(off + row + x1) + __ldg(cnt + row + x1);
+                unsigned b = off[row + x0];
+                unsigned e = off[row + x1] + cnt[row + x1];
                 if (e > S.pnum) e = S.pnum;  // only reachable with inconsistent host-written tables
                 for (unsigned kk = b; kk < e; ++kk) f(kk);
             }
@@ -324,8 +328,8 @@ struct StencilRows {
         const int dz = r / 3 - 1, dy = r % 3 - 1;
         const unsigned c = (unsigned)((int)cell + dz * (int)layer + dy * (int)R0);
         const unsigned x0 = c - ((bits >> (9 + r)) & 1u), x1 = c + ((bits >> (18 + r)) & 1u);
-        unsigned bb = __ldg(S.celloffset + x0);
-        unsigned ee = __ldg(S.celloffset + x1) + __ldg(S.gridcount + x1);
+        unsigned bb = S.celloffset[x0];
+        unsigned ee = S.celloffset[x1] + S.gridcount[x1];
         if (ee > S.pnum) ee = S.pnum;  // only with inconsistent host-written tables
         if (bb > ee) bb = ee;
         *b = bb;

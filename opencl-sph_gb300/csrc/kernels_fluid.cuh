@@ -98,7 +98,7 @@ __device__ __forceinline__ void density_block(const SceneDesc &S, unsigned n, un
     const bool active = k < n;
     const ScenePair B = scene_pair(S);
     const float h = B.h, h2 = B.h2;
-    const float4 *__restrict__ spos = S.spos;
+    const float4 *spos = S.spos;
     const unsigned pnum = S.pnum;
     const StencilRows rows(S, active ? S.srow[k] : make_uint2(0u, 0u));
     if (flat < 9u) {
@@ -499,9 +499,9 @@ __device__ __forceinline__ void walk_pair(const FluidI &I, bool solid_i, float4 
 template <bool MIXED>
 __device__ __forceinline__ void fluid_scan(const SceneDesc &S, unsigned cell, const FluidI &I, BlockSum3 &f,
                                            bool solid_i) {
-    const float4 *__restrict__ spos = S.spos;
-    const float4 *__restrict__ svel = S.svel;
-    const float *__restrict__ sdens = S.sdens;
+    const float4 *spos = S.spos;
+    const float4 *svel = S.svel;
+    const float *sdens = S.sdens;
     for_each_neighbour(S, cell, [&](unsigned kk) {
         const bool solid_j = MIXED && S.phase[min(S.cellparticles[kk], S.pnum - 1)] != 0u;
         if (solid_i && solid_j) return;
@@ -570,8 +570,8 @@ __global__ void __maxnreg__(SPLIT ? 72 : 64)
         BlockSum3 f;
         const bool scan = S.ncand[kc] == SPH_NCAND_SCAN;
         if (!scan && active) {
-            const float4 *__restrict__ spos = S.spos;
-            const float4 *__restrict__ svel = S.svel;
+            const float4 *spos = S.spos;
+            const float4 *svel = S.svel;
             // two neighbours per iteration: both loads are in flight
             // before the first pair's arithmetic (same order)
             // the next row's bounds and low mask word are loaded while this

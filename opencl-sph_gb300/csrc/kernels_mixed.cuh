@@ -66,8 +66,8 @@ __device__ __forceinline__ bool solid_partner(float4 q4, unsigned kk, unsigned k
 template <bool REST, class F>
 __device__ __forceinline__ void for_each_partner(const SceneDesc &S, unsigned k, const StencilRows &rows, float3 ipos,
                                                  float3 ipos0, float le, F &&f) {
-    const float4 *__restrict__ spos = S.spos;
-    const float4 *__restrict__ spos0 = S.spos0;
+    const float4 *spos = S.spos;
+    const float4 *spos0 = S.spos0;
     const NegPoint nip = neg_point(ipos), nip0 = neg_point(ipos0);
 #pragma unroll 1
     for (int r = 0; r < 9; ++r) {

@@ -679,8 +679,8 @@ __device__ __forceinline__ void scan_solid_plane(const SceneDesc &S, unsigned fi
                                                  const SolidConsts &C, SolidPlane &stage, SolidScan &seen, Sum &&sum,
                                                  RowEnd &&row_end) {
     constexpr unsigned STAGE = SPH_SOLID_STAGE;
-    const float4 *__restrict__ spos = S.spos;
-    const float4 *__restrict__ spos0 = S.spos0;
+    const float4 *spos = S.spos;
+    const float4 *spos0 = S.spos0;
     const unsigned lane = threadIdx.x, k = first + lane, pnum = S.pnum;
     unsigned b[3], e[3], ua[3], at[4];
     at[0] = 0;
@@ -955,8 +955,8 @@ __global__ void __maxnreg__(SPLIT ? 80 : 72)
         for (int c = 0; c < 9; ++c) R[c] = stages[0].x0[32 * c + threadIdx.x];
     }
     float D[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-    const float4 *__restrict__ spos = S.spos;
-    const float4 *__restrict__ spos0 = S.spos0;
+    const float4 *spos = S.spos;
+    const float4 *spos0 = S.spos0;
     const float scale = C.mass / S.density0[i];
 #pragma unroll 1
     for (int dz = dz0; dz < dz1; ++dz) {
