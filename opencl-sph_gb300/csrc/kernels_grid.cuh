@@ -315,34 +315,107 @@ __device__ __forceinline__ void gather_one(const SceneDesc &S, unsigned k, unsig
     }
 }
 
+// A cell of m of the scene's n particles is crowded when one walk over all n
+// particles' cells (0.5 ns each by a block) orders it faster than comparing
+// its particles with each other (26 ns a step, m steps a thread).  So there
+// are few such cells: one may start in each 257 entries, 48 in a scene.
+__device__ __forceinline__ bool crowded_cell(unsigned m, unsigned n) { return m > 256u + n / 48u; }
+
+// A crowded cell in canonical order (and, GATHER, its sorted copies), by the
+// whole block: the particles' cells in index order, a run of 32 x
+// SPH_CROWD_ITEMS a warp.
+#define SPH_CROWD_ITEMS 16
+template <bool GATHER>
+__device__ __noinline__ void order_crowded_cell(const SceneDesc &S, unsigned cell, unsigned n, int with_vel,
+                                                int with_solid) {
+    __shared__ unsigned found[32];
+    const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    const unsigned off = S.celloffset[cell], cnt = S.gridcount[cell];
+    const unsigned *cells = S.gridcell;
+    unsigned r = off;
+    for (unsigned i0 = 0; i0 < n; i0 += blockDim.x * SPH_CROWD_ITEMS) {
+        const unsigned i = i0 + warp * 32u * SPH_CROWD_ITEMS + lane;
+        unsigned at[SPH_CROWD_ITEMS], hit = 0;
+#pragma unroll
+        for (unsigned j = 0; j < SPH_CROWD_ITEMS; ++j) at[j] = cells[min(i + 32u * j, n - 1u)];
+#pragma unroll
+        for (unsigned j = 0; j < SPH_CROWD_ITEMS; ++j)
+            hit |= (unsigned)(i + 32u * j < n && at[j] == cell) << j;
+        const unsigned mine = __reduce_add_sync(SPH_FULL_MASK, __popc(hit));
+        __syncthreads();
+        if (lane == 0) found[warp] = mine;
+        __syncthreads();
+        const unsigned f = lane < warps ? found[lane] : 0u;
+        unsigned to = r + __reduce_add_sync(SPH_FULL_MASK, lane < warp ? f : 0u);
+        r += __reduce_add_sync(SPH_FULL_MASK, f);
+        if (!mine) continue;
+#pragma unroll 1
+        for (unsigned j = 0; j < SPH_CROWD_ITEMS; ++j) {
+            const bool in = hit >> j & 1u;
+            const unsigned here = __ballot_sync(SPH_FULL_MASK, in);
+            const unsigned k = to + __popc(here & ((1u << lane) - 1u));
+            to += __popc(here);
+            // (past the cell's end only with inconsistent host-written tables)
+            if (in && k - off < cnt) {
+                S.cellparticles[k] = i + 32u * j;
+                if (GATHER) gather_one(S, k, i + 32u * j, cell, with_vel, 0, with_solid);
+            }
+        }
+    }
+}
+
 // Canonical order inside each cell: ascending particle index.  One thread
 // per entry of the unsorted list: its particle's place in the cell is the
-// number of the cell's particles with a smaller index.  (In a cell of m
-// particles that takes m^2 comparisons; the pair passes test each of them
-// against all others at many times that cost.)  GATHER: a substep, where
-// nothing changes between the order and the pair passes; the particle's
-// sorted copies are written here too.  Bound: latency of the chain entry ->
-// table -> the cell's entries and fields -> stores.  With the scatter 47 ->
-// 33 us at 1M particles, against an order, a sort of crowded cells and a
-// gather in launches of their own (four launches; a 1,000-particle substep
-// 59 -> 55 us).
+// number of the cell's particles with a smaller index.  A crowded cell is
+// ordered by the block that holds its first entry (a pile of 500,000 of 1M
+// particles 40.5 -> 0.94 ms, of 10,000 of 100,000 300 -> 92 us, and 91 -> 92
+// us without a pile, against comparisons in every cell).  GATHER: a substep,
+// where nothing changes between the order and the pair passes; the
+// particle's sorted copies are written here too, and a crowded cell is
+// compared like any other: the pair passes test each of its particles
+// against all others at ten times that cost (20,000 of 1M particles 0.6 of
+// 8.4 ms), and the walk's registers cost every 1M-particle substep 7 us.  Bound: latency of the chain entry -> table ->
+// the cell's entries and fields -> stores.  With the scatter 47 -> 33 us at
+// 1M particles, against an order, a sort of crowded cells and a gather in
+// launches of their own (four launches; a 1,000-particle substep 59 -> 55
+// us).
+#define SPH_CROWDED_STARTS 4  // cells above 256 that can start in 1,024 entries
 template <bool GATHER>
 __global__ void k_rank_cells(const SceneDesc *__restrict__ scenes, BlockMap map, int with_vel, int with_solid) {
+    __shared__ unsigned starts[1 + SPH_CROWDED_STARTS];
     SPH_FOR_WORK(map)
-    if (item < active_count(S)) {
+    const unsigned n = active_count(S);
+    unsigned crowded = 0xffffffffu;  // the crowded cell that starts at this entry
+    if (item < n) {
         const unsigned x = S.unsorted[item], cell = S.unsorted[S.pnum + item];
         // inconsistent tables come only from host-written garbage: skip
         if (x < S.pnum && cell < S.num_cells) {
             const unsigned off = S.celloffset[cell], cnt = S.gridcount[cell];
             if (off <= item && item - off < cnt && cnt <= S.pnum - off) {
-                const unsigned *U = S.unsorted + off;
-                unsigned r = off;
+                if (!GATHER && crowded_cell(cnt, n)) {
+                    if (item == off) crowded = cell;
+                } else {
+                    const unsigned *U = S.unsorted + off;
+                    unsigned r = off;
 #pragma unroll 4
-                for (unsigned a = 0; a < cnt; ++a) r += U[a] < x;
-                S.cellparticles[r] = x;
-                if (GATHER) gather_one(S, r, x, cell, with_vel, 0, with_solid);
+                    for (unsigned a = 0; a < cnt; ++a) r += U[a] < x;
+                    S.cellparticles[r] = x;
+                    if (GATHER) gather_one(S, r, x, cell, with_vel, 0, with_solid);
+                }
             }
         }
+    }
+    if (!GATHER && __syncthreads_or(crowded != 0xffffffffu)) {
+        if (threadIdx.x == 0) starts[0] = 0u;
+        __syncthreads();
+        if (crowded != 0xffffffffu) {
+            const unsigned q = atomicAdd(starts, 1u);
+            if (q < SPH_CROWDED_STARTS) starts[1 + q] = crowded;
+        }
+        __syncthreads();
+        const unsigned num = min(starts[0], (unsigned)SPH_CROWDED_STARTS);
+        for (unsigned q = 0; q < num; ++q) order_crowded_cell<false>(S, starts[1 + q], n, 0, 0);
+        __syncthreads();  // the next entry clears them
     }
     SPH_END_WORK
 }
@@ -374,6 +447,13 @@ __global__ void k_gather(const SceneDesc *__restrict__ scenes, BlockMap map, int
 #define SPH_SMALL_ITEMS 4
 #define SPH_SMALL_PARTICLES (SPH_SMALL_BLOCKS * SPH_SMALL_THREADS * SPH_SMALL_ITEMS)
 #define SPH_SMALL_CELLS 65536
+// Crowded cells here, where a walk takes 6.5 us at most, a thread's
+// comparisons run for up to four particles one after another (17 ns a step),
+// and the cluster's blocks share the cells: 4,096 of 16,384 particles in one
+// cell 300 -> 27 us, all of them 1,133 -> 31 us, 20.0 -> 21.1 us without a
+// pile.
+__device__ __forceinline__ bool crowded_small(unsigned m, unsigned n) { return m > 256u + n / 256u; }
+#define SPH_SMALL_CROWDED (SPH_SMALL_PARTICLES / 257)
 
 template <bool GATHER>
 __global__ void __launch_bounds__(SPH_SMALL_THREADS) k_grid_small(const SceneDesc *__restrict__ scenes, int with_vel,
@@ -382,6 +462,8 @@ __global__ void __launch_bounds__(SPH_SMALL_THREADS) k_grid_small(const SceneDes
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
     __shared__ unsigned totals[SPH_SMALL_BLOCKS];
+    // crowded cells: their number and themselves, in block 0
+    __shared__ unsigned crowded[1 + SPH_SMALL_CROWDED];
     const SceneDesc &S = scenes[0];
     if (scene_idle(S)) return;
     constexpr unsigned threads = SPH_SMALL_BLOCKS * SPH_SMALL_THREADS;
@@ -389,6 +471,8 @@ __global__ void __launch_bounds__(SPH_SMALL_THREADS) k_grid_small(const SceneDes
     const unsigned n = active_count(S), cells = S.num_cells;
     for (unsigned c = me; c < cells; c += threads) S.gridcount[c] = 0u;
     if (me == 0 && S.solid_list) S.solid_list[0] = 0u;
+    if (threadIdx.x == 0) crowded[0] = 0u;
+    unsigned *const all_crowded = cluster.map_shared_rank(crowded, 0);
     unsigned cell[SPH_SMALL_ITEMS], slot[SPH_SMALL_ITEMS];
 #pragma unroll
     for (int j = 0; j < SPH_SMALL_ITEMS; ++j) {
@@ -411,7 +495,14 @@ __global__ void __launch_bounds__(SPH_SMALL_THREADS) k_grid_small(const SceneDes
     const unsigned end = min(cells, (rank + 1) * share);
     const unsigned c0 = min(end, rank * share + threadIdx.x * run), c1 = min(end, c0 + run);
     unsigned sum = 0, total;
-    for (unsigned c = c0; c < c1; ++c) sum += S.gridcount[c];
+    for (unsigned c = c0; c < c1; ++c) {
+        const unsigned m = S.gridcount[c];
+        sum += m;
+        if (crowded_small(m, n)) {
+            const unsigned q = atomicAdd(all_crowded, 1u);
+            if (q < SPH_SMALL_CROWDED) all_crowded[1 + q] = c;
+        }
+    }
     unsigned off = block_exclusive_scan(sum, &total);
     if (threadIdx.x < SPH_SMALL_BLOCKS) cluster.map_shared_rank(totals, threadIdx.x)[rank] = total;
     cluster.sync();  // every block's total is in every block
@@ -428,19 +519,28 @@ __global__ void __launch_bounds__(SPH_SMALL_THREADS) k_grid_small(const SceneDes
 #pragma unroll
     for (int j = 0; j < SPH_SMALL_ITEMS; ++j)
         if (me + j * threads < n) S.unsorted[first[j] + slot[j]] = me + j * threads;
+    // the list's end before the last barrier: block 0 may end after it
+    const unsigned num_crowded = min(all_crowded[0], (unsigned)SPH_SMALL_CROWDED);
+    if (rank && threadIdx.x < num_crowded) crowded[1 + threadIdx.x] = all_crowded[1 + threadIdx.x];
     cluster.sync();  // the cells' lists are complete
 #pragma unroll 1
     for (int j = 0; j < SPH_SMALL_ITEMS; ++j) {
         const unsigned i = me + j * threads;
         if (i >= n) break;
         const unsigned cnt = S.gridcount[cell[0]];
-        const unsigned *U = S.unsorted + first[0];
-        unsigned k = first[0];
+        if (!crowded_small(cnt, n)) {
+            const unsigned *U = S.unsorted + first[0];
+            unsigned k = first[0];
 #pragma unroll 4
-        for (unsigned a = 0; a < cnt; ++a) k += U[a] < i;
-        S.cellparticles[k] = i;
-        if (GATHER) gather_one(S, k, i, cell[0], with_vel, 0, with_solid);
+            for (unsigned a = 0; a < cnt; ++a) k += U[a] < i;
+            S.cellparticles[k] = i;
+            if (GATHER) gather_one(S, k, i, cell[0], with_vel, 0, with_solid);
+        }
 #pragma unroll
         for (int q = 0; q + 1 < SPH_SMALL_ITEMS; ++q) cell[q] = cell[q + 1], first[q] = first[q + 1];
     }
+    // (the loop of a thread ends with its particles: together again)
+    __syncthreads();
+    for (unsigned q = rank; q < num_crowded; q += SPH_SMALL_BLOCKS)
+        order_crowded_cell<GATHER>(S, crowded[1 + q], n, with_vel, with_solid);
 }
