@@ -38,9 +38,14 @@
 //     order with the exact arithmetic of a direct walk: each adds its
 //     density term, and the few that are not within h lose their bit.
 // Values, order and arithmetic of the sums are those of a direct walk,
-// which a row takes whose range does not lie in the staged one (a plane's
-// ranges wider than the buffer, inconsistent host-written tables), or whose
-// particle lies within h of a symmetry plane.
+// which a row takes whose range does not lie in the staged one (inconsistent
+// host-written tables), or whose particle lies within h of a symmetry plane.
+// A plane whose ranges are wider than the buffer is staged row by row, and a
+// row that is wider in pieces, whose candidates are tested as they come.
+// Against a direct walk of every row of such a plane (a few blocks, which
+// end last): 27 particles a cell, 8,000 particles 50 -> 24 us and 97,336
+// 117 -> 64 us, 216 a cell 281 -> 76 and 1,001 -> 457 us, 10,000 of 100,000
+// particles in one cell 1,437 -> 389 us.
 // The sum is blocked: each stencil row's terms are added in candidate
 // order, and the nine row sums with Kahan compensation (one compensated
 // add per row instead of per neighbour).
@@ -50,8 +55,8 @@
 // candidates lie within h (kernels_common.cuh, candidate masks).  The stores
 // of one row are one coalesced store per warp.  num_neighbours is the number
 // of set bits, less the few candidates at exactly h.
-// A plane's buffer of 896 candidates holds its ranges: about 440 for 128
-// particles in a lattice of 8 per cell, 820 for 256.
+// A plane's buffer of 896 candidates holds the ranges of 128 particles:
+// about 440 in a lattice of 8 per cell, 600 in one of 27.
 //
 // SPLIT (small launches): a block is three warps over the same 32 particles,
 // one per z plane, each with a buffer of its own; the nine row sums meet in
@@ -117,7 +122,7 @@ __device__ __forceinline__ void density_block(const SceneDesc &S, unsigned n, un
             e = min(S.celloffset[x1] + S.gridcount[x1], pnum);
         }
         const unsigned a = b & ~3u;
-        stage.range[r] = make_uint2(a, b < e ? (min(e - a, STAGE) + 3u) & ~3u : 0u);
+        stage.range[r] = make_uint2(a, b < e ? (e - a + 3u) & ~3u : 0u);
     }
     const float3 ipos = active ? xyz(spos[k]) : make_float3(0.f, 0.f, 0.f);
     const NegPoint nip = neg_point(ipos);
@@ -141,8 +146,15 @@ __device__ __forceinline__ void density_block(const SceneDesc &S, unsigned n, un
         for (int dy = 0; dy < 3; ++dy) {
             const uint2 g = stage.range[3 * dz + dy];
             ua[dy] = g.x;
-            at[dy + 1] = at[dy] + g.y;
+            at[dy + 1] = at[dy] + min(g.y, STAGE + 4u);  // (no sum overflows)
         }
+    };
+    auto stage_one = [&](float *to, unsigned kk) {
+        // up to three past the range: any value (capacity bounds it)
+        const float *p = reinterpret_cast<const float *>(spos + min(kk, pnum - 1u));
+        copy_word_async(to, p);
+        copy_word_async(to + STAGE, p + 1);
+        copy_word_async(to + 2 * STAGE, p + 2);
     };
     auto stage_plane = [&](int dz) {
         unsigned at[4], ua[3];
@@ -150,14 +162,84 @@ __device__ __forceinline__ void density_block(const SceneDesc &S, unsigned n, un
         if (at[3] > STAGE) return;
         float *to = stage.xyz[SPLIT ? dz : dz & 1];
 #pragma unroll 1
-        for (unsigned t = threadIdx.x; t < at[3]; t += blockDim.x) {
-            const unsigned row0 = t < at[1] ? ua[0] : t < at[2] ? ua[1] - at[1] : ua[2] - at[2];
-            // up to three past the range: any value (capacity bounds it)
-            const float *p = reinterpret_cast<const float *>(spos + min(row0 + t, pnum - 1u));
-            copy_word_async(to + t, p);
-            copy_word_async(to + STAGE + t, p + 1);
-            copy_word_async(to + 2 * STAGE + t, p + 2);
+        for (unsigned t = threadIdx.x; t < at[3]; t += blockDim.x)
+            stage_one(to + t, t + (t < at[1] ? ua[0] : t < at[2] ? ua[1] - at[1] : ua[2] - at[2]));
+    };
+    // the threads that share a buffer together: a split launch's warps have
+    // one each, and may differ in whether their planes fit
+    auto sync = [] {
+        if (SPLIT) __syncwarp();
+        else __syncthreads();
+    };
+    auto stage_row = [&](float *to, unsigned from, unsigned num) {
+        sync();  // what the buffer held is done with
+#pragma unroll 1
+        for (unsigned t = threadIdx.x; t < num; t += blockDim.x) stage_one(to + t, from + t);
+        copies_wait();
+        sync();
+    };
+    // every candidate of [from, from + len) from the copies
+    auto direct = [&](unsigned from, unsigned len, unsigned &lo, unsigned &hi, float &rowsum) {
+#pragma unroll 1
+        for (unsigned t = 0; t < len; ++t) {
+            const float4 j4 = spos[from + t];
+            const float r2 = dist2(j4, nip);
+            if (r2 <= B.le) {
+                const float d = fmaxf(h2 - r2, 0.f);
+                rowsum = __fadd_rn(rowsum, d * d * d);
+                count += r2 <= B.lt;
+                if (MASK && t < 32u) lo |= 0x80000000u >> t;
+                if (MASK && t >= 32u && t < 64u) hi |= 0x80000000u >> (t - 32u);
+            }
+            if (PLANES && P.imask) {
+                const float3 jpos = xyz(j4);
+                const unsigned jm = plane_jmask(P, jpos, h);
+                // subsets of jm in increasing order: the reference's
+                // plane_bits order restricted to the subsets it keeps
+                for (unsigned sb = (0u - jm) & jm; sb; sb = (sb - jm) & jm) {
+                    float3 ref = jpos;
+                    for (unsigned s2 = 0; s2 < P.count; ++s2)
+                        if (sb & (1u << s2)) ref = reflect3(ref, P.p[s2], P.n[s2]);
+                    const float m2 = norm2(sub3(ref, ipos));
+                    if (m2 <= B.lt) {
+                        const float d = fmaxf(h2 - m2, 0.f);
+                        rowsum = __fadd_rn(rowsum, d * d * d);
+                        ++count;
+                    }
+                }
+            }
         }
+    };
+    // a row whose range is wider than the buffer, in pieces, every candidate
+    // as it comes: without a branch, since a term beyond h is zero
+    auto wide_row = [&](int r, unsigned b, unsigned e, float *buf, unsigned &lo, unsigned &hi, float &rowsum) {
+        const uint2 g = stage.range[r];
+        const bool staged = b - g.x < g.y && e - g.x <= g.y && !(PLANES && P.imask);
+#pragma unroll 1
+        for (unsigned p = g.x; p - g.x < g.y; p += STAGE) {
+            stage_row(buf, p, min(g.x + g.y - p, STAGE));
+            const unsigned le = staged ? max(p, min(e, p + STAGE)) : p, lb = min(le, max(b, p));
+            auto visit = [&](unsigned t) {
+                const float r2 = dist2(make_float4(buf[t], buf[STAGE + t], buf[2 * STAGE + t], 0.f), nip);
+                const float d = fmaxf(h2 - r2, 0.f);
+                rowsum = __fadd_rn(rowsum, d * d * d);
+                count += r2 <= B.lt;
+                return r2 <= B.le;
+            };
+            // (a row longer than 64, which the later passes scan, has no bits
+            // past 64)
+            const unsigned lm = MASK ? min(le, max(lb, b + 64u)) : lb;
+#pragma unroll 1
+            for (unsigned kk = lb; kk < lm; ++kk) {
+                const unsigned at = kk - b;
+                if (!visit(kk - p)) continue;
+                if (at < 32u) lo |= 0x80000000u >> at;
+                else hi |= 0x80000000u >> (at - 32u);
+            }
+#pragma unroll 4
+            for (unsigned t = lm - p; t < le - p; ++t) visit(t);
+        }
+        if (!staged) direct(b, e - b, lo, hi, rowsum);
     };
     // the exact walk over the staged candidates of a chunk's bits (candidate
     // src + t at bit 31 - t), in order; returns the bits that are within h
@@ -195,7 +277,7 @@ __device__ __forceinline__ void density_block(const SceneDesc &S, unsigned n, un
         }
         plane_at(dz, at, ua);
         const bool fits = at[3] <= STAGE;
-        const float *buf = stage.xyz[SPLIT ? dz : dz & 1];
+        float *buf = stage.xyz[SPLIT ? dz : dz & 1];
         copies_wait();
         __syncthreads();  // this plane is staged, and the other buffer is free
         if (dz + 1 < dz1) stage_plane(dz + 1);
@@ -208,13 +290,21 @@ __device__ __forceinline__ void density_block(const SceneDesc &S, unsigned n, un
             // the row's density terms in candidate order; the row sums are
             // added with Kahan compensation (blocked summation)
             float rowsum = 0.f;
+            const unsigned range = at[1] - at[0];
+            if (!fits) {
+                // a plane that does not fit is staged row by row
+                if (range > STAGE) wide_row(3 * dz + dy, b[0], e[0], buf, lo, hi, rowsum);
+                else stage_row(buf, ua[0], range);
+            }
             // (an empty row takes the direct walk, of no candidate)
-            if (fits && b[0] - ua[0] < at[1] - at[0] && e[0] - ua[0] <= at[1] - at[0] && !(PLANES && P.imask)) {
+            if (range > STAGE) {
+                // done
+            } else if (b[0] - ua[0] < range && e[0] - ua[0] <= range && !(PLANES && P.imask)) {
                 // chunks of 32 candidates, from the row's start rounded down
                 // to a multiple of four: candidate c0 + t of the rounded row
                 // is bit 31 - t, and the first `o` belong to the cells before
                 const unsigned o = b[0] & 3u, tot = len ? o + len : 0u;
-                const float *src = buf + at[0] + (b[0] - o - ua[0]);
+                const float *src = buf + (fits ? at[0] : 0u) + (b[0] - o - ua[0]);
                 if (tot) {
                     unsigned m = near_bits<STAGE>(src, min((tot + 3u) >> 2, 8u), nx, ny, nz, nb) & (0xffffffffu >> o);
                     if (tot < 32u) m &= ~(0xffffffffu >> tot);
@@ -236,38 +326,7 @@ __device__ __forceinline__ void density_block(const SceneDesc &S, unsigned n, un
                     }
                 }
             } else {
-                // bits of `lo` for candidates [0, 32), of `hi` for [32, 64);
-                // a row longer than 64 (the later passes scan it) records
-                // none past 64
-#pragma unroll 1
-                for (unsigned t = 0; t < len; ++t) {
-                    const float4 j4 = spos[b[0] + t];
-                    const float r2 = dist2(j4, nip);
-                    if (r2 <= B.le) {
-                        const float d = fmaxf(h2 - r2, 0.f);
-                        rowsum = __fadd_rn(rowsum, d * d * d);
-                        count += r2 <= B.lt;
-                        if (MASK && t < 32u) lo |= 0x80000000u >> t;
-                        if (MASK && t >= 32u && t < 64u) hi |= 0x80000000u >> (t - 32u);
-                    }
-                    if (PLANES && P.imask) {
-                        const float3 jpos = xyz(j4);
-                        const unsigned jm = plane_jmask(P, jpos, h);
-                        // subsets of jm in increasing order: the reference's
-                        // plane_bits order restricted to the subsets it keeps
-                        for (unsigned sb = (0u - jm) & jm; sb; sb = (sb - jm) & jm) {
-                            float3 ref = jpos;
-                            for (unsigned s2 = 0; s2 < P.count; ++s2)
-                                if (sb & (1u << s2)) ref = reflect3(ref, P.p[s2], P.n[s2]);
-                            const float m2 = norm2(sub3(ref, ipos));
-                            if (m2 <= B.lt) {
-                                const float d = fmaxf(h2 - m2, 0.f);
-                                rowsum = __fadd_rn(rowsum, d * d * d);
-                                ++count;
-                            }
-                        }
-                    }
-                }
+                direct(b[0], len, lo, hi, rowsum);
             }
             if (SPLIT) stage.rows[3 * dz + dy][threadIdx.x] = rowsum;
             else rho.add(rowsum);

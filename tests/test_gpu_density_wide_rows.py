@@ -1,0 +1,99 @@
+"""GPU: the density pass where a z plane's rows do not fit its staging buffer
+together (more than 8 particles a cell), and where a row does not either
+(piles): staged row by row and in pieces, against the oracle and in both
+forms of the pass; and what it takes."""
+import ctypes
+
+import numpy as np
+import pytest
+
+from helpers import max_rel, oracle_of
+from sph import bindings as bnd
+from sph import scenes
+
+pytestmark = pytest.mark.gpu
+
+
+def cloud(parts, seed):
+    """Particles of `parts`: (number, cell corner, cells wide) each."""
+    rng = np.random.default_rng(seed)
+    pos = np.concatenate([(np.array(c) + w * rng.random((m, 3))) * 0.02 for m, c, w in parts])
+    n = pos.shape[0]
+    pos = pos[rng.permutation(n)]
+    sc = scenes.wcsph_block(2, 2, 2, box=(0.0, 0.4), pnum=n + 5, dt=1e-9, stiffness=1e-3)
+    sc.init = {"position": pos.astype(np.float32), "n": n}
+    return sc
+
+
+# split blocks hold 256 candidates, whole ones 896: planes of rows of about
+# 110 and 330, rows of 350 to 2,700, and piles beside a thin cloud, whose
+# particles' short rows lie in a wide range with theirs (at both ends of it)
+CLOUDS = {"27 a cell": [(2300, (4, 4, 4), (5, 4, 4))], "110 a cell": [(4500, (4, 4, 4), (4, 3, 3))],
+          "300 a cell": [(2600, (4, 4, 4), (3, 3, 1))],
+          "900 a cell": [(2700, (4, 4, 4), (3, 1, 1)), (40, (4, 5, 4), (3, 1, 1))],
+          "pile": [(1500, (8, 8, 8), (1, 1, 1)), (900, (5, 5, 5), (7, 7, 7))],
+          "two piles": [(257, (8, 8, 8), (1, 1, 1)), (1100, (11, 8, 8), (1, 1, 1)), (400, (7, 7, 7), (6, 3, 3))]}
+
+
+@pytest.mark.parametrize("name", sorted(CLOUDS))
+def test_wide_rows_match_oracle(name):
+    from sph.batch import Batch
+    for seed in range(3):
+        sc = cloud(CLOUDS[name], seed)
+        n = sc.init["position"].shape[0]
+        ps = sc.system()
+        o = oracle_of(ps)
+        for call in ("compute_particle_bins", "compute_density"):
+            o.call(call)
+        ps.compute_particle_bins()
+        ps.call_for_all_particles("compute_density")
+        ps.sync_device_to_host()
+        count, dens = (np.array(a[:n]) for a in ps.get_fields("num_neighbours", "density"))
+        assert np.array_equal(count, o.a["num_neighbours"][:n])
+        assert max_rel(dens, o.a["density"][:n]) <= 1e-5  # the other density tests' bound
+        # the fused pass, whose masks the forces walk, split (alone) and
+        # whole (in a batch past the line)
+        ps.update_fused(1)
+        ps.sync_device_to_host()
+        b = Batch()
+        sid = b.add(sc)
+        b.add(scenes.wcsph_block(36, 36, 36, jitter=1e-4, seed=2))
+        b.step(1)
+        whole = b.read(sid)
+        b.close()
+        fused = {f: np.array(ps.get_fields(f)[0][:n]) for f in ("num_neighbours", "density", "force")}
+        assert np.array_equal(fused["num_neighbours"], count) and np.array_equal(fused["density"], dens)
+        for f in fused:
+            assert np.array_equal(whole[f][:n], fused[f]), f
+        # the forces of a named scan of the same state
+        ps2 = sc.system()
+        ps2.compute_particle_bins()
+        ps2.call_for_all_particles("compute_density")
+        ps2.sync_device_to_host()  # a call between: the next one scans
+        ps2.call_for_all_particles("compute_forces_fluids")
+        ps2.sync_device_to_host()
+        assert np.array_equal(ps2.get_fields("force")[0][:n], fused["force"])
+        ps.close()
+        ps2.close()
+
+
+def density_us(side, spacings):
+    sc = scenes.wcsph_block(side, side, side, spacing=0.01, h=0.01 * spacings, box=(0.0, 0.02 * side + 0.08),
+                            jitter=1e-4, dt=1e-6)
+    ps = sc.system()
+    ps.update_fused(1)
+    best = 1e9
+    for _ in range(5):
+        ms, names = (ctypes.c_float * 24)(), (ctypes.c_char_p * 24)()
+        k = bnd.sph_profile_substep(ps.psdata_opencl, 10, ms, names, 24)
+        best = min(best, {names[i]: ms[i] for i in range(k)}[b"density"])
+    ps.close()
+    return best * 1e3
+
+
+@pytest.mark.parametrize("side", [20, 46])  # split over three warps; whole
+def test_time_grows_no_faster_than_the_candidates(side):
+    """27 particles a cell have 27/8 of the candidates of 8; the blocks whose
+    plane did not fit walked directly and took it to 4.2 and 4.7 times."""
+    two, three = density_us(side, 2), density_us(side, 3)
+    assert three <= 27.0 / 8.0 * two, (two, three)
