@@ -553,25 +553,31 @@ __device__ __forceinline__ void walk_pair(const FluidI &I, bool solid_i, float4 
     fluid_pair_p<true>(I, I.pi, xyz(p), xyz(v), p.w, v.w, f);
 }
 
-// The stencil scan: every candidate of the 27 cells, in the reference's
-// order.
-template <bool MIXED>
-__device__ __forceinline__ void fluid_scan(const SceneDesc &S, unsigned cell, const FluidI &I, BlockSum3 &f,
-                                           bool solid_i) {
+// The stencil scan: every candidate of the rows [r0, r1), in the reference's
+// order; row_end(r) closes each.
+template <bool MIXED, class RowEnd>
+__device__ __forceinline__ void fluid_scan(const SceneDesc &S, const StencilRows &rows, int r0, int r1, const FluidI &I,
+                                           BlockSum3 &f, bool solid_i, RowEnd &&row_end) {
     const float4 *spos = S.spos;
     const float4 *svel = S.svel;
     const float *sdens = S.sdens;
-    for_each_neighbour(S, cell, [&](unsigned kk) {
-        const bool solid_j = MIXED && S.phase[min(S.cellparticles[kk], S.pnum - 1)] != 0u;
-        if (solid_i && solid_j) return;
-        const float rho = sdens[kk];
-        float pi = I.pi, pj = fluid_pressure(rho, I.rho0, I.stiff);
-        if (MIXED && (solid_i || solid_j)) {
-            pi = fmaxf(pi, 0.f);
-            pj = fmaxf(pj, 0.f);
+#pragma unroll 1
+    for (int r = r0; r < r1; ++r) {
+        unsigned b, e;
+        rows.row(S, r, &b, &e);
+        for (unsigned kk = b; kk < e; ++kk) {
+            const bool solid_j = MIXED && S.phase[min(S.cellparticles[kk], S.pnum - 1)] != 0u;
+            if (solid_i && solid_j) continue;
+            const float rho = sdens[kk];
+            float pi = I.pi, pj = fluid_pressure(rho, I.rho0, I.stiff);
+            if (MIXED && (solid_i || solid_j)) {
+                pi = fmaxf(pi, 0.f);
+                pj = fmaxf(pj, 0.f);
+            }
+            fluid_pair_p(I, pi, xyz(spos[kk]), xyz(svel[kk]), pj, rcp_approx(rho), f);
         }
-        fluid_pair_p(I, pi, xyz(spos[kk]), xyz(svel[kk]), pj, rcp_approx(rho), f);
-    }, [&] { f.end_row(); });
+        row_end(r);
+    }
 }
 
 template <bool MIXED>
@@ -585,7 +591,7 @@ __global__ void k_forces_fluids(const SceneDesc *__restrict__ scenes, BlockMap m
         const FluidI I = fluid_i(S, xyz(S.spos[k]), xyz(S.svel[k]), S.sdens[k]);
         const bool solid_i = mixed_solid<MIXED>(S, i);
         BlockSum3 f;
-        fluid_scan<MIXED>(S, S.srow[k].x, I, f, solid_i);
+        fluid_scan<MIXED>(S, StencilRows(S, S.srow[k]), 0, 9, I, f, solid_i, [&](int) { f.end_row(); });
         fluid_finish(S, i, I, f, fuse_step, mixed_extra<MIXED>(S, i, solid_i));
     }
     SPH_END_WORK
@@ -595,7 +601,8 @@ __global__ void k_forces_fluids(const SceneDesc *__restrict__ scenes, BlockMap m
 // recorded, row by row and two neighbours at a time, reading each
 // neighbour's position with its pressure in w and its velocity with its
 // reciprocal density in w (two float4 loads).  Lanes whose masks overflowed
-// scan the stencil.
+// scan the stencil (SPLIT: each warp its plane's rows; 8,000 particles of 27
+// a cell 162 -> 67 us, against all nine by one of the three).
 // Bound: latency of the gathers (issue slots 64% used; 2 neighbours in
 // flight a thread, 32 warps an SM).  Masks whose first candidate is the top
 // bit (one leading-zero count finds the next), no count of neighbours here
@@ -627,8 +634,17 @@ __global__ void __maxnreg__(SPLIT ? 72 : 64)
         const StencilRows rows(S, S.srow[kc]);
         const bool solid_i = mixed_solid<MIXED>(S, i);
         BlockSum3 f;
-        const bool scan = S.ncand[kc] == SPH_NCAND_SCAN;
-        if (!scan && active) {
+        auto end_row = [&](int r) {
+            if (SPLIT) {
+                rows_sum[r][0][threadIdx.x] = f.rxy.x;
+                rows_sum[r][1][threadIdx.x] = f.rxy.y;
+                rows_sum[r][2][threadIdx.x] = f.rz;
+                f = BlockSum3();
+            } else {
+                f.end_row();
+            }
+        };
+        if (active && S.ncand[kc] != SPH_NCAND_SCAN) {
             const float4 *spos = S.spos;
             const float4 *svel = S.svel;
             // two neighbours per iteration: both loads are in flight
@@ -670,27 +686,18 @@ __global__ void __maxnreg__(SPLIT ? 72 : 64)
                         }
                     }
                 }
-                if (SPLIT) {
-                    rows_sum[r][0][threadIdx.x] = f.rxy.x;
-                    rows_sum[r][1][threadIdx.x] = f.rxy.y;
-                    rows_sum[r][2][threadIdx.x] = f.rz;
-                    f = BlockSum3();
-                } else {
-                    f.end_row();
-                }
+                end_row(r);
             }
-        } else if (active && r0 == 0) {
-            fluid_scan<MIXED>(S, rows.cell, I, f, solid_i);
+        } else if (active) {
+            fluid_scan<MIXED>(S, rows, r0, r1, I, f, solid_i, end_row);
         }
         if (SPLIT) {
             __syncthreads();
             if (r0 || !active) continue;
-            if (!scan) {
 #pragma unroll
-                for (int r = 0; r < 9; ++r)
-                    f.total.add(make_float3(rows_sum[r][0][threadIdx.x], rows_sum[r][1][threadIdx.x],
-                                            rows_sum[r][2][threadIdx.x]));
-            }
+            for (int r = 0; r < 9; ++r)
+                f.total.add(make_float3(rows_sum[r][0][threadIdx.x], rows_sum[r][1][threadIdx.x],
+                                        rows_sum[r][2][threadIdx.x]));
         }
         fluid_finish(S, i, I, f, fuse_step, mixed_extra<MIXED>(S, i, solid_i));
     }
