@@ -373,7 +373,8 @@ size_t sph_batch_bytes(sph_batch *batch);
 unsigned int sph_batch_size(sph_batch *batch);
 /* Launch shape: threads per block for particle/cell kernels (32..1024) and
  * for pair kernels (32..512), multiples of 32, and the persistent-grid cap
- * (0: one block per work item). */
+ * (0: one block per work item).  Pair kernels that stage rows or sums in
+ * shared memory keep the block their buffers are sized for. */
 int sph_batch_tune(sph_batch *batch, unsigned int block, unsigned int pair_block, unsigned int grid_cap);
 unsigned int sph_batch_kernel_count(sph_batch *batch);
 void *sph_batch_stream(sph_batch *batch);

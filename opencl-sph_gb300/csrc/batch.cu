@@ -65,7 +65,7 @@ struct sph_batch {
     GroupLaunch group[3];    // by SphMaterial
     cudaGraphExec_t graph = nullptr;
     unsigned graph_kernels = 0;
-    unsigned block = 256, pair_block = 128, grid_cap = 0;
+    unsigned block = 256, pair_block = SPH_STAGED_BLOCK, grid_cap = 0;
     size_t bytes = 0;
     CopySeg *copy_segs = nullptr;  // device table of sph_batch_read_field_many
     unsigned copy_cap = 0;
@@ -135,6 +135,7 @@ bool solid_setup(sph_batch *b, BatchScene *sc) {
     size_t o_d = t.add(&sc->desc, sizeof(SceneDesc));
     size_t o_p = t.add(m.particles.data(), m.particles.size() * sizeof(BlockWork));
     size_t o_pp = t.add(m.pair_particles.data(), m.pair_particles.size() * sizeof(BlockWork));
+    size_t o_st = t.add(m.staged.data(), m.staged.size() * sizeof(BlockWork));
     size_t o_c = t.add(m.cells.data(), m.cells.size() * sizeof(BlockWork));
     size_t o_s = t.add(m.scan.data(), m.scan.size() * sizeof(BlockWork));
     char *d = nullptr;
@@ -146,6 +147,7 @@ bool solid_setup(sph_batch *b, BatchScene *sc) {
     L.num_scenes = 1;
     L.particles = map_at(d, o_p, m.particles);
     L.pair_particles = map_at(d, o_pp, m.pair_particles);
+    L.staged = m.staged.empty() ? L.pair_particles : map_at(d, o_st, m.staged);
     L.cells = map_at(d, o_c, m.cells);
     L.scan = map_at(d, o_s, m.scan);
     L.block = b->block;
@@ -193,6 +195,7 @@ bool rebuild(sph_batch *b) {
     size_t o_d = t.add(descs.data(), descs.size() * sizeof(SceneDesc));
     size_t o_p = t.add(all.particles.data(), all.particles.size() * sizeof(BlockWork));
     size_t o_pp = t.add(all.pair_particles.data(), all.pair_particles.size() * sizeof(BlockWork));
+    size_t o_st = t.add(all.staged.data(), all.staged.size() * sizeof(BlockWork));
     size_t o_c = t.add(all.cells.data(), all.cells.size() * sizeof(BlockWork));
     size_t o_s = t.add(all.scan.data(), all.scan.size() * sizeof(BlockWork));
     std::vector<RigidWork> rigid;
@@ -200,10 +203,11 @@ bool rebuild(sph_batch *b) {
         for (unsigned body : b->slots[ids[k]]->rigid)
             if (rigid.size() < SPH_MAX_RIGID_WORK) rigid.push_back(RigidWork{k, body});
     size_t o_rw = t.add(rigid.data(), rigid.size() * sizeof(RigidWork));
-    size_t o_gp[3], o_gpp[3];
+    size_t o_gp[3], o_gpp[3], o_gst[3];
     for (int m = 0; m < 3; ++m) {
         o_gp[m] = t.add(g[m].particles.data(), g[m].particles.size() * sizeof(BlockWork));
         o_gpp[m] = t.add(g[m].pair_particles.data(), g[m].pair_particles.size() * sizeof(BlockWork));
+        o_gst[m] = t.add(g[m].staged.data(), g[m].staged.size() * sizeof(BlockWork));
     }
     if (!balloc(b, (void **)&b->tables, t.host.size(), b->stream, "batch tables")) return false;
     b->table_bytes = t.host.size();
@@ -218,6 +222,7 @@ bool rebuild(sph_batch *b) {
     A.num_scenes = (unsigned)descs.size();
     A.particles = map_at(d, o_p, all.particles);
     A.pair_particles = map_at(d, o_pp, all.pair_particles);
+    A.staged = all.staged.empty() ? A.pair_particles : map_at(d, o_st, all.staged);
     A.cells = map_at(d, o_c, all.cells);
     A.scan = map_at(d, o_s, all.scan);
     A.block = b->block;
@@ -242,6 +247,7 @@ bool rebuild(sph_batch *b) {
         G.L = A;
         G.L.particles = map_at(d, o_gp[m], g[m].particles);
         G.L.pair_particles = map_at(d, o_gpp[m], g[m].pair_particles);
+        G.L.staged = g[m].staged.empty() ? G.L.pair_particles : map_at(d, o_gst[m], g[m].staged);
         G.L.stream = streams[m];
         G.L.carveout = branches > 1 ? 44 : 0;
     }

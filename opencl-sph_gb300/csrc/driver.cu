@@ -238,7 +238,7 @@ Store *create_store(psdata *data, const char *file_list, std::string *err) {
     s->material = sph_material_of(programs);
     s->blob_size = psdata_data_size(*data);
 
-    const unsigned block = 256, pair_block = 128;
+    const unsigned block = 256, pair_block = SPH_STAGED_BLOCK;
     std::vector<SceneDesc> descs(1, probe);
     HostMaps maps;
     sph_build_maps(descs, {0u}, block, pair_block, &maps);
@@ -295,6 +295,7 @@ Store *create_store(psdata *data, const char *file_list, std::string *err) {
     L.num_scenes = 1;
     L.particles = {reinterpret_cast<BlockWork *>(b + o_pm), (unsigned)maps.particles.size()};
     L.pair_particles = {reinterpret_cast<BlockWork *>(b + o_ppm), (unsigned)maps.pair_particles.size()};
+    L.staged = L.pair_particles;
     L.cells = {reinterpret_cast<BlockWork *>(b + o_cm), (unsigned)maps.cells.size()};
     L.scan = {reinterpret_cast<BlockWork *>(b + o_sm), (unsigned)maps.scan.size()};
     L.block = block;

@@ -184,39 +184,42 @@ void sph_launch_gather(const Launch &L, bool vel, bool dens, bool solid) {
                                                                           dens ? 1 : 0, solid ? 1 : 0);
 }
 
-// Blocks of a SPLIT launch: each map entry in groups of 32 particles.
-static unsigned split_per(const Launch &L) { return L.pair_block / 32u; }
-static unsigned split_grid(const Launch &L, const BlockMap &m) {
-    const unsigned long long g = (unsigned long long)m.num * split_per(L);
+// Blocks of a SPLIT launch: each map entry in groups of 32 particles, `per`
+// of them.
+static unsigned split_grid(const Launch &L, const BlockMap &m, unsigned per) {
+    const unsigned long long g = (unsigned long long)m.num * per;
     return g < L.grid_cap ? (g ? (unsigned)g : 1u) : L.grid_cap;
 }
+
+#define SPH_STAGED_WARPS (SPH_STAGED_BLOCK / 32u)
 
 template <bool PLANES>
 static void launch_density(const Launch &L, const BlockMap &m, int original, int mask, int skip_solids) {
     if (L.split_rows)
-        sph_launch(L, k_density<PLANES, true>, split_grid(L, m), dim3(32, 3), sizeof(DensityStage<true>), L.scenes, m,
-                   original, mask, skip_solids, split_per(L));
+        sph_launch(L, k_density<PLANES, true>, split_grid(L, m, SPH_STAGED_WARPS), dim3(32, 3),
+                   sizeof(DensityStage<true>), L.scenes, m, original, mask, skip_solids, SPH_STAGED_WARPS);
     else
-        sph_launch(L, k_density<PLANES, false>, grid_for(m, L.grid_cap), L.pair_block, sizeof(DensityStage<false>),
+        sph_launch(L, k_density<PLANES, false>, grid_for(m, L.grid_cap), SPH_STAGED_BLOCK, sizeof(DensityStage<false>),
                    L.scenes, m, original, mask, skip_solids, 1u);
 }
 
 void sph_launch_density(const Launch &L, bool original, bool mask, bool skip_solids) {
     const int o = original ? 1 : 0, m = mask ? 1 : 0, sk = skip_solids ? 1 : 0;
-    launch_density<false>(L, L.pair_particles, o, m, sk);
-    if (!L.no_symmetry_planes) launch_density<true>(L, L.pair_particles, o, m, 0);
+    launch_density<false>(L, L.staged, o, m, sk);
+    if (!L.no_symmetry_planes) launch_density<true>(L, L.staged, o, m, 0);
 }
 
 void sph_launch_density_fused(const Launch &L, const Launch *fluids) {
-    if (fluids && fluids->pair_particles.num) launch_density<false>(L, fluids->pair_particles, 0, 1, 1);
-    if (!L.no_symmetry_planes) launch_density<true>(L, L.pair_particles, 0, 1, 0);
+    if (fluids && fluids->staged.num) launch_density<false>(L, fluids->staged, 0, 1, 1);
+    if (!L.no_symmetry_planes) launch_density<true>(L, L.staged, 0, 1, 0);
 }
 
 template <bool MIXED>
 static void launch_forces_masked(const Launch &L, int step) {
     const BlockMap &m = L.pair_particles;
+    const unsigned per = L.pair_block / 32u;
     if (L.split_rows)
-        sph_launch(L, k_forces_fluids_masked<MIXED, true>, split_grid(L, m), dim3(32, 3), 0, L.scenes, m, step, split_per(L));
+        sph_launch(L, k_forces_fluids_masked<MIXED, true>, split_grid(L, m, per), dim3(32, 3), 0, L.scenes, m, step, per);
     else
         sph_launch(L, k_forces_fluids_masked<MIXED>, grid_for(m, L.grid_cap), L.pair_block, 0, L.scenes, m, step, 1u);
 }
@@ -270,15 +273,18 @@ void sph_launch_init_original_position(const Launch &L) {
 }
 
 void sph_launch_rotations_and_strains(const Launch &L, bool with_density, bool with_stress) {
-    const unsigned g = grid_for(L.pair_particles, L.grid_cap);
-    const unsigned w = L.pair_block / 32u;
+    const BlockMap &m = L.staged;
+    const unsigned w = SPH_STAGED_WARPS;
     const int d = with_density ? 1 : 0, st = with_density && with_stress ? 1 : 0;
     if (L.split_rows)
-        sph_launch(L, k_rotations_and_strains<true>, split_grid(L, L.pair_particles), dim3(32, 3), solid_smem_bytes(true, 3), L.scenes, L.pair_particles, d, st, split_per(L));
+        sph_launch(L, k_rotations_and_strains<true>, split_grid(L, m, w), dim3(32, 3), solid_smem_bytes(true, 3),
+                   L.scenes, m, d, st, w);
     else
-        sph_launch(L, k_rotations_and_strains<false>, g, dim3(32, w), solid_smem_bytes(false, w), L.scenes, L.pair_particles, d, st, 1u);
+        sph_launch(L, k_rotations_and_strains<false>, grid_for(m, L.grid_cap), dim3(32, w), solid_smem_bytes(false, w),
+                   L.scenes, m, d, st, 1u);
     if (!L.no_symmetry_planes)
-        sph_launch(L, k_rotations_and_strains_planes, g, L.pair_block, 0, L.scenes, L.pair_particles);
+        sph_launch(L, k_rotations_and_strains_planes, grid_for(L.pair_particles, L.grid_cap), L.pair_block, 0, L.scenes,
+                   L.pair_particles);
 }
 
 void sph_launch_stresses(const Launch &L, bool corot, bool sorted, bool planes_only) {
@@ -293,30 +299,36 @@ void sph_launch_stresses(const Launch &L, bool corot, bool sorted, bool planes_o
 }
 
 void sph_launch_deformations(const Launch &L, bool with_density, bool with_stress) {
-    const unsigned g = grid_for(L.pair_particles, L.grid_cap);
-    const unsigned w = L.pair_block / 32u;
+    const BlockMap &m = L.staged;
+    const unsigned w = SPH_STAGED_WARPS;
     const int d = with_density ? 1 : 0, st = with_density && with_stress ? 1 : 0;
     if (L.split_rows)
-        sph_launch(L, k_deformations<true>, split_grid(L, L.pair_particles), dim3(32, 3), solid_smem_bytes(true, 3), L.scenes, L.pair_particles, d, st, split_per(L));
+        sph_launch(L, k_deformations<true>, split_grid(L, m, w), dim3(32, 3), solid_smem_bytes(true, 3), L.scenes, m, d,
+                   st, w);
     else
-        sph_launch(L, k_deformations<false>, g, dim3(32, w), solid_smem_bytes(false, w), L.scenes, L.pair_particles, d,
-                                                                                       st, 1u);
-    if (!L.no_symmetry_planes) sph_launch(L, k_deformations_planes, g, L.pair_block, 0, L.scenes, L.pair_particles);
+        sph_launch(L, k_deformations<false>, grid_for(m, L.grid_cap), dim3(32, w), solid_smem_bytes(false, w), L.scenes,
+                   m, d, st, 1u);
+    if (!L.no_symmetry_planes)
+        sph_launch(L, k_deformations_planes, grid_for(L.pair_particles, L.grid_cap), L.pair_block, 0, L.scenes,
+                   L.pair_particles);
 }
 
 template <bool COROT>
 static void launch_forces_solids(const Launch &L, bool masked, int step) {
-    const BlockMap &m = L.pair_particles;
-    const dim3 part(32, 3), whole(32, L.pair_block / 32u);
-    const unsigned gp = split_grid(L, m), g = grid_for(m, L.grid_cap), per = split_per(L);
+    const BlockMap &m = L.staged;
+    const unsigned w = SPH_STAGED_WARPS, gp = split_grid(L, m, w), g = grid_for(m, L.grid_cap);
+    const dim3 part(32, 3), whole(32, w);
+    const size_t sp = solid_force_smem_bytes(3), sw = solid_force_smem_bytes(w);
     if (L.split_rows) {
-        if (masked) sph_launch(L, k_forces_solids<COROT, true, true>, gp, part, solid_force_smem_bytes(3), L.scenes, m, step, per);
-        else sph_launch(L, k_forces_solids<COROT, false, true>, gp, part, solid_force_smem_bytes(3), L.scenes, m, 0, per);
+        if (masked) sph_launch(L, k_forces_solids<COROT, true, true>, gp, part, sp, L.scenes, m, step, w);
+        else sph_launch(L, k_forces_solids<COROT, false, true>, gp, part, sp, L.scenes, m, 0, w);
     } else {
-        if (masked) sph_launch(L, k_forces_solids<COROT, true, false>, g, whole, solid_force_smem_bytes(whole.y), L.scenes, m, step, 1u);
-        else sph_launch(L, k_forces_solids<COROT, false, false>, g, whole, solid_force_smem_bytes(whole.y), L.scenes, m, 0, 1u);
+        if (masked) sph_launch(L, k_forces_solids<COROT, true, false>, g, whole, sw, L.scenes, m, step, 1u);
+        else sph_launch(L, k_forces_solids<COROT, false, false>, g, whole, sw, L.scenes, m, 0, 1u);
     }
-    if (!L.no_symmetry_planes) sph_launch(L, k_forces_solids_planes<COROT>, g, L.pair_block, 0, L.scenes, m);
+    if (!L.no_symmetry_planes)
+        sph_launch(L, k_forces_solids_planes<COROT>, grid_for(L.pair_particles, L.grid_cap), L.pair_block, 0, L.scenes,
+                   L.pair_particles);
 }
 
 void sph_launch_forces_solids(const Launch &L, bool corot, bool masked, bool fuse_step) {

@@ -15,8 +15,9 @@ struct Launch {
     BlockMap cells;           // `block` cells per entry
     BlockMap scan;            // SPH_SCAN_TILE cells per entry
     unsigned block;           // threads per block for particle/cell kernels
-    unsigned pair_block;      // threads per block for the pair kernels
+    unsigned pair_block;      // threads per block for the pair kernels that stage nothing
     BlockMap pair_particles;  // `pair_block` items per entry
+    BlockMap staged;          // SPH_STAGED_BLOCK items per entry: the pair kernels that stage
     unsigned grid_cap;        // upper bound on blocks per launch (persistent loop)
     cudaStream_t stream;
     // no scene of the table has symmetry planes: the density pass's plane

@@ -144,6 +144,13 @@ struct RigidWork {
 // float4s of a scene's pair constants (kernels_common.cuh, ScenePair).
 #define SPH_PAIR_CONSTS 2
 
+// Items per block of the pair passes that stage their rows or sums in shared
+// memory: their buffers are sized for it, whatever block the caller tunes the
+// other pair passes to.  Over a batch of 64 scenes, at pair blocks of 32, 128
+// and 512 items: density pass 190, 102 and 198 us, first corotational pass
+// 188, 182 and 255, corotational forces 152, 126 and 144.
+#define SPH_STAGED_BLOCK 128
+
 // Block map entry: block b of a launch works on `scene`, items
 // [first, first + block size).
 struct BlockWork {

@@ -416,10 +416,13 @@ void sph_build_maps(const std::vector<SceneDesc> &descs, const std::vector<unsig
     out->pair_particles.clear();
     out->cells.clear();
     out->scan.clear();
+    out->staged.clear();
     for (unsigned s : ids) {
         const SceneDesc &d = descs[s];
         for (unsigned f = 0; f < d.pnum; f += block) out->particles.push_back({s, f});
         for (unsigned f = 0; f < d.pnum; f += pair_block) out->pair_particles.push_back({s, f});
+        if (pair_block != SPH_STAGED_BLOCK)
+            for (unsigned f = 0; f < d.pnum; f += SPH_STAGED_BLOCK) out->staged.push_back({s, f});
         for (unsigned f = 0; f < d.num_cells; f += block) out->cells.push_back({s, f});
         for (unsigned f = 0; f < d.num_cells; f += SPH_SCAN_TILE) out->scan.push_back({s, f});
     }

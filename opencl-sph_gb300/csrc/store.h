@@ -38,6 +38,8 @@ std::vector<unsigned> sph_rigid_bodies(const psdata &h, const SceneDesc &d);
 // Block maps for a table of scenes (host vectors; BlockWork entries).
 struct HostMaps {
     std::vector<BlockWork> particles, pair_particles, cells, scan;
+    // SPH_STAGED_BLOCK items per entry; empty where pair_particles is that
+    std::vector<BlockWork> staged;
 };
 void sph_build_maps(const std::vector<SceneDesc> &descs, const std::vector<unsigned> &scene_ids, unsigned block,
                     unsigned pair_block, HostMaps *out);
