@@ -1265,7 +1265,6 @@ __global__ void __maxnreg__(80)
         for (int c = 0; c < 9; ++c) R[c] = S.rotation[9 * (size_t)i + c];
         corot_nmat(R, I.side.s, false, I.M);
     }
-    const float visc = *S.viscosity;
     float total[6];
     const StencilRows rows(S, S.srow[kc]);
     const bool scan = !MASKED || S.ncand[kc] == SPH_NCAND_SCAN;
@@ -1321,7 +1320,7 @@ __global__ void __maxnreg__(80)
             t.add(part(1));
             t.add(part(2));
         }
-        total[c] = t.times(c < 3 ? 0.5f * I.side.vol0 : visc);
+        total[c] = t.times(c < 3 ? 0.5f * I.side.vol0 : *S.viscosity);
     }
     const float3 fe = make_float3(total[0], total[1], total[2]), fv = make_float3(total[3], total[4], total[5]);
     st3(S.force, i, fe + fv);
