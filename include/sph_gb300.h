@@ -392,7 +392,7 @@ unsigned int sph_batch_status(sph_batch *batch, int id);
  * same names.  `status`, when not NULL, is a device word into which the
  * call ORs its status bits (those of sph_status: bit 1 = a particle lay
  * outside gridbounds and was clamped into an edge cell); NULL drops them.
- * The scratch is a fixed file-scope device array (about 12.2 MiB, held by
+ * The scratch is a fixed file-scope device array (about 12.1 MiB, held by
  * every GPU that loads the library until the process exits), so
  * n <= SPH_NOALLOC_MAX_PARTICLES and rx*ry*rz <= SPH_NOALLOC_MAX_CELLS;
  * larger sizes return -1 with an error message.  The call allocates

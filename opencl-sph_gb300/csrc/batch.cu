@@ -136,7 +136,6 @@ bool solid_setup(sph_batch *b, BatchScene *sc) {
     size_t o_p = t.add(m.particles.data(), m.particles.size() * sizeof(BlockWork));
     size_t o_pp = t.add(m.pair_particles.data(), m.pair_particles.size() * sizeof(BlockWork));
     size_t o_st = t.add(m.staged.data(), m.staged.size() * sizeof(BlockWork));
-    size_t o_c = t.add(m.cells.data(), m.cells.size() * sizeof(BlockWork));
     size_t o_s = t.add(m.scan.data(), m.scan.size() * sizeof(BlockWork));
     char *d = nullptr;
     if (!balloc(b, (void **)&d, t.host.size(), b->stream, "scene setup tables")) return false;
@@ -148,7 +147,6 @@ bool solid_setup(sph_batch *b, BatchScene *sc) {
     L.particles = map_at(d, o_p, m.particles);
     L.pair_particles = map_at(d, o_pp, m.pair_particles);
     L.staged = m.staged.empty() ? L.pair_particles : map_at(d, o_st, m.staged);
-    L.cells = map_at(d, o_c, m.cells);
     L.scan = map_at(d, o_s, m.scan);
     L.block = b->block;
     L.pair_block = b->pair_block;
@@ -196,7 +194,6 @@ bool rebuild(sph_batch *b) {
     size_t o_p = t.add(all.particles.data(), all.particles.size() * sizeof(BlockWork));
     size_t o_pp = t.add(all.pair_particles.data(), all.pair_particles.size() * sizeof(BlockWork));
     size_t o_st = t.add(all.staged.data(), all.staged.size() * sizeof(BlockWork));
-    size_t o_c = t.add(all.cells.data(), all.cells.size() * sizeof(BlockWork));
     size_t o_s = t.add(all.scan.data(), all.scan.size() * sizeof(BlockWork));
     std::vector<RigidWork> rigid;
     for (unsigned k = 0; k < descs.size(); ++k)
@@ -223,7 +220,6 @@ bool rebuild(sph_batch *b) {
     A.particles = map_at(d, o_p, all.particles);
     A.pair_particles = map_at(d, o_pp, all.pair_particles);
     A.staged = all.staged.empty() ? A.pair_particles : map_at(d, o_st, all.staged);
-    A.cells = map_at(d, o_c, all.cells);
     A.scan = map_at(d, o_s, all.scan);
     A.block = b->block;
     A.pair_block = b->pair_block;
@@ -322,8 +318,7 @@ extern "C" sph_batch *sph_batch_create(void) {
     good = good && ok(cudaMemPoolCreate(&b->pool, &props), "sph_batch_create (memory pool)") &&
            ok(cudaMemPoolSetAttribute(b->pool, cudaMemPoolAttrReleaseThreshold, (void *)&keep),
               "sph_batch_create (memory pool)");
-    good = good && ok(sph_prepare_kernels(), "sph_batch_create") &&
-                ok(cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking), "sph_batch_create") &&
+    good = good && ok(cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking), "sph_batch_create") &&
                 ok(cudaStreamCreateWithFlags(&b->side[0], cudaStreamNonBlocking), "sph_batch_create") &&
                 ok(cudaStreamCreateWithFlags(&b->side[1], cudaStreamNonBlocking), "sph_batch_create") &&
                 ok(cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming), "sph_batch_create") &&

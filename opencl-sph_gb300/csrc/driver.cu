@@ -248,14 +248,12 @@ Store *create_store(psdata *data, const char *file_list, std::string *err) {
     size_t o_desc = o_scratch + Arena::align(sph_scratch_bytes(probe));
     size_t o_pm = o_desc + Arena::align(sizeof(SceneDesc));
     size_t o_ppm = o_pm + Arena::align(maps.particles.size() * sizeof(BlockWork));
-    size_t o_cm = o_ppm + Arena::align(maps.pair_particles.size() * sizeof(BlockWork));
-    size_t o_sm = o_cm + Arena::align(maps.cells.size() * sizeof(BlockWork));
+    size_t o_sm = o_ppm + Arena::align(maps.pair_particles.size() * sizeof(BlockWork));
     size_t o_rw = o_sm + Arena::align(maps.scan.size() * sizeof(BlockWork));
     s->rigid_room = std::min(probe.body_capacity, SPH_MAX_RIGID_WORK);
     size_t total = o_rw + Arena::align(s->rigid_room * sizeof(RigidWork));
 
-    if (!cuda_ok(sph_prepare_kernels(), "kernel attributes") ||
-        !cuda_ok(cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking), "cudaStreamCreate") ||
+    if (!cuda_ok(cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking), "cudaStreamCreate") ||
         !cuda_ok(cudaMalloc(&s->arena.base, total), "cudaMalloc(store)")) {
         *err = sph_last_error();
         destroy(s);
@@ -277,7 +275,6 @@ Store *create_store(psdata *data, const char *file_list, std::string *err) {
     bool ok = up(o_blob, data->data, s->blob_size) && up(o_desc, &s->desc, sizeof(SceneDesc)) &&
               up(o_pm, maps.particles.data(), maps.particles.size() * sizeof(BlockWork)) &&
               up(o_ppm, maps.pair_particles.data(), maps.pair_particles.size() * sizeof(BlockWork)) &&
-              up(o_cm, maps.cells.data(), maps.cells.size() * sizeof(BlockWork)) &&
               up(o_sm, maps.scan.data(), maps.scan.size() * sizeof(BlockWork)) &&
               cuda_ok(cudaMemsetAsync(s->desc.status, 0, 4, s->stream), "cudaMemset(status)") &&
               (!s->desc.rigid_state ||
@@ -296,7 +293,6 @@ Store *create_store(psdata *data, const char *file_list, std::string *err) {
     L.particles = {reinterpret_cast<BlockWork *>(b + o_pm), (unsigned)maps.particles.size()};
     L.pair_particles = {reinterpret_cast<BlockWork *>(b + o_ppm), (unsigned)maps.pair_particles.size()};
     L.staged = L.pair_particles;
-    L.cells = {reinterpret_cast<BlockWork *>(b + o_cm), (unsigned)maps.cells.size()};
     L.scan = {reinterpret_cast<BlockWork *>(b + o_sm), (unsigned)maps.scan.size()};
     L.block = block;
     L.pair_block = pair_block;

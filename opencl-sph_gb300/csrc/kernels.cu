@@ -70,27 +70,10 @@ static void launch_grid_small(const Launch &L, bool vel, bool solid) {
     cudaLaunchKernelEx(&cfg, k_grid_small<GATHER>, L.scenes, vel ? 1 : 0, solid ? 1 : 0);
 }
 
-cudaError_t sph_prepare_kernels() {
-    // the density pass's staging buffers may exceed the default limit
-    cudaError_t e = cudaSuccess;
-    auto room = [&](const void *kernel, size_t bytes) {
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    };
-    const size_t whole = sizeof(DensityStage<false>);
-    room((const void *)k_density<false, false>, whole);
-    room((const void *)k_density<true, false>, whole);
-    const size_t most = solid_smem_bytes(false, 16);  // pair blocks of 512
-    room((const void *)k_rotations_and_strains<false>, most);
-    room((const void *)k_deformations<false>, most);
-    if (SPH_SMALL_BLOCKS > 8) {
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(k_grid_small<true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(k_grid_small<false>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    }
-    return e;
-}
+// what a kernel may have without asking for more
+static_assert(sizeof(DensityStage<false>) <= 48 * 1024 && sizeof(DensityStage<true>) <= 48 * 1024 &&
+                  solid_smem_bytes(false, SPH_STAGED_BLOCK / 32) <= 48 * 1024 && solid_smem_bytes(true, 3) <= 48 * 1024,
+              "staging buffers");
 
 // Split against whole fluid passes, us a substep with three scenes' substeps
 // overlapping / one scene's alone: 1,000 particles 16.4 / 47.0 -> 14.6 /

@@ -265,7 +265,6 @@ __device__ __forceinline__ void density_block(const SceneDesc &S, unsigned n, un
         return hit;
     };
     const int dz0 = SPLIT ? (int)threadIdx.y : 0, dz1 = SPLIT ? dz0 + 1 : 3;
-    unsigned *mask = S.nbmask + (size_t)(6 * dz0) * pnum + k;
     stage_plane(dz0);
 #pragma unroll 1
     for (int dz = dz0; dz < dz1; ++dz) {
@@ -331,10 +330,7 @@ __device__ __forceinline__ void density_block(const SceneDesc &S, unsigned n, un
             if (SPLIT) stage.rows[3 * dz + dy][threadIdx.x] = rowsum;
             else rho.add(rowsum);
             if (MASK && active) {
-                // store_row_mask's layout
-                mask[0] = lo;
-                if (len > 32u) mask[pnum] = hi;
-                mask += 2 * (size_t)pnum;
+                store_row_mask(S, k, 3 * dz + dy, len, lo, hi);
                 overflow |= len > 64;
                 total += len;
             }

@@ -12,9 +12,8 @@ struct Launch {
     const SceneDesc *scenes;  // device table
     unsigned num_scenes;
     BlockMap particles;       // `block` items per entry
-    BlockMap cells;           // `block` cells per entry
     BlockMap scan;            // SPH_SCAN_TILE cells per entry
-    unsigned block;           // threads per block for particle/cell kernels
+    unsigned block;           // threads per block for particle kernels
     unsigned pair_block;      // threads per block for the pair kernels that stage nothing
     BlockMap pair_particles;  // `pair_block` items per entry
     BlockMap staged;          // SPH_STAGED_BLOCK items per entry: the pair kernels that stage
@@ -188,14 +187,11 @@ void sph_launch_solid_passes(const Launch &L, bool corot, PhaseMark mark = nullp
 
 // Whether one cluster builds the grid of a scene of this size: a rule on the
 // sizes, and that the device can run the cluster (call outside any stream
-// capture, after sph_prepare_kernels).
+// capture).
 bool sph_small_grid(unsigned pnum, unsigned num_cells);
 
 // Whether a launch over this many particles splits the stencil.
 bool sph_split_rows(unsigned long long particles);
-
-// One-time kernel attributes (call outside any stream capture).
-cudaError_t sph_prepare_kernels();
 
 // cudaGetLastError() after the enqueues above; records and returns it.
 cudaError_t sph_check_launch(const char *what);

@@ -12,7 +12,7 @@
 // sph_compute_particle_bins_noalloc serves them: the caller passes its own
 // device buffers for the inputs and outputs, and the scratch comes from one
 // file-scope device array of fixed size, below.  Every GPU that loads this
-// library holds that array (about 12.2 MiB) until the process exits.
+// library holds that array (about 12.1 MiB) until the process exits.
 //
 // The array is shared by every call on a device and keeps the previous
 // call's contents; everything that must start at zero is cleared at the
@@ -46,8 +46,7 @@ constexpr size_t kN = kScan + align256(4 * kMaxScanTiles);                     /
 constexpr size_t kStatus = kN + 256;                                           // u32 status
 constexpr size_t kDesc = kStatus + 256;                                        // SceneDesc
 constexpr size_t kPMap = kDesc + align256(sizeof(SceneDesc));                  // BlockWork per 256 particles
-constexpr size_t kCMap = kPMap + align256(sizeof(BlockWork) * (kMaxParticles / kBlock));
-constexpr size_t kSMap = kCMap + align256(sizeof(BlockWork) * (kMaxCells / kBlock));
+constexpr size_t kSMap = kPMap + align256(sizeof(BlockWork) * (kMaxParticles / kBlock));
 constexpr size_t kBytes = kSMap + align256(sizeof(BlockWork) * kMaxScanTiles);
 
 }  // namespace
@@ -70,13 +69,10 @@ __global__ void k_noalloc_setup(unsigned char *base, SceneDesc d, unsigned n) {
         *reinterpret_cast<unsigned *>(base + kStatus) = 0u;
     }
     BlockWork *pm = reinterpret_cast<BlockWork *>(base + kPMap);
-    BlockWork *cm = reinterpret_cast<BlockWork *>(base + kCMap);
     BlockWork *sm = reinterpret_cast<BlockWork *>(base + kSMap);
     const unsigned np = (n + kBlock - 1) / kBlock;
-    const unsigned nc = (d.num_cells + kBlock - 1) / kBlock;
     const unsigned ns = (d.num_cells + SPH_SCAN_TILE - 1) / SPH_SCAN_TILE;
     for (unsigned b = t; b < np; b += stride) pm[b] = BlockWork{0u, b * kBlock};
-    for (unsigned b = t; b < nc; b += stride) cm[b] = BlockWork{0u, b * kBlock};
     for (unsigned b = t; b < ns; b += stride) sm[b] = BlockWork{0u, b * SPH_SCAN_TILE};
 }
 
@@ -163,7 +159,6 @@ extern "C" int sph_compute_particle_bins_noalloc(const float *position, unsigned
     L.scenes = reinterpret_cast<const SceneDesc *>(base + kDesc);
     L.num_scenes = 1;
     L.particles = {reinterpret_cast<const BlockWork *>(base + kPMap), (n + kBlock - 1) / kBlock};
-    L.cells = {reinterpret_cast<const BlockWork *>(base + kCMap), (unsigned)((cells + kBlock - 1) / kBlock)};
     L.scan = {reinterpret_cast<const BlockWork *>(base + kSMap), d.num_scan_blocks};
     L.pair_particles = L.particles;
     L.block = kBlock;

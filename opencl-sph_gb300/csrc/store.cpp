@@ -414,7 +414,6 @@ void sph_build_maps(const std::vector<SceneDesc> &descs, const std::vector<unsig
                     unsigned pair_block, HostMaps *out) {
     out->particles.clear();
     out->pair_particles.clear();
-    out->cells.clear();
     out->scan.clear();
     out->staged.clear();
     for (unsigned s : ids) {
@@ -423,7 +422,6 @@ void sph_build_maps(const std::vector<SceneDesc> &descs, const std::vector<unsig
         for (unsigned f = 0; f < d.pnum; f += pair_block) out->pair_particles.push_back({s, f});
         if (pair_block != SPH_STAGED_BLOCK)
             for (unsigned f = 0; f < d.pnum; f += SPH_STAGED_BLOCK) out->staged.push_back({s, f});
-        for (unsigned f = 0; f < d.num_cells; f += block) out->cells.push_back({s, f});
         for (unsigned f = 0; f < d.num_cells; f += SPH_SCAN_TILE) out->scan.push_back({s, f});
     }
 }

@@ -37,7 +37,7 @@ std::vector<unsigned> sph_rigid_bodies(const psdata &h, const SceneDesc &d);
 
 // Block maps for a table of scenes (host vectors; BlockWork entries).
 struct HostMaps {
-    std::vector<BlockWork> particles, pair_particles, cells, scan;
+    std::vector<BlockWork> particles, pair_particles, scan;
     // SPH_STAGED_BLOCK items per entry; empty where pair_particles is that
     std::vector<BlockWork> staged;
 };
