@@ -796,11 +796,34 @@ def _fill(view, val):
         view[...] = arr
 
 
+def oracle_fields(scene):
+    """The fields of the scene's store as the CPU oracle takes them, made
+    here: the reference arm's process maps none of the product's libraries,
+    also where the reference's own builder is not there to make them.  The
+    grid's resolution as that builder's: the extent's float difference over
+    the float radius, divided in double."""
+    sizes = {name: int(val) for name, dims, typ, val in scene.entries
+             if typ == "unsigned int" and dims == "1" and val is not None}
+    fields = {}
+    for name, dims, typ, val in scene.entries:
+        shape = tuple(sizes[d] if d in sizes else int(d) for d in dims.replace(" ", "").split(","))[::-1]
+        arr = np.zeros(shape, np.uint32 if typ == "unsigned int" else np.float32)
+        if val is not None and arr.size:
+            arr.reshape(-1)[:np.size(val)] = np.ravel(val)
+        fields[name] = arr
+    bounds = fields["gridbounds"].reshape(3, 2)
+    extent = np.abs((bounds[:, 1] - bounds[:, 0]).astype(np.float64))
+    fields["gridres"] = (extent / np.float64(fields["smoothingradius"][0])).astype(np.uint32)
+    for name, val in scene.init.items():
+        _fill(fields[name], val)
+    return fields
+
+
 def cpu_sample(scene, material, steps, nthreads, reference, warmup=1):
-    """Times the CPU oracle (or, with `reference`, the reference's own
-    kernels in a store the reference's own builder made) on `steps`
-    substeps of the scene, after `warmup` untimed ones (at least one);
-    returns (particle-steps, seconds, kind)."""
+    """Times the CPU oracle (or, with `reference` and where they were built,
+    the reference's own kernels in a store the reference's own builder made)
+    on `steps` substeps of the scene, after `warmup` untimed ones (at least
+    one); returns (particle-steps, seconds, kind)."""
     kind = "port"
     if reference:
         from oracle import ref
@@ -828,14 +851,8 @@ def cpu_sample(scene, material, steps, nthreads, reference, warmup=1):
                 rs.call(prog, "f32", k, scene.n, nthreads)
         closer = rs.free
     else:
-        from sph import bindings as bnd
-        from sph import init_data_cpu, free_data_cpu
         from oracle.oracle import OracleScene
-        ps = init_data_cpu(scene.spec)
-        v = bnd.store_views(ps)
-        for k, val in scene.init.items():
-            _fill(v[k], val)
-        orc = OracleScene(v, "f32", nthreads=nthreads)
+        orc = OracleScene(oracle_fields(scene), "f32", nthreads=nthreads)
         if material != "fluid":
             orc.setup_solid()
 
@@ -843,7 +860,7 @@ def cpu_sample(scene, material, steps, nthreads, reference, warmup=1):
             orc.substep(material)
 
         def closer():
-            free_data_cpu(ps)
+            pass
     for _ in range(max(1, warmup)):
         one()
     t0 = time.perf_counter()
@@ -1017,8 +1034,11 @@ def run_reference(args, rank, world):
         "data": "synthetic (seeded lattice scenes, seed %d)" % args.seed,
         "config": workload_config(args.workload, args.seed, standalone=True),
         "cpu_baseline": {"value": value, "unit": UNIT, "cores": nthreads, "kind": kind,
-                         "sample": "%d full substeps of every scene of the workload (the reference's kernels in "
-                                   "stores its own builder made)" % args.steps},
+                         "sample": "%d full substeps of every scene of the workload (%s)"
+                                   % (args.steps, "the reference's kernels in stores its own builder made"
+                                      if kind == "reference" else
+                                      "this repository's C restatement of the reference's kernels: the "
+                                      "reference's own were not built here")},
         "e2e": {"value": value, "unit": UNIT, "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0},
     }
 
