@@ -97,14 +97,14 @@ PHASE_BYTES = {
 # kernels of this source: the solid first passes at 72 registers, the solid
 # force passes at 80, the fluid force pass at 64.
 MEASURED_TRAFFIC = {
-    ("wcsph-1m", "density"): 60.09e6,                           # k_density<0, 0>
-    ("wcsph-1m", "forces_fluids+step"): 120.14e6,               # k_forces_fluids_masked<0, 0>
-    ("batched-256", "density"): 289.29e6,                       # k_density<0, 0> (masks, counts, pressure, 1/density too)
-    ("batched-256", "fluid forces+step"): 368.96e6,             # k_forces_fluids_masked<0, 0>
-    ("batched-256", "corotational rotations"): 256.55e6,        # k_rotations_and_strains<0> (with the stress law)
-    ("batched-256", "corotational forces+step"): 245.92e6,      # k_forces_solids<1, 1, 0> (with the step)
-    ("batched-256", "svk deformations"): 131.24e6,              # k_deformations<0> (with the stress law)
-    ("batched-256", "svk forces+step"): 165.05e6,               # k_forces_solids<0, 1, 0> (with the step)
+    ("wcsph-1m", "density"): 58.50e6,                           # k_density<0, 0>
+    ("wcsph-1m", "forces_fluids+step"): 120.08e6,               # k_forces_fluids_masked<0, 0>
+    ("batched-256", "density"): 289.40e6,                       # k_density<0, 0> (masks, counts, pressure, 1/density too)
+    ("batched-256", "fluid forces+step"): 368.53e6,             # k_forces_fluids_masked<0, 0>
+    ("batched-256", "corotational rotations"): 256.27e6,        # k_rotations_and_strains<0> (with the stress law)
+    ("batched-256", "corotational forces+step"): 245.65e6,      # k_forces_solids<1, 1, 0> (with the step)
+    ("batched-256", "svk deformations"): 131.44e6,              # k_deformations<0> (with the stress law)
+    ("batched-256", "svk forces+step"): 165.20e6,               # k_forces_solids<0, 1, 0> (with the step)
 }
 
 # Warp instructions per launch of the same kernels (ncu
@@ -112,14 +112,14 @@ MEASURED_TRAFFIC = {
 # live phase time they give the issue rate, against 4 warp instructions per
 # SM per clock.
 MEASURED_INST = {
-    ("wcsph-1m", "density"): 136.75e6,
-    ("wcsph-1m", "forces_fluids+step"): 117.07e6,
-    ("batched-256", "density"): 353.23e6,
-    ("batched-256", "fluid forces+step"): 300.70e6,
+    ("wcsph-1m", "density"): 141.26e6,
+    ("wcsph-1m", "forces_fluids+step"): 116.78e6,
+    ("batched-256", "density"): 365.20e6,
+    ("batched-256", "fluid forces+step"): 299.95e6,
     ("batched-256", "corotational rotations"): 404.82e6,
-    ("batched-256", "corotational forces+step"): 258.01e6,
+    ("batched-256", "corotational forces+step"): 253.81e6,
     ("batched-256", "svk deformations"): 301.05e6,
-    ("batched-256", "svk forces+step"): 251.40e6,
+    ("batched-256", "svk forces+step"): 246.88e6,
 }
 
 

@@ -222,7 +222,12 @@ int sph_wait_reads(psdata_cuda pso);
  * reference driver issues through call_for_all_particles:
  * scripts/sph/systems.py:194-204 for corotational solids, :225-235 for SVK,
  * src/mex/simstep_fluid.c:18-23 for fluids), as one CUDA graph per substep
- * captured on first use.  Returns 0 or non-zero on failure. */
+ * captured on first use.  The launches' forms follow the store's capacity,
+ * not its active count: up to pnum = 40,000 the pair passes spread a
+ * particle's stencil over three warps, and up to 16,384 (and 65,536 cells)
+ * one launch builds the neighbour grid; a store with room past these lines
+ * takes the forms of a large scene however few particles are active.
+ * Returns 0 or non-zero on failure. */
 int sph_update(psdata_cuda pso, unsigned int num_steps);
 /* Device status word accumulated since the last sph_clear_status():
  * bit 0 = a NaN/Inf position was written, bit 1 = a particle was binned

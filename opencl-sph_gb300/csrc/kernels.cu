@@ -75,12 +75,14 @@ static_assert(sizeof(DensityStage<false>) <= 48 * 1024 && sizeof(DensityStage<tr
                   solid_smem_bytes(false, SPH_STAGED_BLOCK / 32) <= 48 * 1024 && solid_smem_bytes(true, 3) <= 48 * 1024,
               "staging buffers");
 
-// Split against whole fluid passes, us a substep with three scenes' substeps
-// overlapping / one scene's alone: 1,000 particles 16.4 / 47.0 -> 14.6 /
-// 41.2, 8,000 17.7 / 53.6 -> 16.0 / 45.1, 25,000 21.9 / 63.7 -> 20.7 / 54.4,
-// 40,000 27.8 / 72.5 -> 27.9 / 65.0, 64,000 27.4 / 66.0 -> 31.1 / 67: from
+// Split against whole passes of a fluid, us a substep with three scenes' substeps
+// overlapping / one scene's alone: 1,000 particles 14.2 / 40.4 -> 10.3 /
+// 28.8, 8,000 15.8 / 43.1 -> 12.2 / 32.7, 25,000 20.2 / 51.3 -> 17.6 / 41.1,
+// 39,304 22.1 / 53.3 -> 20.2 / 43.1, 64,000 27.2 / 55.7 -> 31.1 / 57.5: from
 // there on the schedulers are full and a block's repeated set-up costs more
-// than its shorter chain saves.
+// than its shorter chain saves.  (Solids: corotational 4,000 31.5 / 88 ->
+// 19.0 / 47, 40,960 60.9 / 127 -> 63.0 / 108; SVK 32,768 44.5 / 101 -> 38.3 /
+// 80, 64,000 63.1 / 118 -> 66.7 / 105.)
 bool sph_split_rows(unsigned long long particles) { return particles <= SPH_SPLIT_PARTICLES; }
 
 // One cluster against five launches, us a substep with three scenes' substeps

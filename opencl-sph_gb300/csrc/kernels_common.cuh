@@ -128,8 +128,9 @@ __device__ __forceinline__ DistBounds dist_bounds(float h) {
 // What the pair passes need of a scene's smoothing radius: h, h^2 (rounded
 // on its own), the distance bounds, 45 / (pi h^6) and the poly6
 // normalisation 315 / (64 pi h^9) (common.cl:78-90).  The bounds take some
-// ten square roots and the factors two divisions, so k_gather, which every
-// pair pass follows, evaluates them once per scene and not in every thread.
+// ten square roots and the factors two divisions, so they are evaluated once
+// per scene with the sorted copies, which every pair pass follows, and not in
+// every thread.
 // With the stencil rows' divisions moved the same way: 1M-particle substep
 // 396 -> 384 us, a 4,000-particle corotational beam 40.1 -> 38.0 us.
 struct ScenePair {
@@ -296,7 +297,7 @@ struct StencilRows {
     // bit r: row r lies in the grid; bit 9 + r: its cell x-1 exists;
     // bit 18 + r: its cell x+1 exists
     unsigned bits;
-    // of a cell: three integer divisions, done once per particle by k_gather
+    // of a cell: three integer divisions, done once per particle (gather_one)
     __device__ __forceinline__ StencilRows(const SceneDesc &S, unsigned cell_) {
         cell = cell_;
         R0 = S.gridres[0];
@@ -315,7 +316,7 @@ struct StencilRows {
             bits |= (1u << r) | (xm << (9 + r)) | (xp << (18 + r));
         }
     }
-    // as k_gather stored it
+    // as gather_one stored it
     __device__ __forceinline__ StencilRows(const SceneDesc &S, uint2 stored) {
         cell = stored.x;
         bits = stored.y;

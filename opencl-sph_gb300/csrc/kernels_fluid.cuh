@@ -4,7 +4,7 @@
 // Pair passes run one thread per cell-sorted particle k (i =
 // cellparticles[k]) so a warp covers a few neighbouring cells and shares
 // their neighbour rows in L1; neighbours are streamed from the float4
-// copies built by k_gather.  Sums are FP32, blocked per stencil row: a
+// copies built by gather_one.  Sums are FP32, blocked per stencil row: a
 // row's terms added in order, the nine row sums with Kahan compensation.
 #pragma once
 
@@ -64,11 +64,11 @@
 // Where there are fewer warps than the schedulers can hold, a warp's own
 // chain of nine rows is the time of the pass.
 //
-// Bound: issue slots, 4,118 warp instructions per 32 particles at 1M (the
-// walk 1,411, near_bits 1,423, the rest row bounds, staging and masks)
-// against 5,001 for testing each candidate exactly as it comes, from rows
-// staged per warp: 160 -> 144 us at 1M particles (ncu), 1M-particle substep
-// 362 -> 349 us, mixed scene 519 -> 477 us.
+// Bound: issue slots, 4,310 warp instructions per 32 particles at 1M (a third
+// each for the walk, near_bits, and row bounds, staging and masks) against
+// 5,001 for testing each candidate exactly as it comes, from rows staged per
+// warp: 160 -> 144 us at 1M particles when it was taken (ncu; 148 with what
+// takes denser planes), 1M-particle substep 384 -> 373 us.
 //
 // The buffers (two in turn, or one per plane), and each row's staged range
 // (first index, padded length).
@@ -603,7 +603,8 @@ __global__ void k_forces_fluids(const SceneDesc *__restrict__ scenes, BlockMap m
 // flight a thread, 32 warps an SM).  Masks whose first candidate is the top
 // bit (one leading-zero count finds the next), no count of neighbours here
 // and a reciprocal root without denormals' scaling: 132.9M -> 117.1M warp
-// instructions, 162 -> 153 us at 1M particles.
+// instructions, 162 -> 153 us at 1M particles; 150 us with one form of the
+// scan, which took the spills with it.
 // At most 64 registers (56: 175 against 168 us with the step at 1M, 72: 174).
 // SPLIT as in the density pass: blocks of (32, 3) threads, a warp per z
 // plane, the row sums added in the same order by the first; 72 registers.

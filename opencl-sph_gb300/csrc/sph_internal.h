@@ -91,8 +91,9 @@ struct SceneDesc {
     // the later passes must scan
     unsigned *nbmask;
     unsigned *ncand;
-    // written by k_gather for the pair passes after it: per sorted particle
-    // (cell, StencilRows bits), and the scene's ScenePair constants
+    // written with the sorted copies (gather_one) for the pair passes after
+    // them: per sorted particle (cell, StencilRows bits), and the scene's
+    // ScenePair constants
     uint2 *srow;
     float4 *pair_consts;
     // solids: cell-sorted copies for the fused substep's pair passes --
