@@ -194,22 +194,15 @@ struct Kahan3 {
     }
     __device__ __forceinline__ float3 get() const { return make_float3(x.s, y.s, z.s); }
 };
-// A sum of products that keeps what its roundings lose, the products' too,
-// in a low part: exactly where a product is no larger than the sum so far,
-// in as many operations as a Kahan sum.  Parts of a sum (Kahan sums too, with
-// their compensations) are joined with the exact rounding error of the
-// addition (the two-sum of Knuth, TAOCP vol. 2, 4.2.2), so that the total is
-// rounded once, with its factor, whatever cancels between them.
+// Parts of a sum, each with what its own compensation holds back: the parts
+// are added with the exact rounding error of each addition (the two-sum of
+// Knuth, TAOCP vol. 2, 4.2.2), so the total is rounded once, with its factor,
+// whatever cancels between them.
 struct CompensatedSum {
     float s, lo;
-    __device__ __forceinline__ CompensatedSum(float s_ = 0.f, float lo_ = 0.f) : s(s_), lo(lo_) {}
-    __device__ __forceinline__ CompensatedSum(const Kahan &k) : s(k.s), lo(-k.c) {}
-    __device__ __forceinline__ void add_product(float a, float b) {
-        const float t = __fmaf_rn(a, b, s);
-        lo = __fadd_rn(lo, __fmaf_rn(a, b, -__fsub_rn(t, s)));
-        s = t;
-    }
-    __device__ __forceinline__ void join(const CompensatedSum &o) {
+    __device__ __forceinline__ CompensatedSum(float s_, float lo_) : s(s_), lo(lo_) {}
+    __device__ __forceinline__ explicit CompensatedSum(const Kahan &k) : s(k.s), lo(-k.c) {}
+    __device__ __forceinline__ void add(const CompensatedSum &o) {
         const float t = __fadd_rn(s, o.s);
         const float b = __fsub_rn(t, s);
         const float err = __fadd_rn(__fsub_rn(s, __fsub_rn(t, b)), __fsub_rn(o.s, b));
@@ -218,14 +211,6 @@ struct CompensatedSum {
     }
     // the sum times a factor
     __device__ __forceinline__ float times(float w) const { return __fmaf_rn(s, w, __fmul_rn(lo, w)); }
-};
-struct CompensatedSum3 {
-    CompensatedSum x, y, z;
-    __device__ __forceinline__ void add_product(float3 v, float w) {
-        x.add_product(v.x, w);
-        y.add_product(v.y, w);
-        z.add_product(v.z, w);
-    }
 };
 // Blocked compensated sum of float3 terms: the terms of one stencil row are
 // added in order onto a row sum (one rounding each, no compensation; the x

@@ -1189,7 +1189,7 @@ struct SolidI {
 // fused multiply-add: within 0.5001 ulp (an error near h grows by
 // h / (h - dist); below 2^-50, where the residual underflows, it vanishes
 // beside any h whose kernels do not overflow).  Error against 64 bits over
-// that of the divided term (mean of 24 scenes): elastic 1.05 -> 0.99,
+// that of the divided term (mean of 24 scenes): elastic 1.05 -> 1.00,
 // viscous 1.13 -> 0.93, against rounded reciprocals and r^2 rsqrt(r^2) alone.
 // IN_RANGE: the caller walks the first pass's masks, whose candidates
 // passed this range test with the same positions and arithmetic (a test
@@ -1201,7 +1201,7 @@ struct SolidI {
 // particles 75.1 -> 76.1).
 template <bool COROT, bool IN_RANGE = false, bool FEW = false>
 __device__ __forceinline__ void solid_pair(const SolidConsts &C, const SolidI &II, const SolidSide &J,
-                                           CompensatedSum3 &fe_s, Kahan3 &fv_s) {
+                                           Kahan3 &fe_s, Kahan3 &fv_s) {
     const SolidSide &I = II.side;
     const float3 x = sub3(I.pos0, J.pos0);
     const float r2 = norm2(sub3(J.pos, I.pos));
@@ -1210,20 +1210,20 @@ __device__ __forceinline__ void solid_pair(const SolidConsts &C, const SolidI &I
     float3 fe;
     if (COROT) {
         const float3 mi = mat_vec(II.M, gx);
-        fe = J.body ? mat_vec_on(mi, J.N, sym_vec(I.s, gx)) : mat_vec_on(mi, J.N, gx);
+        fe = (J.body ? mat_vec_on(mi, J.N, sym_vec(I.s, gx)) : mat_vec_on(mi, J.N, gx)) * J.vol0;
     } else {
         const float3 si = sym_vec(I.s, gx);
         if (FEW) {
-            const float3 both = sym_vec_on(si, J.s, gx), own = si * 2.f;
+            const float3 both = sym_vec_on(si, J.s, gx) * J.vol0, own = si * (2.f * J.vol0);
             fe = make_float3(J.body ? own.x : both.x, J.body ? own.y : both.y, J.body ? own.z : both.z);
         } else {
-            fe = J.body ? si * 2.f : sym_vec_on(si, J.s, gx);
+            fe = J.body ? si * (2.f * J.vol0) : sym_vec_on(si, J.s, gx) * J.vol0;
         }
     }
     const float y = rsqrtf(r2), g = __fmul_rn(r2, y);
     const float dist = r2 > 0.f ? __fmaf_rn(__fmaf_rn(-g, g, r2), __fmul_rn(0.5f, y), g) : 0.f;
     const float lap = r2 <= C.le ? __fmul_rn(C.kv, __fsub_rn(C.h, dist)) : 0.f;
-    fe_s.add_product(fe, J.vol0);
+    fe_s.add(fe);
     fv_s.add_product(sub3(J.vel, I.vel), __fmul_rn(J.mrho, lap));
 }
 
@@ -1231,16 +1231,13 @@ __device__ __forceinline__ void solid_pair(const SolidConsts &C, const SolidI &I
 // walks the masks of the substep's first pair pass, reading the sorted
 // copies; otherwise (a named call) scans every candidate, reading the
 // fields.  Without images the cut-off force equals the force.
-// Blocks as the first pass's.  A plane's sums are compensated, and the three
-// planes' joined with what that holds back and the exact errors of joining
-// them: near equilibrium the two outer planes' elastic sums are large and
-// opposite, and what was dropped between them would be most of the error of
-// the small force that remains.  The elastic sum keeps a low part of its own
-// (rounding left at equilibrium, in 2^-24 of the terms' magnitudes: 0.066; by
-// Kahan sums joined 0.11, one Kahan sum over the stencil 0.106, plane sums
-// added plainly 0.166); the viscous one is a Kahan sum a plane (a low part
-// too: SVK cube of 32,768 particles 31.2 -> 32.0 us a substep).  The totals
-// are kept in shared memory, so that they hold no registers during the walk.
+// Blocks as the first pass's.  A plane's terms are added with Kahan
+// compensation, and the three planes' sums with their compensations and the
+// exact errors of adding them (CompensatedSum): near equilibrium the two
+// outer planes' sums are large and opposite, and what was dropped between
+// them would be most of the error of the small force that remains.  The
+// totals are kept in shared memory, so that they hold no registers during
+// the walk.
 // At most 80 registers: six 128-thread blocks per SM instead of five keep
 // more gathers in flight in this latency-bound pass.
 template <bool COROT, bool MASKED, bool SPLIT>
@@ -1273,8 +1270,7 @@ __global__ void __maxnreg__(80)
     const bool scan = !MASKED || S.ncand[kc] == SPH_NCAND_SCAN;
 #pragma unroll 1
     for (int dz = dz0; dz < dz1; ++dz) {
-        CompensatedSum3 fe_s;
-        Kahan3 fv_s;
+        Kahan3 fe_s, fv_s;
         if (active) {
             auto visit = [&](unsigned kk) {
                 SolidSide J;
@@ -1299,14 +1295,14 @@ __global__ void __maxnreg__(80)
                 for_each_masked(S, k, rows, visit_masked, 3 * dz, 3 * dz + 3);
             }
         }
-        const CompensatedSum v[6] = {fe_s.x, fe_s.y, fe_s.z, fv_s.x, fv_s.y, fv_s.z};
+        const Kahan v[6] = {fe_s.x, fe_s.y, fe_s.z, fv_s.x, fv_s.y, fv_s.z};
         float (&to)[12][32] = sums[SPLIT ? dz : (int)threadIdx.y];
 #pragma unroll
         for (int c = 0; c < 6; ++c) {
-            CompensatedSum t = v[c];
+            CompensatedSum t(v[c]);
             if (!SPLIT && dz != dz0) {
-                t = CompensatedSum{to[c][threadIdx.x], to[6 + c][threadIdx.x]};
-                t.join(v[c]);
+                t = CompensatedSum(to[c][threadIdx.x], to[6 + c][threadIdx.x]);
+                t.add(CompensatedSum(v[c]));
             }
             to[c][threadIdx.x] = t.s;
             to[6 + c][threadIdx.x] = t.lo;
@@ -1318,11 +1314,11 @@ __global__ void __maxnreg__(80)
     }
 #pragma unroll
     for (int c = 0; c < 6; ++c) {
-        auto part = [&](unsigned q) { return CompensatedSum{sums[q][c][threadIdx.x], sums[q][6 + c][threadIdx.x]}; };
+        auto part = [&](unsigned q) { return CompensatedSum(sums[q][c][threadIdx.x], sums[q][6 + c][threadIdx.x]); };
         CompensatedSum t = part(SPLIT ? 0u : threadIdx.y);
         if (SPLIT) {
-            t.join(part(1));
-            t.join(part(2));
+            t.add(part(1));
+            t.add(part(2));
         }
         total[c] = t.times(c < 3 ? 0.5f * I.side.vol0 : *S.viscosity);
     }

@@ -15,8 +15,7 @@ pytestmark = pytest.mark.gpu
 # In units of 2^-24 times the sum of the terms' magnitudes, emulated in
 # numpy over 200 stresses and both places of a particle in its cell: one
 # Kahan sum over the stencil leaves 0.08 rms, one per z plane joined with
-# its compensation 0.10 (with a low part of its own 0.06), one per z plane
-# without it 0.20.
+# its compensation 0.10, one per z plane without it 0.20.
 @pytest.mark.parametrize("material", ["corot", "svk"])
 @pytest.mark.parametrize("dims", [(14, 14, 14), (36, 36, 33)])  # split over three warps; whole
 def test_equilibrium_forces_keep_the_sums_compensation(material, dims):
